@@ -36,54 +36,73 @@ struct ModeSetup {
   double2 s;  // e^{-2 pi i c k0 / n} / (wf T (1 + 2L))
 };
 
-__device__ inline ModeSetup SetupMode(const SigIter &it, int32_t k0) {
+// The mode's setup by the lanes of one warp. The two erf of WindowInFreq are
+// evaluated by the even and the odd lanes, each one of them (FP64 runs at two
+// lanes per clock, so a warp pays for an erf once per evaluation).
+__device__ inline ModeSetup SetupMode(const SigIter &it, int32_t k0, int lane) {
   const int64_t n = it.n, B = it.bins;
   const ModN mod{uint32_t(n), it.n_inv};
   ModeSetup m;
   m.k1 = mod(int64_t(it.a) * k0 + it.b);
   m.beta = int(mod.quot(m.k1 * B));
   const double xi0 = double(m.k1) / double(n) - (double(m.beta) + 0.5) / double(B);
-  const double wf = WindowInFreq(it, xi0);
+  const double h = 0.5 * it.width;
+  const double e = erf((xi0 + ((lane & 1) ? -h : h)) * it.erf_d);
+  const double wf = 0.5 * (__shfl_sync(0xffffffffu, e, 0) - __shfl_sync(0xffffffffu, e, 1));
   const double scale = 1.0 / (wf * double(it.trials * (1 + 2 * it.bits)));
   m.s = cscale(Phase64(it, -int64_t(it.c) * k0), scale);
   return m;
 }
 
-// forward: one thread per mode, bins from ubuf (trials x rows x bins_cap)
-__global__ void k_estimate(const SigIter *__restrict__ its, const int32_t *k0s,
-                           int64_t m, double2 *coef) {
+// forward: one warp per mode, its lanes over the (trial, row) values of the
+// mode's bin in ubuf (trials x rows x bins_cap), then a shuffle tree. The
+// work of a mode is a few FP64 operations per row, so what matters is that
+// the modes spread over the SMs' FP64 pipes and that no lane walks the rows
+// one after another: at 200 modes and 25 rows a thread per mode (two blocks)
+// took 25 us of a 162 us call, which a warp per mode in a block of its own
+// brings to 150 us.
+__global__ void __launch_bounds__(32) k_estimate(const SigIter *__restrict__ its,
+                                                 const int32_t *k0s, int64_t m,
+                                                 double2 *coef) {
   const SigIter &it = *its;
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  const ModeSetup ms = SetupMode(it, k0s[i]);
-  double2 acc = make_double2(0.0, 0.0);
-  for (int t = 0; t < it.trials; ++t) {
-    for (int r = 0; r < it.rows; ++r) {
+  const int lane = threadIdx.x;
+  for (int64_t i = blockIdx.x; i < m; i += gridDim.x) {
+    const ModeSetup ms = SetupMode(it, k0s[i], lane);
+    double2 acc = make_double2(0.0, 0.0);
+    for (int j = lane; j < it.trials * it.rows; j += 32) {
+      const int t = j / it.rows, r = j - t * it.rows;
       const int64_t tau = int64_t(it.q[t]) + RowOffset(r, it.bins);
-      const double2 u = it.ubuf[(size_t(t) * it.rows + r) * it.bins_cap + ms.beta];
+      const double2 u = it.ubuf[size_t(j) * it.bins_cap + ms.beta];
       acc = cadd(acc, cmul(u, Phase64(it, -tau * ms.k1)));
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+      acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+    }
+    if (lane == 0) coef[i] = cmul(acc, ms.s);
   }
-  coef[i] = cmul(acc, ms.s);
 }
 
 // adjoint, step 1: G (in the fold buffer, zeroed) += conj(s_k) g_k
 // e^{2 pi i tau k1 / n}, stored conjugated for the forward FFT that follows
-// (conj(DFT(conj(G))) is the inverse DFT of G).
-__global__ void k_adjoint_spread(const SigIter *__restrict__ its,
-                                 const int32_t *k0s, const double2 *g,
-                                 int64_t m) {
+// (conj(DFT(conj(G))) is the inverse DFT of G). One warp per mode, its lanes
+// over the rows, as k_estimate (a thread per mode took 29 us; the adjoint's
+// call went from 565 to 545 us).
+__global__ void __launch_bounds__(32) k_adjoint_spread(const SigIter *__restrict__ its,
+                                                       const int32_t *k0s,
+                                                       const double2 *g, int64_t m) {
   const SigIter &it = *its;
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  const ModeSetup ms = SetupMode(it, k0s[i]);
-  const double2 w = cmul(cconj(ms.s), g[i]);
+  const int lane = threadIdx.x;
   double2 *G = reinterpret_cast<double2 *>(it.fold);
-  for (int t = 0; t < it.trials; ++t) {
-    for (int r = 0; r < it.rows; ++r) {
+  for (int64_t i = blockIdx.x; i < m; i += gridDim.x) {
+    const ModeSetup ms = SetupMode(it, k0s[i], lane);
+    const double2 w = cmul(cconj(ms.s), g[i]);
+    for (int j = lane; j < it.trials * it.rows; j += 32) {
+      const int t = j / it.rows, r = j - t * it.rows;
       const int64_t tau = int64_t(it.q[t]) + RowOffset(r, it.bins);
       const double2 v = cconj(cmul(w, Phase64(it, tau * ms.k1)));
-      double2 *dst = G + (size_t(t) * it.rows + r) * it.bins_cap + ms.beta;
+      double2 *dst = G + size_t(j) * it.bins_cap + ms.beta;
       atomicAdd(&dst->x, v.x);
       atomicAdd(&dst->y, v.y);
     }
@@ -118,19 +137,22 @@ __global__ void k_adjoint_scatter(const SigIter *__restrict__ its, double2 *dx) 
   atomicAdd(&dx[j].y, v.y);
 }
 
+// A block (one warp) per mode up to 2^20 of them, striding beyond.
+unsigned ModeBlocks(int64_t m) {
+  return unsigned(m < (int64_t(1) << 20) ? m : (int64_t(1) << 20));
+}
+
 }  // namespace
 
 void LaunchEstimate(const SigIter *d_it, const int32_t *k0, int64_t m,
                     double2 *coef, cudaStream_t s) {
   if (m <= 0) return;
-  k_estimate<<<unsigned((m + 127) / 128), 128, 0, s>>>(d_it, k0, m, coef);
+  k_estimate<<<ModeBlocks(m), 32, 0, s>>>(d_it, k0, m, coef);
 }
 
 void LaunchAdjointSpread(const SigIter *d_it, const int32_t *k0, const double2 *g,
                          int64_t m, cudaStream_t s) {
-  if (m > 0) {
-    k_adjoint_spread<<<unsigned((m + 127) / 128), 128, 0, s>>>(d_it, k0, g, m);
-  }
+  if (m > 0) k_adjoint_spread<<<ModeBlocks(m), 32, 0, s>>>(d_it, k0, g, m);
 }
 
 void LaunchAdjointScatter(const SigIter *d_it, int64_t items, double2 *dx,

@@ -196,3 +196,26 @@ def test_gradient_matches_dense_dft_rows(ctx):
     err = np.linalg.norm(proj - g) / np.linalg.norm(g)
     print(f"||n D_S A^H g - g|| / ||g|| = {err:.2e} over {ks.size} modes")
     assert err < 1e-4
+
+
+@pytest.mark.parametrize("n,bins,trials,modes", [
+    (1 << 14, 101, 1, 1),      # one mode, rows below a warp
+    (1 << 14, 7, 3, 40),       # 3 x 23 rows: more than two warps' lanes
+    (16381, 51, 15, 9),        # the most trials, prime n
+])
+def test_estimate_rows_over_lanes(ctx, port, n, bins, trials, modes):
+    """A warp per mode walks the trials x rows values: fewer and more of them
+    than lanes, against the formula on the oracle's bins (1e-10) and the
+    adjoint identity (1e-12, as above)."""
+    rng = np.random.default_rng(n + bins)
+    k = rng.choice(n, modes, replace=False).astype(np.int32)
+    x = _tone_signal(n, k, np.exp(2j * np.pi * rng.random(modes)), 1e-3, rng)
+    su = _setup(ctx, n, bins, 1e-5, trials, 5)
+    sig = ctx.upload(x)
+    got = ctx.estimate(sig, su, k)
+    want = _reference_estimate(port, x, su, k)
+    assert np.abs(got - want).max() <= 1e-10 * np.abs(want).max()
+    g = rng.standard_normal(modes) + 1j * rng.standard_normal(modes)
+    ahg = ctx.adjoint(n, su, k, g)
+    lhs, rhs = np.vdot(g, got), np.vdot(ahg, x)
+    assert abs(lhs - rhs) <= 1e-12 * np.linalg.norm(g) * np.linalg.norm(got) * 10
