@@ -3,6 +3,7 @@
 // Data layout in device memory, per signal and iteration (all row-major):
 //   x      : n complex samples, complex64 (float2) or complex128 (double2)
 //   wt32/64: window at |t| for t in [0, p2] (the window is even), FP32 / FP64
+//   wmod   : wt64 modulated by the binning phase of row 0, complex128
 //   fold   : trials x rows x bins_cap complex (FP32 or FP64), folded samples
 //   ubuf   : trials x rows x bins_cap complex128, bins after the size-B FFT
 //   table  : open-addressing hash of found modes, key k0 (-1 = empty) and
@@ -109,6 +110,11 @@ struct SigIter {
   float *wt32;
   double *wt64;
   float2 *wtff;         // wt64 as float-float (hi, lo); may be null
+  // FP64 path: the window modulated by the row-independent part of the
+  // binning phase, wt(t) e^{2 pi i (b t / n - t / (2 bins))} for t in [0, p2]
+  // (conjugate at -t), and per trial and row [t * rows + r] the rest of it with
+  // the row factor, e^{2 pi i (b (q_t + off_r) mod n)/n} (k_window_mod)
+  double2 *wmod, *row_fac;
   void *fold;           // FP32: float2, FP64: double2
   // a second fold buffer of the same size: in the fixed-bins phase the next
   // iteration (planned ahead) folds into it while this iteration's row

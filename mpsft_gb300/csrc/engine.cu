@@ -258,6 +258,8 @@ void CarveSignal(Carve &cv, const Shape &s, SigIter *it, int32_t **ctl) {
   it->wt32 = cv.take<float>(size_t(s.p2_cap) + 1);
   it->wt64 = cv.take<double>(size_t(s.p2_cap) + 1);
   it->wtff = cv.take<float2>(size_t(s.p2_cap) + 1);
+  it->wmod = cv.take<double2>(size_t(s.p2_cap) + 1);
+  it->row_fac = cv.take<double2>(size_t(s.trials) * s.rows_cap);
   const size_t cells = size_t(s.trials) * s.rows_cap * s.bins_cap;
   // 16-byte cells: the FP32 path may redo an iteration in FP64
   it->fold = cv.take<double2>(cells);
@@ -791,6 +793,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   }
   if (fp64) {
     LaunchWindow(d_its, nsig, mx.p2, s);
+    LaunchWindowMod(d_its, nsig, mx.bins, false, false, s);
   } else if (!ahead) {
     LaunchWindow32(d_its, nsig, mx.p2, s);
   }
@@ -831,7 +834,8 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   // Bluestein setup, mode preparation with bucketing, window(s), fold, FFT,
   // decide (ahead: the next iteration's plan and fold, bucketing, FP64
   // window, FFT, decide)
-  if (launched) *launched += ahead ? 6 : (fp64 ? 6 : 7);
+  // FP64: the modulated window instead of the second window table
+  if (launched) *launched += ahead ? 6 : 7;
   if (!fp64) {
     // side stream: the listed bins' FP64 mode terms (before any merge
     // changes a coefficient), then the merge of the other bins, beside the
@@ -852,6 +856,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
     if (redo) {
       LaunchModePrep(d_its, nsig, mx.cap, s, true);
       LaunchBluesteinSetup(d_its, nsig, mx.m, true, ctx->tw32, ctx->tw64, s, true);
+      LaunchWindowMod(d_its, nsig, mx.bins, false, true, s);
       if (timer && ctx->profiling) LaunchDelay(20000, s);
       if (timer) {
         int rc = timer->Begin(1);
@@ -866,7 +871,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
       LaunchRowFFT(d_its, nsig, mx.rows, mx.trials, mx.m, true, ctx->tw32,
                    ctx->tw64, s, true);
       LaunchDecide(d_its, nsig, mx.bins, mx.trials, false, false, s, true);
-      if (launched) *launched += 5;
+      if (launched) *launched += 6;
     }
   }
   if (side_merge) {
@@ -2323,11 +2328,16 @@ int BinInTimeImpl(mpsft_ctx *ctx, const mpsft_signal *sig, int32_t bins,
   FillIter(&it, sig, bins, bits, w, tf, &q, 1);
   cudaStream_t st = ctx->stream;
   // the window tables: evaluated on the device, or the caller's uploaded
-  auto window = [&](bool all64) -> int {
-    if (wt) return UploadWindowTable(ctx, it, wt, st);
-    if (all64) {
-      LaunchWindow(d_it, 1, it.p2, st);
-    } else {
+  auto window = [&]() -> int {
+    if (wt) {
+      const int r = UploadWindowTable(ctx, it, wt, st);
+      if (r) return r;
+    }
+    if (direct) {
+      if (!wt) LaunchWindow(d_it, 1, it.p2, st);
+    } else if (fp64) {
+      LaunchWindowMod(d_it, 1, bins, !wt, false, st);
+    } else if (!wt) {
       LaunchWindow32(d_it, 1, it.p2, st);
     }
     return MPSFT_OK;
@@ -2352,7 +2362,7 @@ int BinInTimeImpl(mpsft_ctx *ctx, const mpsft_signal *sig, int32_t bins,
                                     cudaMemcpyHostToDevice, st));
     MPSFT_CUDA(ctx, cudaMemcpyAsync(d_it, &it, sizeof(it), cudaMemcpyHostToDevice,
                                     st));
-    rc = window(true);
+    rc = window();
     if (rc) return rc;
     LaunchRebin(d_it, 1, bins, sig->dtype == MPSFT_C128, true, st);
     MPSFT_CUDA(ctx, cudaGetLastError());
@@ -2376,7 +2386,7 @@ int BinInTimeImpl(mpsft_ctx *ctx, const mpsft_signal *sig, int32_t bins,
                                   ctx->stream));
   // the window the solves use: FP64 for the FP64 path, FP32-evaluated for
   // FP32 (a caller's table: as given, and rounded to FP32)
-  rc = window(fp64);
+  rc = window();
   if (rc) return rc;
   LaunchBluesteinSetup(d_it, 1, it.fft_m, fp64, ctx->tw32, ctx->tw64, st);
   BinTimer timer{ctx};
@@ -2561,7 +2571,7 @@ namespace {
 
 // Shared setup of mpsft_estimate / mpsft_adjoint: validates, carves one
 // signal's buffers plus `extra` bytes, fills and uploads the descriptor, and
-// builds the FP64 window, Bluestein and unit-phase tables.
+// builds the modulated window, FP64 Bluestein and unit-phase tables.
 int EstimateSetup(mpsft_ctx *ctx, int32_t n, const void *x,
                   const mpsft_estimate_setup *su, size_t extra, Carve *cv,
                   SigIter *it, SigIter **d_it) {
@@ -2605,7 +2615,7 @@ int EstimateSetup(mpsft_ctx *ctx, int32_t n, const void *x,
   MPSFT_CUDA(ctx, cudaMemcpyAsync(*d_it, it, sizeof(SigIter),
                                   cudaMemcpyHostToDevice, st));
   LaunchPhaseTables(*d_it, 1, PhaseTableEntries(n), st);
-  LaunchWindow(*d_it, 1, it->p2, st);
+  LaunchWindowMod(*d_it, 1, su->bins, true, false, st);
   LaunchBluesteinSetup(*d_it, 1, it->fft_m, true, ctx->tw32, ctx->tw64, st);
   MPSFT_CUDA(ctx, cudaGetLastError());
   return MPSFT_OK;
@@ -2683,17 +2693,10 @@ int mpsft_adjoint(mpsft_ctx *ctx, int32_t n, const mpsft_estimate_setup *setup,
                                     cudaMemcpyHostToDevice, st));
   }
   LaunchAdjointSpread(d_it, d_k0, d_g, m, st);
-  // inverse DFT of every row as conj(DFT(conj(G))): the row transform with
-  // unit row factors
-  for (int t = 0; t < it.trials; ++t) {
-    it.bq_re[t] = 1.0;
-    it.bq_im[t] = 0.0;
-  }
-  MPSFT_CUDA(ctx, cudaMemcpyAsync(d_it, &it, sizeof(SigIter),
-                                  cudaMemcpyHostToDevice, st));
+  // inverse DFT of every row as conj(DFT(conj(G)))
   LaunchRowFFT(d_it, 1, it.rows, it.trials, it.fft_m, true, ctx->tw32, ctx->tw64,
                st);
-  LaunchAdjointScatter(d_it, int64_t(it.trials) * it.rows * it.p, d_dx, st);
+  LaunchAdjointScatter(d_it, it.p, it.rows, it.trials, d_dx, st);
   MPSFT_CUDA(ctx, cudaGetLastError());
   MPSFT_CUDA(ctx, cudaMemcpyAsync(dx, d_dx, sizeof(double2) * size_t(n),
                                   cudaMemcpyDeviceToHost, st));

@@ -17,8 +17,8 @@
 // subtract), so no 64-bit division runs per sample. FP32: the phase is carried
 // in fixed-point turns (exact reduction mod 1 by wrap-around) and converted
 // only for sincospif; products in FP32; the per-lane sums and the lane tree
-// use compensated (TwoSum) addition. FP64: per-sample double phase and
-// sincospi, plain sums (the straightforward port).
+// use compensated (TwoSum) addition. FP64: the modulated window wmod
+// (k_window_mod), plain sums.
 #include "common.cuh"
 #include "launch.h"
 
@@ -48,39 +48,21 @@ template <> __device__ inline float2 to_f2<double2>(double2 v) {
   return make_float2(float(v.x), float(v.y));
 }
 template <typename TX> __device__ inline double2 to_d2x(TX v);
+// float -> double by integer shifts for normal values (the conversion
+// instruction runs on the FP64 pipes, two lanes per clock); zeros, subnormals,
+// infinities and NaN take the conversion.
+__device__ inline double Widen(float v) {
+  const uint32_t b = __float_as_uint(v);
+  if ((b & 0x7f800000u) - 0x00800000u < 0x7f000000u) {
+    const uint32_t hi = (b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u);
+    return __hiloint2double(int(hi), int(b << 29));
+  }
+  return double(v);
+}
 template <> __device__ inline double2 to_d2x<float2>(float2 v) {
-  return make_double2(v.x, v.y);
+  return make_double2(Widen(v.x), Widen(v.y));
 }
 template <> __device__ inline double2 to_d2x<double2>(double2 v) { return v; }
-
-// Per-lane setup shared by both precisions.
-struct LaneSetup {
-  int cnt;          // folds handled by this lane
-  int64_t t;        // first t of this lane
-  uint32_t j1, j2;  // gather indices of rows q + off and q - off
-  uint32_t m;       // (b (t + off)) mod n
-  uint32_t a8, m8;  // per-step increments (step 8B in t)
-};
-
-__device__ inline LaneSetup MakeLane(const SigIter &it, int beta, int lane8,
-                                     bool valid, int64_t off, int64_t q) {
-  LaneSetup L;
-  const int B = it.bins;
-  const int64_t n = it.n;
-  const int f = it.folds;
-  // t = beta mod B and |t| <= p2; -p2 = (B + 1)/2 mod B since p = f B, f odd.
-  const int tmin = -it.p2 + int(PosMod(int64_t(beta) - (B + 1) / 2, B));
-  L.t = tmin + int64_t(lane8) * B;
-  L.cnt = (valid && f > lane8) ? (f - lane8 + kFoldLanes - 1) / kFoldLanes : 0;
-  const int64_t a = it.a, b = it.b, c = it.c;
-  L.j1 = uint32_t(PosMod(a * PosMod(q + L.t + off, n) + c, n));
-  L.j2 = uint32_t(PosMod(a * PosMod(q - L.t - off, n) + c, n));
-  L.m = uint32_t(PosMod(b * PosMod(L.t + off, n), n));
-  const int64_t s8 = PosMod(int64_t(kFoldLanes) * B, n);
-  L.a8 = uint32_t(PosMod(a * s8, n));
-  L.m8 = uint32_t(PosMod(b * s8, n));
-  return L;
-}
 
 __device__ inline uint32_t StepUp(uint32_t j, uint32_t d, uint32_t n) {
   j += d;
@@ -363,7 +345,19 @@ __global__ void __launch_bounds__(256, 4)
   }
 }
 
+// The FP64 fold: F_tau without its row-independent phases, which wmod holds,
+// and without e^{2 pi i b off / n}, which the row transform applies with the
+// row factor (row_fac). A sample costs its gather, four FP64 multiply-adds and
+// (complex64 input) two widenings; a pair of rows shares wmod's load. FP64
+// runs at two lanes per clock and SM, so the FP64 operations bound this kernel
+// while the samples come from L2: with a sincospi per pair the launch took
+// 42 us cold at 501 bins, 31 rows, n = 4194301 complex128 (now 17 us, the rate
+// of random DRAM reads). Against an 80-bit evaluation the bins are 4.4e-16 to
+// 5.4e-16 off (5.0e-16 to 6.2e-16 with the sincospi per pair). Eight lanes
+// share a bin, kFold64Batch folds of both rows in flight.
 // cond: only signals whose iteration is redone in FP64 take part.
+constexpr int kFold64Batch = 4;
+
 template <typename TX>
 __global__ void __launch_bounds__(256)
     k_bin_fold64(const SigIter *__restrict__ its, int gmax, int cond) {
@@ -377,42 +371,58 @@ __global__ void __launch_bounds__(256)
   const int tr = blockIdx.y / gmax;
   if (tr >= it.trials || g > it.bits) return;
 
-  const int lane8 = threadIdx.x & (kFoldLanes - 1);
+  const int lane = threadIdx.x & (kFoldLanes - 1);
   const int beta = blockIdx.x * 32 + (threadIdx.x >> 3);
   const bool valid = beta < B;
+  const bool pair = g > 0;
   const uint32_t n = uint32_t(it.n);
-  const int64_t off = g == 0 ? 0 : (int64_t(B) << (g - 1));
-  const LaneSetup L = MakeLane(it, beta, lane8, valid, off, it.q[tr]);
-  const int64_t twoB = 2 * int64_t(B);
-  // -t/(2B) mod 1 is the same for every fold of this lane.
-  const double ct = -double(PosMod(L.t, twoB)) / double(twoB);
-  const double inv_n = 1.0 / double(n);
+  const ModN mod{n, it.n_inv};
+  const int64_t off = pair ? (int64_t(B) << (g - 1)) : 0;
+  // first t of this lane: t = beta mod B with |t| <= p2 (-p2 = (B + 1)/2 mod B
+  // since p = f B with f odd), then every kFoldLanes-th fold
+  int tm = beta - (B + 1) / 2;
+  if (tm < 0) tm += B;
+  int t = -it.p2 + tm + lane * B;
+  const int f = it.folds;
+  const int cnt = (valid && f > lane) ? (f - lane + kFoldLanes - 1) / kFoldLanes : 0;
+  const int64_t q = it.q[tr];
+  const int64_t a = it.a, c = it.c;
+  uint32_t j1 = mod(a * mod(q + t + off) + c);
+  uint32_t j2 = mod(a * mod(q - t - off) + c);
+  const int D = kFoldLanes * B;
+  const uint32_t aD = mod(a * mod(D));
 
   const TX *__restrict__ x = reinterpret_cast<const TX *>(it.x);
-  const double *__restrict__ wt = it.wt64;
-  const bool pair = g > 0;
-
+  const double2 *__restrict__ wm = it.wmod;
   double r1 = 0, i1 = 0, r2 = 0, i2 = 0;
-  uint32_t j1 = L.j1, j2 = L.j2, m = L.m;
-  int64_t t = L.t;
-  for (int k = 0; k < L.cnt; ++k) {
-    const double2 v1 = to_d2x(__ldg(&x[j1]));
-    double2 v2 = make_double2(0, 0);
-    if (pair) v2 = to_d2x(__ldg(&x[j2]));
-    double s, c;
-    sincospi(2.0 * (double(m) * inv_n + ct), &s, &c);
-    const double w = __ldg(&wt[t < 0 ? -t : t]);
-    const double wr = c * w, wi = s * w;
-    r1 += v1.x * wr - v1.y * wi;
-    i1 += v1.x * wi + v1.y * wr;
-    if (pair) {
-      r2 += v2.x * wr + v2.y * wi;
-      i2 += v2.y * wr - v2.x * wi;
+  for (int k0 = 0; k0 < cnt; k0 += kFold64Batch) {
+    TX x1[kFold64Batch], x2[kFold64Batch];
+    double2 w[kFold64Batch];
+#pragma unroll
+    for (int u = 0; u < kFold64Batch; ++u) {
+      if (k0 + u < cnt) {
+        x1[u] = __ldg(&x[j1]);
+        if (pair) x2[u] = __ldg(&x[j2]);
+        w[u] = __ldg(&wm[t < 0 ? -t : t]);
+        if (t < 0) w[u].y = -w[u].y;
+        j1 = StepUp(j1, aD, n);
+        j2 = StepDown(j2, aD, n);
+        t += D;
+      }
     }
-    j1 = StepUp(j1, L.a8, n);
-    j2 = StepDown(j2, L.a8, n);
-    m = StepUp(m, L.m8, n);
-    t += int64_t(kFoldLanes) * B;
+#pragma unroll
+    for (int u = 0; u < kFold64Batch; ++u) {
+      if (k0 + u < cnt) {
+        const double2 v1 = to_d2x(x1[u]);
+        r1 = fma(v1.x, w[u].x, fma(-v1.y, w[u].y, r1));
+        i1 = fma(v1.x, w[u].y, fma(v1.y, w[u].x, i1));
+        if (pair) {
+          const double2 v2 = to_d2x(x2[u]);
+          r2 = fma(v2.x, w[u].x, fma(v2.y, w[u].y, r2));
+          i2 = fma(v2.y, w[u].x, fma(-v2.x, w[u].y, i2));
+        }
+      }
+    }
   }
 #pragma unroll
   for (int o = 1; o < kFoldLanes; o <<= 1) {
@@ -421,7 +431,7 @@ __global__ void __launch_bounds__(256)
     r2 += __shfl_xor_sync(0xffffffffu, r2, o);
     i2 += __shfl_xor_sync(0xffffffffu, i2, o);
   }
-  if (lane8 == 0 && valid) {
+  if (lane == 0 && valid) {
     double2 *fold = reinterpret_cast<double2 *>(it.fold);
     const size_t base = size_t(tr) * it.rows;
     const int rplus = g == 0 ? 0 : 2 * g - 1;

@@ -1,8 +1,9 @@
 // Size-B forward DFT of every folded row (FFTPlan::Run of size B,
 // src/base.cc:86-97, called at src/binner.cc:428 and 509-510), by Bluestein's
 // chirp-z method over the shared-memory radix-2 FFT (any odd B, including
-// large primes), followed by the row factor e^{2 pi i (b q mod n)/n} that the
-// fold left out. Output: complex128 bins in ubuf.
+// large primes), followed by the row factor that the fold left out,
+// e^{2 pi i (b q mod n)/n} (FP32) or e^{2 pi i (b (q + off) mod n)/n} (FP64).
+// Output: complex128 bins in ubuf.
 //
 // One CTA per (row, trial, signal). FP32 path: the convolution runs in FP32
 // (M <= 16384 points, 128 KB of shared memory); FP64 path: in FP64
@@ -164,7 +165,9 @@ __global__ void __launch_bounds__(kRowFftThreads)
     }
   } else if (live) {
     const double inv_m = 1.0 / double(M);
-    const double2 bq = make_double2(it.bq_re[tr], it.bq_im[tr]);
+    const double2 bq = sizeof(V) == sizeof(double2)
+                           ? it.row_fac[tr * it.rows + row]
+                           : make_double2(it.bq_re[tr], it.bq_im[tr]);
     double2 *dst = it.ubuf + (size_t(tr) * it.rows + row) * it.bins_cap;
     for (int k0 = tid; k0 < B; k0 += 8 * nth) {
       V w[8];

@@ -39,6 +39,15 @@ __device__ double SincPi(double x) {
   return r;
 }
 
+// FP64 window at t = i >= 0, in the reference's evaluation order.
+__device__ double Window64At(const SigIter &it, int i) {
+  if (i == 0) return it.width;
+  const double t = double(i);
+  const double u = __dmul_rn(__dmul_rn(t, M_PI), it.sigma_f);
+  return __dmul_rn(__dmul_rn(it.width, SincPi(__dmul_rn(__dmul_rn(t, M_PI), it.width))),
+                   exp(__dmul_rn(__dmul_rn(-2.0, u), u)));
+}
+
 // FP64 window (the reference's evaluation order) into wt64 and, when
 // present, the float-float copy wtff; with_fp32 also rounds it into wt32.
 __global__ void k_window64(const SigIter *__restrict__ its, int with_fp32) {
@@ -47,16 +56,7 @@ __global__ void k_window64(const SigIter *__restrict__ its, int with_fp32) {
   if (!it.active || it.tables_valid) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i > it.p2) return;
-  double v;
-  if (i == 0) {
-    v = it.width;
-  } else {
-    const double t = double(i);
-    const double u = __dmul_rn(__dmul_rn(t, M_PI), it.sigma_f);
-    v = __dmul_rn(__dmul_rn(it.width, SincPi(__dmul_rn(__dmul_rn(t, M_PI),
-                                                       it.width))),
-                  exp(__dmul_rn(__dmul_rn(-2.0, u), u)));
-  }
+  const double v = Window64At(it, i);
   it.wt64[i] = v;
   if (with_fp32) it.wt32[i] = float(v);
   if (it.wtff != nullptr) {
@@ -82,6 +82,92 @@ __global__ void k_window32(const SigIter *__restrict__ its) {
     v = w * (sinpif(y) / (float(M_PI) * y)) * expf(-2.f * u * u);
   }
   it.wt32[i] = v;
+}
+
+// e^{2 pi i m / n} of a residue m in [0, n), reduced to half a turn first.
+__device__ double2 UnitRoot64(int64_t m, int64_t n) {
+  if (2 * m > n) m -= n;
+  double s, c;
+  sincospi(2.0 * (double(m) / double(n)), &s, &c);
+  return make_double2(c, s);
+}
+
+// The modulated window of the FP64 binning, wmod[t] = wt(t) e^{2 pi i (b t/n -
+// t/(2B))} for t in [0, p2], and the row factors row_fac = e^{2 pi i (b (q +
+// off) mod n)/n}: the binning's phase at t of row q + off is
+// e^{2 pi i b off / n} times wmod's, so one table serves every row.
+//
+// With t = r + f B the phase is that of r times e^{2 pi i (b f B mod n)/n}
+// (-1)^f: one FP64 sincospi per r (its angle one exact integer over 2nB) and
+// one per f instead of one per t. FP64 evaluations are what bounds this kernel
+// (a sincospi is about 50 operations, the window twice that, on pipes of two
+// lanes per clock), so a block covers only 8 r's and one signal's bins spread
+// over every SM (501 bins, 18537 window points evaluated: 18 us with 32 r's in
+// 16 blocks, 12.5 us with 8); the last block has the row factors. eval: the
+// window itself is evaluated here (and stored in wt64 when present), else
+// read from wt64.
+constexpr int kModCols = 8, kModThreads = 128;
+constexpr int kModFolds = kFoldLanes * kMaxFoldsPerLane / 2 + 1;  // f = t / B
+static_assert(kModCols + kModFolds <= kModThreads, "a thread per phase");
+
+__global__ void __launch_bounds__(kModThreads)
+    k_window_mod(const SigIter *__restrict__ its, int eval, int cond) {
+  PdlEnter();
+  __shared__ double2 zr[kModCols], zf[kModFolds];
+  const SigIter &it = its[blockIdx.y];
+  if (!it.active) return;
+  if (cond ? !RedoFP64(it) : it.force_fp64) return;
+  const int B = it.bins;
+  const int r0 = blockIdx.x * kModCols;
+  const int64_t n = it.n;
+  const ModN mod{uint32_t(n), it.n_inv};
+  const int64_t b = mod(it.b);
+  const int tid = threadIdx.x;
+  if (blockIdx.x == gridDim.x - 1) {
+    const int rows = it.rows;
+    for (int i = tid; i < it.trials * rows; i += kModThreads) {
+      const int t = i / rows, row = i - t * rows;
+      int64_t off = 0;
+      if (row > 0) {
+        off = int64_t(B) << ((row - 1) >> 1);
+        if ((row & 1) == 0) off = -off;
+      }
+      it.row_fac[i] = UnitRoot64(mod(b * mod(int64_t(it.q[t]) + off)), n);
+    }
+    return;
+  }
+  if (r0 >= B) return;
+  const int nf = it.p2 / B + 1;
+  if (tid < kModCols) {
+    const int64_t r = r0 + tid;
+    const int64_t nB = n * B;
+    int64_t num = 2 * B * int64_t(mod(b * r)) - r * n;  // over 2 n B turns
+    if (num > nB) num -= 2 * nB;
+    double s, c;
+    sincospi(double(num) / double(nB), &s, &c);
+    zr[tid] = make_double2(c, s);
+  } else if (tid < kModCols + nf) {
+    const int f = tid - kModCols;
+    const double2 z = UnitRoot64(mod(b * mod(int64_t(f) * B)), n);
+    zf[f] = (f & 1) ? make_double2(-z.x, -z.y) : z;
+  }
+  __syncthreads();
+  const int r = r0 + (tid & (kModCols - 1));
+  if (r < B) {
+    const double2 z = zr[tid & (kModCols - 1)];
+    for (int f = tid / kModCols; f < nf; f += kModThreads / kModCols) {
+      const int t = r + f * B;
+      if (t > it.p2) break;
+      double w;
+      if (eval) {
+        w = Window64At(it, t);
+        if (it.wt64 != nullptr) it.wt64[t] = w;
+      } else {
+        w = it.wt64[t];
+      }
+      it.wmod[t] = cscale(cmul(z, zf[f]), w);
+    }
+  }
 }
 
 // ph_lo[l] = e^{2 pi i l / n} for l < 2^ph_k and ph_hi[h] = e^{2 pi i h 2^ph_k / n}
@@ -166,6 +252,12 @@ void LaunchPhaseTables(const SigIter *d_its, int nsig, int64_t entries,
 void LaunchWindow(const SigIter *d_its, int nsig, int max_p2, cudaStream_t s) {
   dim3 grid((max_p2 + 1 + 255) / 256, nsig);
   Launch(k_window64, grid, 256, 0, s, d_its, 1);
+}
+
+void LaunchWindowMod(const SigIter *d_its, int nsig, int max_bins, bool eval, bool cond,
+                     cudaStream_t s) {
+  dim3 grid((max_bins + kModCols - 1) / kModCols + 1, nsig);
+  Launch(k_window_mod, grid, kModThreads, 0, s, d_its, eval ? 1 : 0, cond ? 1 : 0);
 }
 
 void LaunchWindow64(const SigIter *d_its, int nsig, int max_p2, cudaStream_t s) {

@@ -59,6 +59,12 @@ void LaunchWindow(const SigIter *d_its, int nsig, int max_p2, cudaStream_t s);
 void LaunchWindow32(const SigIter *d_its, int nsig, int max_p2, cudaStream_t s);
 void LaunchWindow64(const SigIter *d_its, int nsig, int max_p2, cudaStream_t s);
 
+// The modulated window and row factors of the FP64 binning (wmod, row_fac).
+// eval: the window evaluated in the same kernel (into wt64 too when it is not
+// null); otherwise read from wt64.
+void LaunchWindowMod(const SigIter *d_its, int nsig, int max_bins, bool eval, bool cond,
+                     cudaStream_t s);
+
 // Bluestein chirp and FFT(conjugate chirp) of every active signal.
 // fp64 selects double tables.
 // cond: only signals whose iteration is redone in FP64 (more near-tie bins
@@ -179,13 +185,14 @@ void LaunchPencil(const double2 *u3, int64_t count, double *sigma,
 
 // Coefficient estimate of a fixed frequency set from the bins in ubuf
 // (c = A x), and the pieces of its adjoint: spread g, conjugated, over the
-// rows of the fold buffer (zeroed by the caller), then, after a row FFT with
-// unit row factors into ubuf, scatter-add into dx (zeroed, n entries).
+// rows of the fold buffer (zeroed by the caller), then, after the FP64 row FFT
+// into ubuf, scatter-add over the window support p of every row into dx
+// (zeroed, n entries).
 void LaunchEstimate(const SigIter *d_it, const int32_t *k0, int64_t m,
                     double2 *coef, cudaStream_t s);
 void LaunchAdjointSpread(const SigIter *d_it, const int32_t *k0, const double2 *g,
                          int64_t m, cudaStream_t s);
-void LaunchAdjointScatter(const SigIter *d_it, int64_t items, double2 *dx,
+void LaunchAdjointScatter(const SigIter *d_it, int p, int rows, int trials, double2 *dx,
                           cudaStream_t s);
 
 // Whether the kernels with large blocks or shared memory can be launched on

@@ -4,7 +4,7 @@
 // start-up because allocation can block or fragment the pool).
 //
 // All scratch lives in one file-scope __device__ array of a fixed size
-// (kNoAllocScratchBytes, 2.5 MiB), which every GPU that loads this
+// (kNoAllocScratchBytes, about 2.7 MiB), which every GPU that loads this
 // library holds until the process exits. The caller passes the input samples
 // and the output bin matrix as device pointers and a stream; nothing here calls
 // cudaMalloc, cudaFree or any allocating library routine, and nothing is
@@ -40,10 +40,13 @@ constexpr size_t Align256(size_t v) { return (v + 255) & ~size_t(255); }
 constexpr size_t kOffReady = 0;
 constexpr size_t kOffIter = kOffReady + 256;
 constexpr size_t kOffTw32 = kOffIter + Align256(sizeof(SigIter));
-constexpr size_t kOffTw64 = kOffTw32 + Align256(sizeof(float2) * kTwiddleEntries);
-constexpr size_t kOffWt32 = kOffTw64 + Align256(sizeof(double2) * kTwiddleEntries);
-constexpr size_t kOffWt64 = kOffWt32 + Align256(sizeof(float) * (kNaMaxP2 + 1));
-constexpr size_t kOffFold = kOffWt64 + Align256(sizeof(double) * (kNaMaxP2 + 1));
+// the twiddle blocks of transforms up to kNaMaxM points
+constexpr int kNaTwiddles = kNaMaxM - 1;
+constexpr size_t kOffTw64 = kOffTw32 + Align256(sizeof(float2) * kNaTwiddles);
+constexpr size_t kOffRowFac = kOffTw64 + Align256(sizeof(double2) * kNaTwiddles);
+// the FP32 window or the FP64 modulated window (a call uses one)
+constexpr size_t kOffWt = kOffRowFac + Align256(sizeof(double2) * kNaMaxRows);
+constexpr size_t kOffFold = kOffWt + Align256(sizeof(double2) * (kNaMaxP2 + 1));
 constexpr size_t kOffChirp =
     kOffFold + Align256(sizeof(double2) * size_t(kNaMaxRows) * kNaMaxBins);
 constexpr size_t kOffChat = kOffChirp + Align256(sizeof(double2) * kNaMaxBins);
@@ -65,7 +68,7 @@ __global__ void __launch_bounds__(1024)
                     uint32_t *ready) {
   if (threadIdx.x == 0) *dst = it;
   if (*(volatile uint32_t *)ready == kTwiddlesReady) return;
-  for (int e = threadIdx.x; e < kTwiddleEntries; e += blockDim.x) {
+  for (int e = threadIdx.x; e < kNaTwiddles; e += blockDim.x) {
     TwiddleAt(e, tw32, tw64);
   }
   __threadfence();
@@ -119,8 +122,9 @@ extern "C" int mpsft_bin_in_time_noalloc(const void *x_device, int64_t n,
   SigIter it;
   std::memset(&it, 0, sizeof(it));
   FillIter(&it, &sig, bins, bits, delta, tf, &q, 1);
-  it.wt32 = reinterpret_cast<float *>(base + kOffWt32);
-  it.wt64 = reinterpret_cast<double *>(base + kOffWt64);
+  it.wt32 = reinterpret_cast<float *>(base + kOffWt);
+  it.wmod = reinterpret_cast<double2 *>(base + kOffWt);
+  it.row_fac = reinterpret_cast<double2 *>(base + kOffRowFac);
   it.fold = base + kOffFold;
   it.ubuf = reinterpret_cast<double2 *>(out_device);
   it.bins_cap = bins;
@@ -136,7 +140,7 @@ extern "C" int mpsft_bin_in_time_noalloc(const void *x_device, int64_t n,
   k_noalloc_setup<<<1, 1024, 0, st>>>(it, d_it, tw32, tw64,
                                       reinterpret_cast<uint32_t *>(base + kOffReady));
   if (fp64) {
-    LaunchWindow(d_it, 1, it.p2, st);
+    LaunchWindowMod(d_it, 1, bins, true, false, st);
   } else {
     LaunchWindow32(d_it, 1, it.p2, st);
   }

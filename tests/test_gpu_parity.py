@@ -601,3 +601,48 @@ def test_batched_result_layouts(ctx):
     assert offs3[-1] == short and np.array_equal(offs3[:-1], offs[:-1])
     for s in sigs:
         s.free()
+
+
+@pytest.mark.parametrize("n,bins,bits,delta,b", [
+    (1 << 12, 1, 4, 1e-5, 77),       # one bin: every t folds into it
+    (4093, 3, 0, 1e-6, 0),           # row 0 alone, no modulation
+    (1 << 14, 31, 9, 1e-5, 16383),   # below, at and above a block of bins
+    (16381, 33, 8, 1e-6, 5),
+    (1 << 15, 63, 31, 1e-5, 9),      # the most rows whose offsets fit
+    (65521, 1025, 5, 1e-12, 65520),  # many folds
+])
+def test_fp64_bins_from_modulated_window(ctx, port, n, bins, bits, delta, b):
+    """FP64 bins at the edges of the modulated window's blocks against the
+    oracle (1e-11 of max|U|, as above), complex64 and complex128 input."""
+    bits = min(bits, 31 - bins.bit_length())
+    rng = np.random.default_rng(n + bins)
+    x = (rng.standard_normal(n) + 1j * rng.standard_normal(n)).astype(np.complex64)
+    a, c, q = int(rng.integers(1, n)) | 1, int(rng.integers(0, n)), int(rng.integers(0, n))
+    want = port.bin_in_time(x.astype(np.complex128), bins, bits, delta, a, b, c, q)
+    for dtype in (np.complex64, np.complex128):
+        sig = ctx.upload(x.astype(dtype))
+        u = ctx.bin_in_time(sig, bins, bits, delta, a, b, c, q, precision=m.FP64)
+        assert rel_err(u, want) < TOL_BINS[m.FP64]
+        sig.free()
+
+
+def test_fp64_bins_widen_every_float(ctx):
+    """complex64 samples enter the FP64 binning exactly: zeros of both signs,
+    subnormals, the smallest and largest normals, infinities and NaN give the
+    bins of the same samples in complex128 bit for bit."""
+    tiny = np.finfo(np.float32).tiny
+    vals = np.array([0.0, -0.0, 1e-45, -3e-39, tiny, -tiny, 3.4028235e38, 1.0, -1.5],
+                    np.float32)
+    rng = np.random.default_rng(2)
+    n = 1 << 12
+    for extra in ([], [np.inf], [np.nan]):
+        v = np.concatenate([vals, np.array(extra, np.float32)])
+        x = np.zeros(n, np.complex64)
+        x.real, x.imag = rng.choice(v, n), rng.choice(v, n)
+        out = []
+        for dtype in (np.complex64, np.complex128):
+            sig = ctx.upload(x.astype(dtype))
+            out.append(ctx.bin_in_time(sig, 51, 6, 1e-5, 77, 5, 9, 31, precision=m.FP64))
+            sig.free()
+        assert np.array_equal(out[0].view(np.float64), out[1].view(np.float64),
+                              equal_nan=True)
