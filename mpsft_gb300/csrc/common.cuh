@@ -429,13 +429,22 @@ __host__ __device__ constexpr int TwiddleBase(int log2n) { return (1 << (log2n -
 
 // Entry i of the table, in FP64 and rounded to FP32 (every table of the
 // library is filled by this): e^{-2 pi i k / kMaxFFT} with k = e kMaxFFT / N.
+// The FP64 entries of the second quarter turn are those of the first rotated by
+// -i (sincospi's cosine and sine of pi/4 differ in the last bit), so that a
+// transform may take a twiddle either way.
 __device__ inline void TwiddleAt(int i, float2 *tw32, double2 *tw64) {
   const int L = 32 - __clz(i + 1);  // i + 1 in [2^(L-1), 2^L)
   const int k = (i - TwiddleBase(L)) << (kMaxFFTLog2 - L);
   double s, c;
   sincospi(-2.0 * double(k) / double(kMaxFFT), &s, &c);
-  tw64[i] = make_double2(c, s);
   tw32[i] = make_float2(float(c), float(s));
+  if (k >= kMaxFFT / 4) {
+    double s0, c0;
+    sincospi(-2.0 * double(k - kMaxFFT / 4) / double(kMaxFFT), &s0, &c0);
+    c = s0;
+    s = -c0;
+  }
+  tw64[i] = make_double2(c, s);
 }
 
 __device__ inline float2 cmulf(float2 a, float2 b) {

@@ -12,6 +12,8 @@
 // at a small fraction of its FP32 rate, with long latencies): the row factor
 // is applied as a float-float value, and each product is formed with exact
 // FMA products and a two-sum, then rounded once to FP32.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "fft.cuh"
@@ -59,6 +61,9 @@ __device__ __forceinline__ int RowsPerBlock(int M) {
   return r < 1 ? 1 : (r > kRowsMax ? kRowsMax : r);
 }
 
+// FP64 operations bound the FP64 transform (fft.cuh, BlockConv): at 501 bins
+// (M = 1024) and one row per SM 40 us (cold) with whole radix-2 stages, 37 us
+// now; at 101 bins (M = 256) 27 and 18 us.
 template <typename V>
 __global__ void __launch_bounds__(kRowFftThreads)
     k_row_fft(const SigIter *__restrict__ its, int max_trials,
@@ -93,49 +98,92 @@ __global__ void __launch_bounds__(kRowFftThreads)
     bq_ff[1] = make_float2(__double2float_rn(br - double(hr)),
                            __double2float_rn(bi - double(hi)));
   }
-  // element loops: up to 8 elements per thread with their loads issued
-  // together (a thread covers M / nth elements)
-  if (live) {
-    const V *__restrict__ src = reinterpret_cast<const V *>(it.fold) +
-                                (size_t(tr) * it.rows + row) * it.bins_cap;
-    for (int j0 = tid; j0 < M; j0 += 8 * nth) {
-      V v[8];
+  const int L = it.fft_log2m, half = M / 2;
+  if constexpr (sizeof(V) == sizeof(double2)) {
+    // element loops: up to 4 elements per thread with their loads issued
+    // together; the first forward stage (span M/2, its upper inputs zero since
+    // B <= M/2) is part of the fill
+    if (live) {
+      const V *__restrict__ src = reinterpret_cast<const V *>(it.fold) +
+                                  (size_t(tr) * it.rows + row) * it.bins_cap;
+      if (half == 0 && tid == 0) a[0] = vmul(src[0], __ldg(&chirp[0]));
+      for (int j0 = tid; j0 < half; j0 += 4 * nth) {
+        V v[4], w[4];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int j = j0 + u * nth;
-        if (j < M) {
-          v[u] = j < B ? vmul(src[j], __ldg(&chirp[j]))
-                       : vmake2(0.0, 0.0, (V *)nullptr);
+        for (int u = 0; u < 4; ++u) {
+          const int j = j0 + u * nth;
+          v[u] = vmake2(0.0, 0.0, (V *)nullptr);
+          if (j < B) {
+            v[u] = vmul(src[j], __ldg(&chirp[j]));
+            w[u] = Twiddle(tw, L, j, false);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int j = j0 + u * nth;
+          if (j < half) {
+            a[Pad(j)] = v[u];
+            a[Pad(j + half)] = j < B ? vmul(v[u], w[u]) : v[u];
+          }
         }
       }
+    }
+    __syncthreads();
+    // forward DIF (bit-reversed out), product with chat (stored bit-reversed),
+    // inverse DIT (natural out) but for its last stage; rows past the last run
+    // the barriers only
+    BlockConv(a, live ? M : 0, L > 0 ? L - 1 : 0, StagesPerPass(rpb * M), chat, tw, tid,
+              nth);
+  } else {
+    // element loops: up to 8 elements per thread with their loads issued
+    // together (a thread covers M / nth elements)
+    if (live) {
+      const V *__restrict__ src = reinterpret_cast<const V *>(it.fold) +
+                                  (size_t(tr) * it.rows + row) * it.bins_cap;
+      for (int j0 = tid; j0 < M; j0 += 8 * nth) {
+        V v[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int j = j0 + u * nth;
-        if (j < M) a[Pad(j)] = v[u];
+        for (int u = 0; u < 8; ++u) {
+          const int j = j0 + u * nth;
+          if (j < M) {
+            v[u] = j < B ? vmul(src[j], __ldg(&chirp[j]))
+                         : vmake2(0.0, 0.0, (V *)nullptr);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int j = j0 + u * nth;
+          if (j < M) a[Pad(j)] = v[u];
+        }
       }
     }
-  }
-  __syncthreads();
-  // forward DIF (bit-reversed out), product with chat (stored bit-reversed),
-  // inverse DIT (natural out); rows past the last run the barriers only
-  BlockFFTDif(a, live ? M : 0, it.fft_log2m, tw, false, tid, nth);
-  if (live) {
-    for (int j0 = tid; j0 < M; j0 += 8 * nth) {
-      V w[8];
+    __syncthreads();
+    // forward DIF (bit-reversed out), product with chat (stored bit-reversed),
+    // inverse DIT (natural out); rows past the last run the barriers only
+    BlockFFTDif(a, live ? M : 0, it.fft_log2m, tw, false, tid, nth);
+    if (live) {
+      for (int j0 = tid; j0 < M; j0 += 8 * nth) {
+        V w[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int j = j0 + u * nth;
-        if (j < M) w[u] = __ldg(&chat[j]);
-      }
+        for (int u = 0; u < 8; ++u) {
+          const int j = j0 + u * nth;
+          if (j < M) w[u] = __ldg(&chat[j]);
+        }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int j = j0 + u * nth;
-        if (j < M) a[Pad(j)] = vmul(a[Pad(j)], w[u]);
+        for (int u = 0; u < 8; ++u) {
+          const int j = j0 + u * nth;
+          if (j < M) a[Pad(j)] = vmul(a[Pad(j)], w[u]);
+        }
       }
     }
+    __syncthreads();
+    BlockFFTDit(a, live ? M : 0, it.fft_log2m, tw, true, tid, nth);
   }
-  __syncthreads();
-  BlockFFTDit(a, live ? M : 0, it.fft_log2m, tw, true, tid, nth);
+  // output k of the inverse transform (FP64: the lower half of its last stage)
+  auto conv_out = [&](int k) -> V {
+    if (sizeof(V) == sizeof(float2) || half == 0) return a[Pad(k)];
+    return vadd(a[Pad(k)], vmul(a[Pad(k + half)], Twiddle(tw, L, k, true)));
+  };
   float ss = 0.f;  // this thread's share of the row's sum of |U|^2
   float mx = 0.f;  // and of its largest |U|
   if (live && out32) {
@@ -180,8 +228,8 @@ __global__ void __launch_bounds__(kRowFftThreads)
       for (int u = 0; u < 8; ++u) {
         const int k = k0 + u * nth;
         if (k < B) {
-          const double2 y = cscale(to_d2(vmul(a[Pad(k)], w[u])), inv_m);
-          dst[k] = cmul(bq, y);
+          const double2 y = cscale(to_d2(vmul(conv_out(k), w[u])), inv_m);
+          dst[k] = vmul(bq, y);
           const double y2 = y.x * y.x + y.y * y.y;
           ss += float(y2);
           mx = fmaxf(mx, float(sqrt(y2)));
@@ -210,6 +258,161 @@ __global__ void __launch_bounds__(kRowFftThreads)
     float t = 0.f;
     for (int j = 0; j < nseg; ++j) t += seg_ss[lr * nseg + j];
     it.row_ms[tr * it.rows + row] = t / float(B);
+  }
+}
+
+// The FP64 row transform with one row over a cluster of C blocks, for launches
+// of few rows (one signal's call): FP64 operations bound it, and a block per
+// row leaves most SMs' pipes idle. Block c holds the c-th of C slices of the
+// bit-reversed array, Ms = M / C elements. The first log2 C forward stages need
+// no exchange: every block reads the row's samples and evaluates its own
+// outputs of them (the upper half of the input is zero). The stages within a
+// slice run as in k_row_fft; the last log2 C inverse stages read the C
+// slices' element k through distributed shared memory, each block a C-th of
+// the k, and only the outputs below M/2. A transform too small to split
+// (M < kSplitMin C) runs whole on block 0.
+// 31 rows of 501 bins (M = 1024), cold: 37 us with a block per row, 21 us
+// with 4.
+constexpr int kSplitThreads = 256;
+constexpr int kSplitMin = 64;  // elements per slice at least
+
+// One row of one block of the cluster: fill, local stages, exchange, epilogue
+// (dst = row factor * output); returns the block's sum and maximum of |U|^2.
+template <int C>
+__device__ __forceinline__ void SplitRow(const SigIter &it, int tr, int row, int c,
+                                         cooperative_groups::cluster_group cl,
+                                         double2 *a, const double2 *__restrict__ tw,
+                                         bool work, float *ss, float *mx) {
+  constexpr int kLog = C == 8 ? 3 : (C == 4 ? 2 : (C == 2 ? 1 : 0));
+  constexpr int H = C > 1 ? C / 2 : 1;  // slices of the lower half
+  const int B = it.bins, L = it.fft_log2m, M = it.fft_m, Ms = M / C;
+  const int tid = threadIdx.x, lg = L - kLog;
+  const double2 *__restrict__ chirp = it.chirp64;
+  if (work) {
+    const double2 *__restrict__ src = reinterpret_cast<const double2 *>(it.fold) +
+                                      (size_t(tr) * it.rows + row) * it.bins_cap;
+    for (int k = tid; k < Ms; k += kSplitThreads) {
+      double2 v[H];
+#pragma unroll
+      for (int m = 0; m < H; ++m) {
+        const int j = k + m * Ms;
+        v[m] = make_double2(0.0, 0.0);
+        if (j < B) {
+          v[m] = vmul(src[j], __ldg(&chirp[j]));
+          if (C > 1 && (c & (C / 2))) v[m] = vmul(v[m], Twiddle(tw, L, j, false));
+        }
+      }
+#pragma unroll
+      for (int st = 1; st < kLog; ++st) {
+        const int cnt = C >> (st + 1);
+#pragma unroll
+        for (int m = 0; m < H; ++m) {
+          if (m < cnt) {
+            if (c & cnt) {
+              v[m] = vmul(vsub(v[m], v[m + cnt]), Twiddle(tw, L - st, k + m * Ms, false));
+            } else {
+              v[m] = vadd(v[m], v[m + cnt]);
+            }
+          }
+        }
+      }
+      a[Pad(k)] = v[0];
+    }
+  }
+  __syncthreads();
+  BlockConv(a, work ? Ms : 0, lg, StagesPerPass(Ms), it.chat64 + size_t(c) * Ms, tw, tid,
+            kSplitThreads);
+  cl.sync();  // every slice is done
+  if (work) {
+    const double inv_m = 1.0 / double(M);
+    const double2 bq = it.row_fac[tr * it.rows + row];
+    double2 *dst = it.ubuf + (size_t(tr) * it.rows + row) * it.bins_cap;
+    const double2 *part[C];
+#pragma unroll
+    for (int i = 0; i < C; ++i) part[i] = C > 1 ? cl.map_shared_rank(a, i) : a;
+    const int k1 = (c + 1) * (Ms / C);
+    for (int k = c * (Ms / C) + tid; k < k1; k += kSplitThreads) {
+      double2 x[C];
+#pragma unroll
+      for (int i = 0; i < C; ++i) x[i] = part[i][Pad(k)];
+#pragma unroll
+      for (int s = 0; s < kLog; ++s) {
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+          if ((i & (1 << s)) == 0) {
+            const int e = k + (i & ((1 << s) - 1)) * Ms;
+            const double2 v = vmul(x[i + (1 << s)], Twiddle(tw, lg + s + 1, e, true));
+            const double2 u = x[i];
+            x[i] = vadd(u, v);
+            if (s + 1 < kLog) x[i + (1 << s)] = vsub(u, v);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < H; ++i) {
+        const int j = k + i * Ms;
+        if (j < B) {
+          const double2 y = cscale(vmul(x[i], __ldg(&chirp[j])), inv_m);
+          dst[j] = vmul(bq, y);
+          const double y2 = y.x * y.x + y.y * y.y;
+          *ss += float(y2);
+          *mx = fmaxf(*mx, float(sqrt(y2)));
+        }
+      }
+    }
+  }
+}
+
+template <int C>
+__global__ void __launch_bounds__(kSplitThreads)
+    k_row_fft_split(const SigIter *__restrict__ its, const double2 *__restrict__ tw,
+                    int cond) {
+  PdlEnter(its, kTraceRowFft);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ float part_ss[C], part_mx[C];  // block 0's: every block's share
+  __shared__ float warp_ss[kSplitThreads / 32], warp_mx[kSplitThreads / 32];
+  const SigIter &it = its[blockIdx.z];
+  const int row = blockIdx.x / C, tr = blockIdx.y;
+  // (the same for every block of a cluster)
+  if (!it.active || tr >= it.trials || row >= it.rows) return;
+  if (cond ? !RedoFP64(it) : it.force_fp64) return;
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int c = int(cl.block_rank());
+  double2 *a = reinterpret_cast<double2 *>(smem_raw);
+  float ss = 0.f, mx = 0.f;
+  if (it.fft_m >= kSplitMin * C) {
+    SplitRow<C>(it, tr, row, c, cl, a, tw, true, &ss, &mx);
+  } else {
+    SplitRow<1>(it, tr, row, 0, cl, a, tw, c == 0, &ss, &mx);
+  }
+  // the row's largest magnitude and sum of |U|^2 in a fixed order: a shuffle
+  // tree, the warps in order, the blocks in order
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    warp_ss[threadIdx.x >> 5] = ss;
+    warp_mx[threadIdx.x >> 5] = mx;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kSplitThreads / 32; ++w) {
+      ss += warp_ss[w];
+      mx = fmaxf(mx, warp_mx[w]);
+    }
+    *cl.map_shared_rank(&part_ss[c], 0) = ss;
+    *cl.map_shared_rank(&part_mx[c], 0) = mx;
+  }
+  cl.sync();  // the shares are in block 0, and no block reads another's slice any more
+  if (c == 0 && threadIdx.x == 0 && it.row_max != nullptr) {
+    for (int i = 1; i < C; ++i) {
+      ss += part_ss[i];
+      mx = fmaxf(mx, part_mx[i]);
+    }
+    it.row_max[tr * it.rows + row] = mx;
+    it.row_ms[tr * it.rows + row] = ss / float(it.bins);
   }
 }
 
@@ -331,6 +534,23 @@ inline size_t RowFftSlots(int max_m) {
   return one > packed ? one : packed;
 }
 
+// Shared memory of a split row's block: a slice of the largest transform, or
+// a whole one too small to split.
+inline size_t SplitSlots(int max_m, int c) {
+  return size_t(PadLen(std::max(max_m / c, kSplitMin * c)));
+}
+
+template <int C>
+void LaunchRowSplit(const SigIter *d_its, dim3 grid, int max_m, const double2 *tw,
+                    cudaStream_t s, bool cond) {
+  const size_t sm = SplitSlots(max_m, C) * sizeof(double2);
+  cudaFuncSetAttribute(k_row_fft_split<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       int(sm));
+  grid.x *= C;
+  LaunchCluster(k_row_fft_split<C>, grid, kSplitThreads, sm, s, C, d_its, tw,
+                cond ? 1 : 0);
+}
+
 void LaunchRowFFT(const SigIter *d_its, int nsig, int max_rows,
                   int max_trials, int max_m, bool fp64, const float2 *tw32,
                   const double2 *tw64, cudaStream_t s, bool cond) {
@@ -344,9 +564,21 @@ void LaunchRowFFT(const SigIter *d_its, int nsig, int max_rows,
     Launch(k_row_dft_small, g, 64 * kDirectRowsPerBlock, 0, s, d_its, cond ? 1 : 0);
     return;
   }
+  // FP64 with so few rows that they do not fill the SMs' FP64 pipes: a row over
+  // a cluster of as many blocks as leave an SM to each (two blocks on one SM
+  // share its pipes and gain nothing), slices of kSplitMin elements or more
+  const int64_t total = int64_t(max_rows) * max_trials * nsig;
+  if (fp64) {
+    int c = 8;
+    while (c > 1 && (total * c > 152 || max_m < kSplitMin * c)) c /= 2;
+    const dim3 g(max_rows, max_trials, nsig);
+    if (c == 8) return LaunchRowSplit<8>(d_its, g, max_m, tw64, s, cond);
+    if (c == 4) return LaunchRowSplit<4>(d_its, g, max_m, tw64, s, cond);
+    if (c == 2) return LaunchRowSplit<2>(d_its, g, max_m, tw64, s, cond);
+  }
   // (a power of two, so that a row's threads are whole shuffle segments)
   int rpb_cap = 1;
-  while (int64_t(rpb_cap) * 2 <= int64_t(max_rows) * max_trials * nsig / (2 * 152)) {
+  while (int64_t(rpb_cap) * 2 <= total / (2 * 152)) {
     rpb_cap *= 2;
   }
   const int rpb = std::max(
@@ -375,6 +607,13 @@ bool FftKernelsLaunchable() {
                        cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm32));
   cudaFuncSetAttribute(k_row_fft<double2>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm64));
+  // split rows: the largest transform over the smallest cluster
+  int n3 = 0;
+  const size_t sms = SplitSlots(kMaxFFT64, 2) * sizeof(double2);
+  cudaFuncSetAttribute(k_row_fft_split<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       int(sms));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n3, k_row_fft_split<2>, kSplitThreads, sms);
+  if (n3 == 0) return false;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n1, k_row_fft<float2>, 512, sm32);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n2, k_row_fft<double2>, 512, sm64);
   return n1 > 0 && n2 > 0;

@@ -13,6 +13,30 @@ namespace mpsft {
 // kernel before it.
 extern thread_local bool g_launch_pdl;
 
+// A launch of clusters of `cluster` blocks along x (1: no clusters).
+template <typename... P, typename... A>
+inline void LaunchCluster(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                          cudaStream_t s, int cluster, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
+  if (g_launch_pdl) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = unsigned(cluster);
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 template <typename... P, typename... A>
 inline void Launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
                    cudaStream_t s, A... args) {
@@ -20,17 +44,7 @@ inline void Launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
     kernel<<<grid, block, smem, s>>>(args...);
     return;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  LaunchCluster(kernel, grid, block, smem, s, 1, args...);
 }
 
 // The FFT twiddle table (kTwiddleEntries entries, TwiddleAt).

@@ -646,3 +646,27 @@ def test_fp64_bins_widen_every_float(ctx):
             sig.free()
         assert np.array_equal(out[0].view(np.float64), out[1].view(np.float64),
                               equal_nan=True)
+
+
+@pytest.mark.parametrize("bits", [1, 12, 20])
+@pytest.mark.parametrize("bins", [1, 3, 5, 9, 65, 127, 129, 255, 257, 511, 513, 1023, 2047,
+                                  4095, 8191])
+def test_row_transform_sizes(ctx, port, bins, bits):
+    """The size-B transform at the edges of every Bluestein size (M = 1, 8 ..
+    16384; passes of one, two and three stages) and, in FP64, with a row over
+    clusters of 8, 4 and 2 blocks (3, 25 and 41 rows) or too small to split,
+    against the oracle, within the bins' tolerances (FP64 up to 4095 bins)."""
+    n = 1 << 14
+    if bins > 4095 and bits > 1:
+        pytest.skip("FP32 only, any rows")
+    rng = np.random.default_rng(bins)
+    x = (rng.standard_normal(n) + 1j * rng.standard_normal(n)).astype(np.complex64)
+    a, b, c, q = 4097, 77, 5, 4099
+    want = port.bin_in_time(x.astype(np.complex128), bins, bits, 1e-5, a, b, c, q)
+    sig = ctx.upload(x)
+    for prec in PRECS:
+        if prec == m.FP64 and bins > 4095:
+            continue
+        u = ctx.bin_in_time(sig, bins, bits, 1e-5, a, b, c, q, precision=prec)
+        assert rel_err(u, want) < TOL_BINS[prec]
+    sig.free()
