@@ -196,8 +196,8 @@ struct SigIter {
   // FP32 path only: 1 when this signal's FP32 rounding is not small against
   // its noise thresholds, so this iteration runs on the FP64 kernels
   int32_t force_fp64;
-  // 1 when the window and FP32 Bluestein tables for this iteration's bins are
-  // in place (the previous iteration's, the context's table cache, or built
+  // 1 when the window and Bluestein tables (FP32; FP64 for a signal with
+  // force_fp64) for this iteration's bins are in place (the previous iteration's, the context's table cache, or built
   // in this iteration by another signal of the batch): the table kernels skip
   // this signal
   int32_t tables_valid;

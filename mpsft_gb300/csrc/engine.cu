@@ -736,8 +736,7 @@ Maxima MaximaOf(const std::vector<SigIter> &h_its) {
 }
 
 // The kernels of one iteration of every active signal, on stream s (and the
-// context's side stream, forked from and joined back into s). any_forced:
-// some signal of an FP32 call takes the FP64 kernels (precision policy).
+// context's side stream, forked from and joined back into s).
 // The fixed-bins phase's pipelined body: while this iteration decides, the
 // next one (descriptors its_ahead) is planned and gathered/folded on the
 // prefold stream, into the second fold buffer (only this iteration's row FFT
@@ -748,11 +747,67 @@ struct Ahead {
   int32_t plan_max;
 };
 
+// An iteration of an FP32 call whose every signal takes the FP64 kernels (the
+// precision policy, or nearly noiseless signals throughout): the FP64 kernels of
+// the redo alone. The FP32 chain would only return block by block, a kernel after
+// the other: about 100 us of every iteration of a batch of 24 signals.
+int LaunchForcedIteration(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
+                          const Maxima &mx, bool x_c128, BinTimer *timer,
+                          int64_t *launched, cudaStream_t s) {
+  // side stream: mode preparation and bucketing (the decisions wait for them);
+  // low-priority stream: the Bluestein tables (the row transforms do)
+  MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_fork, s));
+  MPSFT_CUDA(ctx, cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
+  LaunchModePrep(d_its, nsig, mx.cap, ctx->side, true);
+  LaunchBucket(d_its, nsig, mx.bins, mx.cap, ctx->side, false);
+  MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_join, ctx->side));
+  MPSFT_CUDA(ctx, cudaStreamWaitEvent(ctx->side64, ctx->ev_fork, 0));
+  LaunchBluesteinSetup(d_its, nsig, mx.m, true, ctx->tw32, ctx->tw64, ctx->side64, true);
+  MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_blue, ctx->side64));
+  LaunchWindow64(d_its, nsig, mx.p2, s);
+  LaunchWindowMod(d_its, nsig, mx.bins, false, true, s);
+  if (timer) {
+    // (tag 0: the iteration's FP32 binning, which has no signal)
+    int rc = timer->Begin();
+    if (rc == MPSFT_OK) rc = timer->End();
+    if (rc) return rc;
+    if (ctx->profiling) {
+      MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join, 0));
+      MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_blue, 0));
+      LaunchDelay(20000, s);
+    }
+    rc = timer->Begin(1);
+    if (rc) return rc;
+  }
+  LaunchBinFold(d_its, nsig, mx.bins, mx.bits, mx.trials, x_c128, true, s, true);
+  if (timer) {
+    int rc = timer->End();
+    if (rc) return rc;
+  }
+  MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_blue, 0));
+  LaunchRowFFT(d_its, nsig, mx.rows, mx.trials, mx.m, true, ctx->tw32, ctx->tw64, s,
+               true);
+  MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join, 0));
+  LaunchDecide(d_its, nsig, mx.bins, mx.trials, false, false, s, true);
+  LaunchMerge(d_its, nsig, mx.bins, s);
+  if (launched) *launched += 9;
+  MPSFT_CUDA(ctx, cudaGetLastError());
+  return MPSFT_OK;
+}
+
+// forced: which signals of an FP32 call take the FP64 kernels (precision
+// policy).
+enum Forced { kNoneForced = 0, kSomeForced = 1, kAllForced = 2 };
+
 int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
                            const Maxima &mx, bool x_c128, bool fp64,
-                           bool any_forced, BinTimer *timer, int64_t *launched,
+                           Forced forced, BinTimer *timer, int64_t *launched,
                            cudaStream_t s, const Ahead *ahead = nullptr) {
   if (mx.bins == 0) return MPSFT_OK;
+  if (forced == kAllForced && !fp64 && mx.m <= kMaxFFT64) {
+    return LaunchForcedIteration(ctx, d_its, nsig, mx, x_c128, timer, launched, s);
+  }
+  const bool any_forced = forced != kNoneForced;
   // fork: tables, mode preparation and bucketing on the side stream while
   // the window and the gather/fold run on the main one; the row FFT waits
   // for the Bluestein tables only, the decisions for the rest (ahead: the
@@ -888,12 +943,17 @@ int LaunchIteration(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
                     const std::vector<SigIter> &h_its, bool x_c128, bool fp64,
                     BinTimer *timer, int64_t *launched = nullptr,
                     int32_t tune_bins = 0) {
-  bool any_forced = false;
-  for (const SigIter &it : h_its) any_forced |= it.active && it.force_fp64;
+  int active = 0, forced = 0;
+  for (const SigIter &it : h_its) {
+    active += it.active;
+    forced += it.active && it.force_fp64;
+  }
   Maxima mx = MaximaOf(h_its);
   mx.tune_bins = tune_bins;
-  const int rc = LaunchIterationKernels(ctx, d_its, nsig, mx, x_c128, fp64, any_forced,
-                                        timer, launched, ctx->stream);
+  const int rc = LaunchIterationKernels(
+      ctx, d_its, nsig, mx, x_c128, fp64,
+      forced == 0 ? kNoneForced : (forced < active ? kSomeForced : kAllForced), timer,
+      launched, ctx->stream);
   if (rc != MPSFT_OK) return rc;
   // (in the solve graph, k_finish inserts the spilled candidates)
   LaunchInsertSpills(d_its, nsig, ctx->stream);
@@ -1050,7 +1110,7 @@ int GraphLoop(mpsft_ctx *ctx, const mpsft_signal *const *sigs,
               mpsft_rng *const *rngs, const std::vector<Shape> &shapes,
               SigIter *d_its, SigIter *d_its_ahead, std::vector<SigIter> *its,
               DrawTables *dt,
-              const std::vector<int32_t> &force, bool any_forced, bool fp64,
+              const std::vector<int32_t> &force, Forced forced, bool fp64,
               bool x_c128, int64_t *launches, const ResultStage &rs,
               std::vector<SolveCtl> *ctl_out) {
   const int tmax = dt->tmax;
@@ -1132,11 +1192,11 @@ int GraphLoop(mpsft_ctx *ctx, const mpsft_signal *const *sigs,
     }
   }
   // the fixed-bins phase runs pipelined on the FP32 path without FP64 redo
-  const bool pipe = !fp64 && !(any_forced && mx.m <= kMaxFFT64);
+  const bool pipe = !fp64 && !(forced != kNoneForced && mx.m <= kMaxFFT64);
   // graph (rebuilt when the launch shape or the arena changes)
   const std::vector<int64_t> key = {
       int64_t(reinterpret_cast<uintptr_t>(ctx->arena)), nsig, mx.bins, mx.bits,
-      mx.rows, mx.p2, mx.m, mx.cap, mx.trials, fp64, x_c128, any_forced,
+      mx.rows, mx.p2, mx.m, mx.cap, mx.trials, fp64, x_c128, int64_t(forced),
       small_bins, mx_small.p2, pipe, ctx->tuning_version, ctx->force_shape};
   if (ctx->graph_key != key || ctx->graph_exec == nullptr) {
     if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
@@ -1237,7 +1297,7 @@ int GraphLoop(mpsft_ctx *ctx, const mpsft_signal *const *sigs,
       per_body = 1;
       const Ahead ah{d_its_ahead, ctx->d_solve_ctl, ph.plan_max};
       rc = LaunchIterationKernels(ctx, d_its, nsig, ph.shape, x_c128, fp64,
-                                  any_forced, nullptr, &per_body, ctx->cap,
+                                  forced, nullptr, &per_body, ctx->cap,
                                   ph.pipelined ? &ah : nullptr);
       cudaError_t we = cudaSuccess;
       if (ph.pipelined) {
@@ -1532,15 +1592,17 @@ int SolveMany(mpsft_ctx *ctx, const mpsft_signal *const *sigs,
   }
   // precision policy, once per solve (FP32 calls)
   std::vector<int32_t> force(nsig, 0);
-  bool any_forced = false;
+  int n_forced = 0;
   for (int i = 0; i < nsig; ++i) {
     const mpsft_solve_options &o = opts[i];
     const int32_t b0 = shapes[i].bins_cap;
     force[i] = !fp64 && PolicyForcesFP64(o.near_tie_margin, b0, energy[i],
                                          3.0 * o.sigma / std::sqrt(double(b0)),
                                          o.sigma / std::sqrt(double(b0)));
-    any_forced |= force[i] != 0;
+    n_forced += force[i] != 0;
   }
+  const Forced forced =
+      n_forced == 0 ? kNoneForced : (n_forced < nsig ? kSomeForced : kAllForced);
   struct Run {
     int32_t iter = 0, stale = 0, found = 0, status = MPSFT_OK;
     bool done = false;
@@ -1585,7 +1647,7 @@ int SolveMany(mpsft_ctx *ctx, const mpsft_signal *const *sigs,
   std::vector<SolveCtl> h_ctl;
   if (!host_loop) {
     rc = GraphLoop(ctx, sigs, opts, nsig, rngs, shapes, d_its, d_its_ahead, &its, &draws,
-                   force, any_forced, fp64, x_c128, &launches, rs, &h_ctl);
+                   force, forced, fp64, x_c128, &launches, rs, &h_ctl);
     if (rc == kGraphUnavailable) {
       // no iteration ran and the tables are untouched; the RNGs are back
       // where they were
@@ -1654,9 +1716,9 @@ int SolveMany(mpsft_ctx *ctx, const mpsft_signal *const *sigs,
       SetNearTie(&it, fp64, o.near_tie_margin, bins, force[i] != 0);
       run[i].fp64_iters += it.force_fp64;
       // same bins as the last iteration: window and Bluestein tables stand
-      // (a forced FP64 iteration leaves the FP32 tables unbuilt)
-      it.tables_valid = (run[i].last_bins == bins && !it.force_fp64) ? 1 : 0;
-      run[i].last_bins = it.force_fp64 ? -1 : bins;
+      // (FP64 ones in every iteration of a forced signal, FP32 ones otherwise)
+      it.tables_valid = run[i].last_bins == bins ? 1 : 0;
+      run[i].last_bins = bins;
       run[i].gathers += BinGathers(it, fp64 || it.force_fp64);
       run[i].bin_bytes += BinBytes(it, fp64 || it.force_fp64);
       mpsft_bin_launch &r = rec[it.force_fp64 ? 1 : 0];

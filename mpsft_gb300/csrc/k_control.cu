@@ -158,7 +158,8 @@ __global__ void k_plan(SolveCtl *__restrict__ ctl, SigIter *__restrict__ its,
     it.tables_valid = build ? 0 : 1;
     if (build) it.win_slot = h;
   } else {
-    it.tables_valid = (c.last_bins == bins && !c.force_fp64) ? 1 : 0;
+    // (a signal is forced to FP64 throughout a solve or never)
+    it.tables_valid = c.last_bins == bins ? 1 : 0;
   }
   if (!ahead) {
     it.flags[0] = 0;
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(1024)
         c.status = kSolveIterCap;
       }
       if (c.status != 0 || c.stale >= c.max_stale) c.done = 1;
-      c.last_bins = it.force_fp64 ? -1 : it.bins;
+      c.last_bins = it.bins;
       // the tables this signal built are complete (every table kernel of
       // the iteration has run)
       if (it.win_slot >= 0) c.win_valid[it.win_slot] = 1;

@@ -79,9 +79,9 @@ __global__ void k_mode_prep(const SigIter *__restrict__ its, int cond) {
   const SigIter &it = its[blockIdx.y];
   if (!it.active) return;
   if (cond && !RedoFP64(it)) return;
-  // a few blocks per signal striding over the occupied slots (a grid over
-  // the whole table would flood the SMs with empty blocks at the start of
-  // every iteration, ahead of the other streams' kernels)
+  // a bounded number of blocks per signal striding over the occupied slots (a
+  // grid over the whole table would flood the SMs with empty blocks at the
+  // start of every iteration, ahead of the other streams' kernels)
   const int count = *it.tab_count;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count;
        i += gridDim.x * blockDim.x) {
@@ -639,10 +639,12 @@ void LaunchExportTables(const SigIter *d_its, int nsig, int max_cap,
 
 void LaunchModePrep(const SigIter *d_its, int nsig, int max_cap, cudaStream_t s,
                     bool cond) {
-  // the occupied count is only known on the device: up to 8 blocks per
-  // signal stride over it (a table holds at most max_cap / 2 entries)
-  dim3 grid(std::min(8, std::max(1, max_cap / 2 / 256)), nsig);
-  Launch(k_mode_prep, grid, 256, 0, s, d_its, cond ? 1 : 0);
+  // the occupied count is only known on the device: up to 32 blocks per
+  // signal stride over it (a table holds at most max_cap / 2 entries). Small
+  // blocks: a mode's two FP64 erf bind its SM's FP64 pipes, so one signal's
+  // modes have to spread over many SMs
+  dim3 grid(std::min(32, std::max(1, max_cap / 2 / 64)), nsig);
+  Launch(k_mode_prep, grid, 64, 0, s, d_its, cond ? 1 : 0);
 }
 
 // Shared memory of k_bucket: the keys, then two ints per bin.
@@ -698,8 +700,10 @@ void LaunchListedTerms(const SigIter *d_its, int nsig, int max_trials, cudaStrea
 
 void LaunchMerge(const SigIter *d_its, int nsig, int max_bins,
                  cudaStream_t s) {
-  dim3 grid((max_bins + 255) / 256, nsig);
-  Launch(k_merge, grid, 256, 0, s, d_its);
+  // a warp per block: a candidate's two FP64 erf and its division bind the
+  // SM's FP64 pipes (1001 bins of one signal: 19 us on 4 SMs of 256 threads)
+  dim3 grid((max_bins + 31) / 32, nsig);
+  Launch(k_merge, grid, 32, 0, s, d_its);
 }
 
 void LaunchInsertSpills(const SigIter *d_its, int nsig, cudaStream_t s) {

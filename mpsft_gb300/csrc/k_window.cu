@@ -204,7 +204,12 @@ __global__ void __launch_bounds__(512)
   V *a = reinterpret_cast<V *>(smem_raw);
   const SigIter &it = its[blockIdx.x];
   if (!it.active) return;
-  if (cond ? !RedoFP64(it) : (it.force_fp64 || it.tables_valid)) return;
+  // (tables_valid: the FP64 tables of a signal forced to FP64 in every
+  // iteration; of another signal redone in FP64, its FP32 tables)
+  if (cond ? (!RedoFP64(it) || (it.force_fp64 && it.tables_valid))
+           : (it.force_fp64 || it.tables_valid)) {
+    return;
+  }
   const int B = it.bins, M = it.fft_m;
   V *chirp = ChirpOf(it, (V *)nullptr);
   V *chat = ChatOf(it, (V *)nullptr);
