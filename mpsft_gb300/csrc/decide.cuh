@@ -263,23 +263,10 @@ __device__ __forceinline__ int DecideTail(const SigIter &it, int beta, int mode,
   const uint32_t mask = __ballot_sync(0xffffffffu, has_bit && count > TR / 2);
   // bit 0 is the most significant digit of xi
   const uint32_t xs = L > 0 ? (__brev(mask) >> (32 - L)) : 0u;
-  // the FP32 path (also in its FP64 kernels) leaves pending candidates that
-  // the merge finishes on full warps; the FP64 path finishes them here
-  const bool pending = fp32 || it.eps_rel > 0.f;
-  int64_t k1;
-  double wf = 0.0;
-  if (pending) {
-    k1 = RoundK1(n, beta, xs, L, B, it.psi);
-  } else {
-    const double xi1 = ldexp(2.0 * double(xs) + 1.0, -(L + 1));
-    k1 = int64_t(round(double(n) * (double(beta) + xi1) / double(B)));
-    const double xi0 = double(k1) / double(n) - (double(beta) + 0.5) / double(B);
-    wf = WindowInFreq(it, xi0);
-    if (fabs(wf) < it.win_thr) {
-      NoCandidate(it, beta, lane);
-      return listed;
-    }
-  }
+  // (the window response at k1, its threshold, the division and k0 follow in
+  // the merge, one thread per bin: here every FP64 operation of them would
+  // occupy a whole warp's slot)
+  const int64_t k1 = RoundK1(n, beta, xs, L, B, it.psi);
 
   // ---- coefficient (src/iterate.cc:146-171)
   V fac_t[TMAX];
@@ -375,38 +362,141 @@ __device__ __forceinline__ int DecideTail(const SigIter &it, int beta, int mode,
     for (int o = 16; o > 0; o >>= 1) e = fmaxf(e, __shfl_xor_sync(0xffffffffu, e, o));
     err = double(e);
   }
-  if (pending) {
-    if (lane == 0) {
-      it.cand_k0[beta] = int32_t(k1);
-      it.cand_coef[beta] = make_double2(double(ax), double(ay));
-      it.cand_err[beta] = err;
-      it.cand_valid[beta] = 2;
-    }
-    return listed;
-  }
   if (lane == 0) {
-    double2 coef = make_double2(double(ax) / double(TR * (1 + 2 * L)),
-                                double(ay) / double(TR * (1 + 2 * L)));
-    const ModN mod{uint32_t(n), it.n_inv};
-    const int32_t k0 = int32_t(mod(int64_t(it.a_inv) * mod(k1 - it.b)));
-    coef = cmul(coef, Phase64(it, -int64_t(it.c) * k0));
-    coef = make_double2(coef.x / wf, coef.y / wf);
-    it.cand_k0[beta] = k0;
-    it.cand_coef[beta] = coef;
-    it.cand_err[beta] = 0.0;
-    it.cand_valid[beta] = 1;
-    it.flags[0] = 1;
+    it.cand_k0[beta] = int32_t(k1);
+    it.cand_coef[beta] = make_double2(double(ax), double(ay));
+    it.cand_err[beta] = err;
+    it.cand_valid[beta] = 2;
   }
   return listed;
 }
 
+// FP64 subtraction of a bin's found modes (in increasing k0), by one warp.
+// GB300's schedulers take 64 cycles per FP64 warp instruction, so these
+// instructions are what the subtraction costs: with many modes in a bin (40 at
+// 2000 modes in 51 bins) most of an FP64 iteration's decisions.
+//
+// Both take trials [t0, min(t0 + TMAX, trials)) (u0, up, um start at t0), so
+// that many trials go in groups that fit the registers, with the same sums.
+//
+// Row 0: the modes' terms summed, a mode per lane, by shuffles.
+template <int TMAX>
+__device__ __forceinline__ void SubtractRow0(const SigIter &it, int nm, int st, int t0,
+                                             double2 *u0) {
+  const int lane = threadIdx.x & 31, TR = it.trials - t0;
+  double2 sum[TMAX];
+#pragma unroll
+  for (int t = 0; t < TMAX; ++t) sum[t] = make_double2(0.0, 0.0);
+  for (int i = lane; i < nm; i += 32) {
+    const int sl = it.bkt_list[st + i];
+#pragma unroll
+    for (int t = 0; t < TMAX; ++t) {
+      if (t < TR) sum[t] = cadd(sum[t], it.mode_base[size_t(sl) * it.trials + t0 + t]);
+    }
+  }
+  // the lanes that hold a mode: a power of two of them
+  const int width = nm >= 32 ? 32 : (nm <= 1 ? 1 : 1 << (32 - __clz(nm - 1)));
+  for (int o = width >> 1; o > 0; o >>= 1) {
+#pragma unroll
+    for (int t = 0; t < TMAX; ++t) {
+      if (t < TR) {
+        sum[t].x += __shfl_xor_sync(0xffffffffu, sum[t].x, o);
+        sum[t].y += __shfl_xor_sync(0xffffffffu, sum[t].y, o);
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < TMAX; ++t) {
+    if (t < TR) {
+      u0[t].x -= __shfl_sync(0xffffffffu, sum[t].x, 0);
+      u0[t].y -= __shfl_sync(0xffffffffu, sum[t].y, 0);
+    }
+  }
+}
+
+// The rows 2s+1, 2s+2 of bit s (up, um of lane s): the modes' terms times the
+// row factor e^{+-2 pi i (B 2^s k1 mod n)/n} (src/binner.cc:584-589). Both
+// rows take the same four sums of products of term and factor, four multiply-adds
+// per mode; up to 16 bits, each half of the warp takes every second mode.
+// kBatch modes' loads are issued together.
+template <int TMAX>
+__device__ __forceinline__ void SubtractRows(const SigIter &it, int nm, int st, int t0,
+                                             double2 *up, double2 *um) {
+  constexpr int kBatch = TMAX == 1 ? 4 : 2;
+  const int lane = threadIdx.x & 31, TR = it.trials - t0;
+  const bool halves = it.bits <= 16;
+  const int s = halves ? lane & 15 : lane, h = halves ? lane >> 4 : 0;
+  const int step = halves ? 2 : 1;
+  const int64_t off = s < it.bits ? int64_t(it.bins) << s : 0;
+  const ModN mod{uint32_t(it.n), it.n_inv};
+  const uint32_t lo_mask = (1u << it.ph_k) - 1u;
+  double rr[TMAX], ii[TMAX], ri[TMAX], ir[TMAX];
+#pragma unroll
+  for (int t = 0; t < TMAX; ++t) rr[t] = ii[t] = ri[t] = ir[t] = 0.0;
+  for (int i0 = h; i0 < nm; i0 += kBatch * step) {
+    int sl[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int i = i0 + u * step;
+      sl[u] = it.bkt_list[st + (i < nm ? i : i0)];
+    }
+    double2 bs[kBatch][TMAX], hi[kBatch], lo[kBatch];
+    int64_t k1[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      k1[u] = it.mode_k1[sl[u]];
+#pragma unroll
+      for (int t = 0; t < TMAX; ++t) {
+        if (t < TR) bs[u][t] = it.mode_base[size_t(sl[u]) * it.trials + t0 + t];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const uint32_t r = mod(off * k1[u]);
+      hi[u] = it.ph_hi[r >> it.ph_k];
+      lo[u] = it.ph_lo[r & lo_mask];
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      if (i0 + u * step < nm) {
+        const double2 f = cmul(hi[u], lo[u]);
+#pragma unroll
+        for (int t = 0; t < TMAX; ++t) {
+          if (t < TR) {
+            rr[t] = fma(bs[u][t].x, f.x, rr[t]);
+            ii[t] = fma(bs[u][t].y, f.y, ii[t]);
+            ri[t] = fma(bs[u][t].x, f.y, ri[t]);
+            ir[t] = fma(bs[u][t].y, f.x, ir[t]);
+          }
+        }
+      }
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < TMAX; ++t) {
+    if (t < TR) {
+      if (halves) {
+        rr[t] += __shfl_xor_sync(0xffffffffu, rr[t], 16);
+        ii[t] += __shfl_xor_sync(0xffffffffu, ii[t], 16);
+        ri[t] += __shfl_xor_sync(0xffffffffu, ri[t], 16);
+        ir[t] += __shfl_xor_sync(0xffffffffu, ir[t], 16);
+      }
+      if (lane < it.bits) {
+        up[t] = make_double2(up[t].x - (rr[t] - ii[t]), up[t].y - (ri[t] + ir[t]));
+        um[t] = make_double2(um[t].x - (rr[t] + ii[t]), um[t].y - (ir[t] - ri[t]));
+      }
+    }
+  }
+}
+
 // The bin loop body of Iterate for one bin (warp-wide). T = float: the FP32
 // path with near-tie detection, FP32 arithmetic only (GB300 runs FP64 at a
-// small fraction of its FP32 rate): a surviving bin leaves a pending
-// candidate (cand_valid = 2: k1 in cand_k0, the unscaled coefficient sum in
-// cand_coef, its error bound in cand_err) that the merge finishes in FP64 on
-// full warps. T = double: FP64 decisions to the end (the FP64 path, and the
-// near-tie bins after their re-binning).
+// small fraction of its FP32 rate). T = double: FP64 decisions (the FP64 path,
+// and the near-tie bins after their re-binning). A surviving bin leaves a
+// pending candidate (cand_valid = 2: k1 in cand_k0, the unscaled coefficient
+// sum in cand_coef, its error bound in cand_err) that the merge finishes in
+// FP64 on full warps.
 template <typename T, int TMAX, typename Src>
 __device__ int DecideBin(const SigIter &it, int beta, const Src &src,
                           int mode) {
@@ -429,7 +519,18 @@ __device__ int DecideBin(const SigIter &it, int beta, const Src &src,
   for (int t = 0; t < TMAX; ++t) {
     if (t < TR) u0[t] = O::from(src.get(t, 0));
   }
-  const int npre = min(nm, 32);
+  // FP64: its own subtraction, up to five trials at a time
+  constexpr bool kSums = sizeof(T) == 8;
+  constexpr int kGroup = TMAX < 5 ? TMAX : 5;
+  const int npre = kSums ? 0 : min(nm, 32);
+  if constexpr (kSums) {
+    if (nm > 0) {
+#pragma unroll
+      for (int t0 = 0; t0 < TMAX; t0 += kGroup) {
+        if (t0 < TR) SubtractRow0<kGroup>(it, nm, st, t0, u0 + t0);
+      }
+    }
+  }
   V pre_base[TMAX];
   float mode_err = 0.f;  // FP32 error carried into this bin by the found modes
   int pre_k1 = 0;  // k1 of the lane's mode (row factors below)
@@ -439,7 +540,7 @@ __device__ int DecideBin(const SigIter &it, int beta, const Src &src,
     pre_k1 = it.mode_k1[sl];
     if (fp32) mode_err = it.mode_errw[sl];
   }
-  for (int i = 0; i < nm; ++i) {
+  for (int i = 0; i < (kSums ? 0 : nm); ++i) {
     V bs[TMAX];
     if (i < 32) {
 #pragma unroll
@@ -544,7 +645,15 @@ __device__ int DecideBin(const SigIter &it, int beta, const Src &src,
   // four modes at a time: their row factors e^{2 pi i (B 2^s k1 mod n)/n}
   // (src/binner.cc:584-589) are evaluated side by side, then subtracted in
   // the bin's mode order
-  for (int i0 = 0; i0 < nm; i0 += 4) {
+  if constexpr (kSums) {
+    if (nm > 0) {
+#pragma unroll
+      for (int t0 = 0; t0 < TMAX; t0 += kGroup) {
+        if (t0 < TR) SubtractRows<kGroup>(it, nm, st, t0, up + t0, um + t0);
+      }
+    }
+  }
+  for (int i0 = 0; i0 < (kSums ? 0 : nm); i0 += 4) {
     V fac[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {

@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 && TMAX == 1) ? 6 : 1)
   const SigIter &it = its[blockIdx.y];
   if (!it.active) return;
   if (cond ? !RedoFP64(it) : it.force_fp64) return;
-  const int beta = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int beta = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (beta >= it.bins) return;
   int e;
   if constexpr (sizeof(T) == sizeof(float)) {
@@ -431,8 +431,8 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------------------------------------------------------- merge
-// Candidate of bin beta -> table. A pending FP32 candidate is finished here
-// in FP64 (src/iterate.cc:139-171): the window response at
+// Candidate of bin beta -> table. A pending candidate is finished here in
+// FP64 (src/iterate.cc:139-171): the window response at
 // xi0 = k1/n - (beta + 1/2)/B and its threshold, the average over the
 // T (1 + 2L) values, k0 = a^-1 (k1 - b) mod n, the factor e^{-2 pi i c k0/n}
 // and the division by the window response.
@@ -604,8 +604,12 @@ __global__ void __launch_bounds__(1024)
 template <typename T, int TMAX>
 void LaunchDecideT(const SigIter *d_its, int nsig, int max_bins, int mode,
                    int cond, int mark, cudaStream_t s) {
-  dim3 grid((max_bins + 7) / 8, nsig);
-  Launch(k_decide<T, TMAX>, grid, 256, 0, s, d_its, mode, cond, mark);
+  // eight bins per block; FP64 with few bins one, so that they spread over
+  // every SM's FP64 pipes (101 bins of one signal in three trials: 28 us in 13
+  // blocks of eight, 21 us in blocks of one)
+  const int w = sizeof(T) == 8 && int64_t(max_bins) * nsig <= 152 * 16 ? 1 : 8;
+  dim3 grid((max_bins + w - 1) / w, nsig);
+  Launch(k_decide<T, TMAX>, grid, 32 * w, 0, s, d_its, mode, cond, mark);
 }
 
 template <typename T>

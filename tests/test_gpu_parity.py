@@ -670,3 +670,19 @@ def test_row_transform_sizes(ctx, port, bins, bits):
         u = ctx.bin_in_time(sig, bins, bits, 1e-5, a, b, c, q, precision=prec)
         assert rel_err(u, want) < TOL_BINS[prec]
     sig.free()
+
+
+@pytest.mark.parametrize("bits", [0, 9, 16, 17])
+@pytest.mark.parametrize("count", [1, 2, 3, 8, 9, 31, 32, 33, 65])
+def test_bin_in_freq_modes_per_bin(ctx, port, count, bits):
+    """FP64 subtraction with every mode in one bin: fewer and more modes than
+    a warp's lanes and than a half-warp's batches, bits in both halves of the
+    warp and beyond, against the oracle (1e-12 of max|U|, as above)."""
+    n, bins = 1 << 20, 3
+    rng = np.random.default_rng(count)
+    k = rng.choice(n // 3 - 2, count, replace=False).astype(np.int32)
+    coef = rng.standard_normal(count) + 1j * rng.standard_normal(count)
+    u = rng.standard_normal((1 + 2 * bits, bins)) * (1 + 0.5j)
+    got = ctx.bin_in_freq(u, n, bins, bits, 1e-5, 1, 0, 77, 991, k, coef)
+    want = port.bin_in_freq(u, n, bins, bits, 1e-5, 1, 0, 77, 991, k, coef)
+    assert rel_err(got, want) < 1e-12
