@@ -467,7 +467,8 @@ class Context:
     def bin_in_time(self, sig: "Signal", bins: int, bits: int, delta: float,
                     a: int, b: int, c: int, q: int,
                     precision: int = FP32) -> np.ndarray:
-        out = np.zeros((1 + 2 * bits, bins), np.complex128)
+        # (the call fills every element; fresh zeroed pages cost as much as it)
+        out = np.empty((1 + 2 * bits, bins), np.complex128)
         _check(self, self._lib.mpsft_bin_in_time(
             self._h, sig._h, bins, bits, delta, a, b, c, q, precision, _ptr(out), 0))
         return out
@@ -478,7 +479,7 @@ class Context:
         """BinInTime::Run windowed by a Window's own table wt (p entries, the
         reference's index order t = 0, 1..p2, -p2..-1)."""
         wt = np.ascontiguousarray(wt, np.float64)
-        out = np.zeros((1 + 2 * bits, bins), np.complex128)
+        out = np.empty((1 + 2 * bits, bins), np.complex128)
         _check(self, self._lib.mpsft_bin_in_time_wt(
             self._h, sig._h, bins, bits, wt.size, _ptr(wt), a, b, c, q, precision,
             _ptr(out), 0))
@@ -524,7 +525,7 @@ class Context:
                  k0: np.ndarray) -> np.ndarray:
         """Coefficient estimate of the fixed set k0 (a linear map of x)."""
         k0 = np.ascontiguousarray(k0, np.int32)
-        out = np.zeros(k0.size, np.complex128)
+        out = np.empty(k0.size, np.complex128)
         _check(self, self._lib.mpsft_estimate(self._h, sig._h, ctypes.byref(setup),
                                               _ptr(k0), k0.size, _ptr(out)))
         return out
@@ -534,7 +535,7 @@ class Context:
         """A^H g for the estimate of k0 (complex128, n entries)."""
         k0 = np.ascontiguousarray(k0, np.int32)
         g = np.ascontiguousarray(g, np.complex128)
-        out = np.zeros(n, np.complex128)
+        out = np.empty(n, np.complex128)
         _check(self, self._lib.mpsft_adjoint(self._h, n, ctypes.byref(setup),
                                              _ptr(k0), k0.size, _ptr(g), _ptr(out)))
         return out

@@ -552,6 +552,133 @@ int EnsureWinCache(mpsft_ctx *ctx, double delta, int32_t bmin, int32_t bmax,
   return MPSFT_OK;
 }
 
+// ---- tables of the single-signal calls --------------------------------
+// The window, Bluestein and unit-phase tables of a bins, estimate or Iterate
+// call depend on the bins, the window delta and n alone; a caller makes many
+// calls with the same ones (every trial of the reference's Iterate, every
+// iteration at min_bins), so the context keeps them: at most kTableMax tables
+// and kTableBudget bytes. A table is handed out as built only after the call
+// that built it has completed (CommitTables after its last wait), so neither
+// an error in between nor another stream sees it unfinished. Building them took
+// 16 us of a 501-bin FP32 call's 88, 108 us of an 8001-bin one's 341.
+enum TableKind {
+  kTabBlue32,       // chirp32, chat32
+  kTabBlue32Roots,  // chirp32, chat32, r2b64
+  kTabBlue64,       // chirp64, chat64
+  kTabWin32,        // wt32
+  kTabWin64,        // wt64
+  kTabWinFF,        // wt64, wtff
+  kTabPhase,        // ph_lo, ph_hi
+};
+constexpr size_t kTableBudget = size_t(64) << 20;
+constexpr size_t kTableMax = 64;
+
+void BeginTables(mpsft_ctx *ctx) { ++ctx->table_call; }
+void CommitTables(mpsft_ctx *ctx) {
+  for (mpsft_ctx::Table &e : ctx->tables) {
+    if (e.used == ctx->table_call) e.built = true;
+  }
+}
+
+void DropTable(mpsft_ctx *ctx, size_t i) {
+  cudaFree(ctx->tables[i].ptr);
+  ctx->table_bytes -= ctx->tables[i].bytes;
+  ctx->tables.erase(ctx->tables.begin() + i);
+}
+
+// The context's table of this kind and key, and whether this call has to build
+// it; null when it does not fit (the caller then builds into its own buffers).
+unsigned char *CtxTable(mpsft_ctx *ctx, int kind, int32_t bins, int64_t n, double delta,
+                        size_t bytes, bool *build) {
+  for (mpsft_ctx::Table &e : ctx->tables) {
+    if (e.kind == kind && e.bins == bins && e.n == n && e.delta == delta) {
+      *build = !e.built;
+      e.used = ctx->table_call;
+      return e.ptr;
+    }
+  }
+  *build = true;
+  if (bytes > kTableBudget) return nullptr;
+  while (ctx->tables.size() >= kTableMax || ctx->table_bytes + bytes > kTableBudget) {
+    size_t old = 0;
+    for (size_t i = 1; i < ctx->tables.size(); ++i) {
+      if (ctx->tables[i].used < ctx->tables[old].used) old = i;
+    }
+    if (ctx->tables[old].used == ctx->table_call) return nullptr;  // all of this call
+    DropTable(ctx, old);  // (every call waits for its kernels before it returns)
+  }
+  void *p = nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  ctx->tables.push_back({kind, bins, n, delta, static_cast<unsigned char *>(p), bytes,
+                         ctx->table_call, false});
+  ctx->table_bytes += bytes;
+  return static_cast<unsigned char *>(p);
+}
+
+// Bluestein tables of it->bins; returns whether they are to be built.
+bool UseBluestein(mpsft_ctx *ctx, SigIter *it, bool fp64, bool roots) {
+  bool build = true;
+  const size_t B = size_t(it->bins), M = size_t(it->fft_m);
+  Carve cv{nullptr};
+  if (fp64) {
+    cv.take<double2>(B), cv.take<double2>(M);
+    cv.base = CtxTable(ctx, kTabBlue64, it->bins, 0, 0.0, cv.off, &build);
+    if (cv.base == nullptr) return true;
+    cv.off = 0;
+    it->chirp64 = cv.take<double2>(B);
+    it->chat64 = cv.take<double2>(M);
+    return build;
+  }
+  cv.take<float2>(B), cv.take<float2>(M), cv.take<double2>(roots ? 2 * B : 0);
+  cv.base = CtxTable(ctx, roots ? kTabBlue32Roots : kTabBlue32, it->bins, 0, 0.0, cv.off,
+                     &build);
+  if (cv.base == nullptr) return true;
+  cv.off = 0;
+  it->chirp32 = cv.take<float2>(B);
+  it->chat32 = cv.take<float2>(M);
+  if (roots) it->r2b64 = cv.take<double2>(2 * B);
+  return build;
+}
+
+// Window tables of (it->bins, delta): kind kTabWin32, kTabWin64 or kTabWinFF.
+bool UseWindow(mpsft_ctx *ctx, SigIter *it, double delta, TableKind kind) {
+  bool build = true;
+  const size_t e = size_t(it->p2) + 1;
+  Carve cv{nullptr};
+  if (kind == kTabWin32) {
+    cv.take<float>(e);
+  } else {
+    cv.take<double>(e), cv.take<float2>(kind == kTabWinFF ? e : 0);
+  }
+  cv.base = CtxTable(ctx, kind, it->bins, 0, delta, cv.off, &build);
+  if (cv.base == nullptr) return true;
+  cv.off = 0;
+  if (kind == kTabWin32) {
+    it->wt32 = cv.take<float>(e);
+    return build;
+  }
+  it->wt64 = cv.take<double>(e);
+  if (kind == kTabWinFF) it->wtff = cv.take<float2>(e);
+  return build;
+}
+
+// FP64 unit-phase tables of it->n.
+bool UsePhases(mpsft_ctx *ctx, SigIter *it) {
+  bool build = true;
+  const size_t lo = size_t(1) << PhaseTableK(it->n), hi = size_t(PhaseTableHi(it->n));
+  Carve cv{nullptr};
+  cv.take<double2>(lo), cv.take<double2>(hi);
+  cv.base = CtxTable(ctx, kTabPhase, 0, it->n, 0.0, cv.off, &build);
+  if (cv.base == nullptr) return true;
+  cv.off = 0;
+  it->ph_lo = cv.take<double2>(lo);
+  it->ph_hi = cv.take<double2>(hi);
+  return build;
+}
+
 int32_t NextPow2(int64_t v) {
   int32_t p = 1;
   while (p < v) p <<= 1;
@@ -736,7 +863,8 @@ Maxima MaximaOf(const std::vector<SigIter> &h_its) {
 }
 
 // The kernels of one iteration of every active signal, on stream s (and the
-// context's side stream, forked from and joined back into s).
+// context's side stream, forked from and joined back into s). tables: the
+// window and Bluestein tables are in place (CtxTable).
 // The fixed-bins phase's pipelined body: while this iteration decides, the
 // next one (descriptors its_ahead) is planned and gathered/folded on the
 // prefold stream, into the second fold buffer (only this iteration's row FFT
@@ -753,7 +881,7 @@ struct Ahead {
 // the other: about 100 us of every iteration of a batch of 24 signals.
 int LaunchForcedIteration(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
                           const Maxima &mx, bool x_c128, BinTimer *timer,
-                          int64_t *launched, cudaStream_t s) {
+                          int64_t *launched, cudaStream_t s, bool tables) {
   // side stream: mode preparation and bucketing (the decisions wait for them);
   // low-priority stream: the Bluestein tables (the row transforms do)
   MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_fork, s));
@@ -762,9 +890,11 @@ int LaunchForcedIteration(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   LaunchBucket(d_its, nsig, mx.bins, mx.cap, ctx->side, false);
   MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_join, ctx->side));
   MPSFT_CUDA(ctx, cudaStreamWaitEvent(ctx->side64, ctx->ev_fork, 0));
-  LaunchBluesteinSetup(d_its, nsig, mx.m, true, ctx->tw32, ctx->tw64, ctx->side64, true);
+  if (!tables) {
+    LaunchBluesteinSetup(d_its, nsig, mx.m, true, ctx->tw32, ctx->tw64, ctx->side64, true);
+  }
   MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_blue, ctx->side64));
-  LaunchWindow64(d_its, nsig, mx.p2, s);
+  if (!tables) LaunchWindow64(d_its, nsig, mx.p2, s);
   LaunchWindowMod(d_its, nsig, mx.bins, false, true, s);
   if (timer) {
     // (tag 0: the iteration's FP32 binning, which has no signal)
@@ -790,7 +920,7 @@ int LaunchForcedIteration(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join, 0));
   LaunchDecide(d_its, nsig, mx.bins, mx.trials, false, false, s, true);
   LaunchMerge(d_its, nsig, mx.bins, s);
-  if (launched) *launched += 9;
+  if (launched) *launched += tables ? 7 : 9;
   MPSFT_CUDA(ctx, cudaGetLastError());
   return MPSFT_OK;
 }
@@ -802,10 +932,11 @@ enum Forced { kNoneForced = 0, kSomeForced = 1, kAllForced = 2 };
 int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
                            const Maxima &mx, bool x_c128, bool fp64,
                            Forced forced, BinTimer *timer, int64_t *launched,
-                           cudaStream_t s, const Ahead *ahead = nullptr) {
+                           cudaStream_t s, const Ahead *ahead = nullptr,
+                           bool tables = false) {
   if (mx.bins == 0) return MPSFT_OK;
   if (forced == kAllForced && !fp64 && mx.m <= kMaxFFT64) {
-    return LaunchForcedIteration(ctx, d_its, nsig, mx, x_c128, timer, launched, s);
+    return LaunchForcedIteration(ctx, d_its, nsig, mx, x_c128, timer, launched, s, tables);
   }
   const bool any_forced = forced != kNoneForced;
   // fork: tables, mode preparation and bucketing on the side stream while
@@ -831,7 +962,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
                                nsig, x_c128));
     MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_join_p, ctx->pre));
   }
-  if (!ahead) {
+  if (!ahead && !tables) {
     LaunchBluesteinSetup(d_its, nsig, mx.m, fp64, ctx->tw32, ctx->tw64, ctx->side);
     MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_blue, ctx->side));
   }
@@ -841,15 +972,15 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   // FP32 path: the FP64 window tables (for the near-tie re-binning and the
   // FP64 kernels) are built on the low-priority stream and joined only
   // before the re-binning; the binning uses an FP32 evaluation
-  if (!fp64) {
+  if (!fp64 && !tables) {
     MPSFT_CUDA(ctx, cudaStreamWaitEvent(ctx->side64, ctx->ev_fork, 0));
     LaunchWindow64(d_its, nsig, mx.p2, ctx->side64);
     MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_join64, ctx->side64));
   }
   if (fp64) {
-    LaunchWindow(d_its, nsig, mx.p2, s);
+    if (!tables) LaunchWindow(d_its, nsig, mx.p2, s);
     LaunchWindowMod(d_its, nsig, mx.bins, false, false, s);
-  } else if (!ahead) {
+  } else if (!ahead && !tables) {
     LaunchWindow32(d_its, nsig, mx.p2, s);
   }
   if (timer && ctx->profiling) {
@@ -857,7 +988,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
     // first), and its launch enqueued while a short delay kernel holds the
     // stream, so that its events time the kernel, not a host launch gap
     MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join, 0));
-    if (!fp64) MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join64, 0));
+    if (!fp64 && !tables) MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join64, 0));
     LaunchDelay(20000, s);
   }
   if (timer) {
@@ -874,7 +1005,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
     int rc = timer->End();
     if (rc) return rc;
   }
-  if (!ahead) MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_blue, 0));
+  if (!ahead && !tables) MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_blue, 0));
   LaunchRowFFT(d_its, nsig, mx.rows, mx.trials, mx.m, fp64, ctx->tw32, ctx->tw64,
                s);
   MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join, 0));  // join
@@ -890,7 +1021,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   // decide (ahead: the next iteration's plan and fold, bucketing, FP64
   // window, FFT, decide)
   // FP64: the modulated window instead of the second window table
-  if (launched) *launched += ahead ? 6 : 7;
+  if (launched) *launched += ahead ? 6 : (tables ? (fp64 ? 5 : 4) : 7);
   if (!fp64) {
     // side stream: the listed bins' FP64 mode terms (before any merge
     // changes a coefficient), then the merge of the other bins, beside the
@@ -903,7 +1034,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
       LaunchMerge(d_its, nsig, mx.bins, ctx->side);
       MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_join_m, ctx->side));
     }
-    MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join64, 0));
+    if (!tables) MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join64, 0));
     LaunchRebin(d_its, nsig, kMaxListed, x_c128, false, s);
     MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join_l, 0));
     LaunchDecideListed(d_its, nsig, mx.trials, redo, side_merge, s);
@@ -942,7 +1073,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
 int LaunchIteration(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
                     const std::vector<SigIter> &h_its, bool x_c128, bool fp64,
                     BinTimer *timer, int64_t *launched = nullptr,
-                    int32_t tune_bins = 0) {
+                    int32_t tune_bins = 0, bool tables = false) {
   int active = 0, forced = 0;
   for (const SigIter &it : h_its) {
     active += it.active;
@@ -953,49 +1084,12 @@ int LaunchIteration(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   const int rc = LaunchIterationKernels(
       ctx, d_its, nsig, mx, x_c128, fp64,
       forced == 0 ? kNoneForced : (forced < active ? kSomeForced : kAllForced), timer,
-      launched, ctx->stream);
+      launched, ctx->stream, nullptr, tables);
   if (rc != MPSFT_OK) return rc;
   // (in the solve graph, k_finish inserts the spilled candidates)
   LaunchInsertSpills(d_its, nsig, ctx->stream);
   if (launched) *launched += 1;
   MPSFT_CUDA(ctx, cudaGetLastError());
-  return MPSFT_OK;
-}
-
-struct ModeOut {
-  std::vector<std::pair<int32_t, double2>> modes;
-};
-
-int DownloadTable(mpsft_ctx *ctx, const SigIter &it,
-                  std::vector<std::pair<int32_t, double2>> *out) {
-  std::vector<int32_t> keys(it.tab_cap);
-  std::vector<double2> coefs(it.tab_cap);
-  MPSFT_CUDA(ctx, cudaMemcpyAsync(keys.data(), it.tab_key,
-                                  sizeof(int32_t) * it.tab_cap,
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-  MPSFT_CUDA(ctx, cudaMemcpyAsync(coefs.data(), it.tab_coef,
-                                  sizeof(double2) * it.tab_cap,
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-  MPSFT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  out->clear();
-  for (int i = 0; i < it.tab_cap; ++i) {
-    if (keys[i] != kEmptyKey) out->emplace_back(keys[i], coefs[i]);
-  }
-  std::sort(out->begin(), out->end(),
-            [](const std::pair<int32_t, double2> &l,
-               const std::pair<int32_t, double2> &r) { return l.first < r.first; });
-  return MPSFT_OK;
-}
-
-int ClearTable(mpsft_ctx *ctx, const SigIter &it, int32_t *ctl) {
-  MPSFT_CUDA(ctx, cudaMemsetAsync(it.tab_key, 0xFF,
-                                  sizeof(int32_t) * it.tab_cap, ctx->stream));
-  MPSFT_CUDA(ctx, cudaMemsetAsync(it.tab_coef, 0, sizeof(double2) * it.tab_cap,
-                                  ctx->stream));
-  MPSFT_CUDA(ctx, cudaMemsetAsync(it.tab_err, 0, sizeof(double) * it.tab_cap,
-                                  ctx->stream));
-  MPSFT_CUDA(ctx, cudaMemsetAsync(ctl, 0, sizeof(int32_t) * kCtlWords,
-                                  ctx->stream));
   return MPSFT_OK;
 }
 
@@ -1988,6 +2082,7 @@ int mpsft_ctx_destroy(mpsft_ctx *ctx) {
   if (ctx->tw64) cudaFree(ctx->tw64);
   if (ctx->win_dev) cudaFree(ctx->win_dev);
   if (ctx->ph_cache) cudaFree(ctx->ph_cache);
+  for (mpsft_ctx::Table &e : ctx->tables) cudaFree(e.ptr);
   if (ctx->side64) {
     cudaStreamSynchronize(ctx->side64);
     cudaStreamDestroy(ctx->side64);
@@ -2389,7 +2484,14 @@ int BinInTimeImpl(mpsft_ctx *ctx, const mpsft_signal *sig, int32_t bins,
   const Transform tf{a, b, c, InverseMod(a, n)};
   FillIter(&it, sig, bins, bits, w, tf, &q, 1);
   cudaStream_t st = ctx->stream;
-  // the window tables: evaluated on the device, or the caller's uploaded
+  // the window and Bluestein tables: the context's, evaluated on the device
+  // when they are new, or (window) the caller's uploaded
+  bool new_window = true, new_blue = true;
+  if (!direct) {
+    BeginTables(ctx);
+    if (!wt) new_window = UseWindow(ctx, &it, delta, fp64 ? kTabWin64 : kTabWin32);
+    new_blue = UseBluestein(ctx, &it, fp64, false);
+  }
   auto window = [&]() -> int {
     if (wt) {
       const int r = UploadWindowTable(ctx, it, wt, st);
@@ -2398,8 +2500,8 @@ int BinInTimeImpl(mpsft_ctx *ctx, const mpsft_signal *sig, int32_t bins,
     if (direct) {
       if (!wt) LaunchWindow(d_it, 1, it.p2, st);
     } else if (fp64) {
-      LaunchWindowMod(d_it, 1, bins, !wt, false, st);
-    } else if (!wt) {
+      LaunchWindowMod(d_it, 1, bins, !wt && new_window, false, st);
+    } else if (!wt && new_window) {
       LaunchWindow32(d_it, 1, it.p2, st);
     }
     return MPSFT_OK;
@@ -2450,7 +2552,7 @@ int BinInTimeImpl(mpsft_ctx *ctx, const mpsft_signal *sig, int32_t bins,
   // FP32 (a caller's table: as given, and rounded to FP32)
   rc = window();
   if (rc) return rc;
-  LaunchBluesteinSetup(d_it, 1, it.fft_m, fp64, ctx->tw32, ctx->tw64, st);
+  if (new_blue) LaunchBluesteinSetup(d_it, 1, it.fft_m, fp64, ctx->tw32, ctx->tw64, st);
   BinTimer timer{ctx};
   rc = timer.Begin();
   if (rc) return rc;
@@ -2460,14 +2562,13 @@ int BinInTimeImpl(mpsft_ctx *ctx, const mpsft_signal *sig, int32_t bins,
   if (rc) return rc;
   LaunchRowFFT(d_it, 1, it.rows, 1, it.fft_m, fp64, ctx->tw32, ctx->tw64, st);
   MPSFT_CUDA(ctx, cudaGetLastError());
-  const size_t row_bytes = sizeof(double2) * size_t(bins);
-  MPSFT_CUDA(ctx, cudaMemcpy2DAsync(
-                      out, row_bytes, it.ubuf, sizeof(double2) * it.bins_cap,
-                      row_bytes, it.rows,
-                      out_on_device ? cudaMemcpyDeviceToDevice
-                                    : cudaMemcpyDeviceToHost,
+  // (bins_cap = bins: the rows are adjacent)
+  MPSFT_CUDA(ctx, cudaMemcpyAsync(
+                      out, it.ubuf, sizeof(double2) * size_t(bins) * it.rows,
+                      out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                       st));
   MPSFT_CUDA(ctx, cudaStreamSynchronize(st));
+  CommitTables(ctx);
   if (ctx->profiling) {
     mpsft_bin_launch rec{};
     rec.signals = 1;
@@ -2543,11 +2644,12 @@ int BinInFreqImpl(mpsft_ctx *ctx, int32_t n, int32_t bins, int32_t bits,
   it.x = nullptr;
   it.unit_wf = wf ? 1 : 0;
   cudaStream_t st = ctx->stream;
+  BeginTables(ctx);
+  const bool new_phases = UsePhases(ctx, &it);
   MPSFT_CUDA(ctx, cudaMemcpyAsync(d_it, &it, sizeof(it), cudaMemcpyHostToDevice,
                                   st));
-  LaunchPhaseTables(d_it, 1, PhaseTableEntries(n), st);
-  rc = ClearTable(ctx, it, ctl);
-  if (rc) return rc;
+  if (new_phases) LaunchPhaseTables(d_it, 1, PhaseTableEntries(n), st);
+  LaunchClearTables(d_it, 1, it.tab_cap, st);
   if (m > 0) {
     MPSFT_CUDA(ctx, cudaMemcpyAsync(d_k0, k0, sizeof(int32_t) * m,
                                     cudaMemcpyHostToDevice, st));
@@ -2568,20 +2670,18 @@ int BinInFreqImpl(mpsft_ctx *ctx, int32_t n, int32_t bins, int32_t bits,
     // the pageable source must outlive the copy
     if (wf) MPSFT_CUDA(ctx, cudaStreamSynchronize(st));
   }
-  const size_t row_bytes = sizeof(double2) * size_t(bins);
-  MPSFT_CUDA(ctx, cudaMemcpy2DAsync(it.ubuf, sizeof(double2) * it.bins_cap,
-                                    inout, row_bytes, row_bytes, it.rows,
-                                    cudaMemcpyHostToDevice, st));
+  // (bins_cap = bins: the rows are adjacent)
+  const size_t u_bytes = sizeof(double2) * size_t(bins) * it.rows;
+  MPSFT_CUDA(ctx, cudaMemcpyAsync(it.ubuf, inout, u_bytes, cudaMemcpyHostToDevice, st));
   LaunchBucket(d_it, 1, bins, s.tab_cap, st, true);
   LaunchDecide(d_it, 1, bins, 1, false, true, st);
   MPSFT_CUDA(ctx, cudaGetLastError());
-  MPSFT_CUDA(ctx, cudaMemcpy2DAsync(inout, row_bytes, it.ubuf,
-                                    sizeof(double2) * it.bins_cap, row_bytes,
-                                    it.rows, cudaMemcpyDeviceToHost, st));
+  MPSFT_CUDA(ctx, cudaMemcpyAsync(inout, it.ubuf, u_bytes, cudaMemcpyDeviceToHost, st));
   int32_t h_ctl[kCtlWords];
   MPSFT_CUDA(ctx, cudaMemcpyAsync(h_ctl, ctl, sizeof(h_ctl),
                                   cudaMemcpyDeviceToHost, st));
   MPSFT_CUDA(ctx, cudaStreamSynchronize(st));
+  CommitTables(ctx);
   if (h_ctl[1] & kStatusCapacity) {
     return Fail(ctx, MPSFT_ERR_CAPACITY, "mode table full");
   }
@@ -2633,7 +2733,8 @@ namespace {
 
 // Shared setup of mpsft_estimate / mpsft_adjoint: validates, carves one
 // signal's buffers plus `extra` bytes, fills and uploads the descriptor, and
-// builds the modulated window, FP64 Bluestein and unit-phase tables.
+// builds the modulated window and what the context does not hold yet of the
+// FP64 window, Bluestein and unit-phase tables.
 int EstimateSetup(mpsft_ctx *ctx, int32_t n, const void *x,
                   const mpsft_estimate_setup *su, size_t extra, Carve *cv,
                   SigIter *it, SigIter **d_it) {
@@ -2674,11 +2775,18 @@ int EstimateSetup(mpsft_ctx *ctx, int32_t n, const void *x,
   const Transform tf{su->a, su->b, su->c, 0};
   FillIter(it, &fake, su->bins, su->bits, su->window_delta, tf, su->q, su->trials);
   cudaStream_t st = ctx->stream;
+  // (the caller commits the tables after its wait)
+  BeginTables(ctx);
+  const bool new_phases = UsePhases(ctx, it);
+  const bool new_window = UseWindow(ctx, it, su->window_delta, kTabWin64);
+  const bool new_blue = UseBluestein(ctx, it, true, false);
   MPSFT_CUDA(ctx, cudaMemcpyAsync(*d_it, it, sizeof(SigIter),
                                   cudaMemcpyHostToDevice, st));
-  LaunchPhaseTables(*d_it, 1, PhaseTableEntries(n), st);
-  LaunchWindowMod(*d_it, 1, su->bins, true, false, st);
-  LaunchBluesteinSetup(*d_it, 1, it->fft_m, true, ctx->tw32, ctx->tw64, st);
+  if (new_phases) LaunchPhaseTables(*d_it, 1, PhaseTableEntries(n), st);
+  LaunchWindowMod(*d_it, 1, su->bins, new_window, false, st);
+  if (new_blue) {
+    LaunchBluesteinSetup(*d_it, 1, it->fft_m, true, ctx->tw32, ctx->tw64, st);
+  }
   MPSFT_CUDA(ctx, cudaGetLastError());
   return MPSFT_OK;
 }
@@ -2726,6 +2834,7 @@ int mpsft_estimate(mpsft_ctx *ctx, const mpsft_signal *sig,
                                     cudaMemcpyDeviceToHost, st));
   }
   MPSFT_CUDA(ctx, cudaStreamSynchronize(st));
+  CommitTables(ctx);
   return MPSFT_OK;
 }
 
@@ -2763,6 +2872,7 @@ int mpsft_adjoint(mpsft_ctx *ctx, int32_t n, const mpsft_estimate_setup *setup,
   MPSFT_CUDA(ctx, cudaMemcpyAsync(dx, d_dx, sizeof(double2) * size_t(n),
                                   cudaMemcpyDeviceToHost, st));
   MPSFT_CUDA(ctx, cudaStreamSynchronize(st));
+  CommitTables(ctx);
   return MPSFT_OK;
 }
 
@@ -2843,9 +2953,16 @@ int IterateImpl(mpsft_ctx *ctx, const mpsft_signal *sig,
   int32_t *ctl;
   CarveSignal(probe, s, &it, &ctl);
   const int64_t m0 = *mm_size;
+  // the results' staging: control words, entry count and sorted flag, then the
+  // table's keys and coefficients (at most the given modes and one per bin)
+  const size_t entries = size_t(m0) + size_t(bins);
+  const size_t off_keys = 256, off_coefs = off_keys + ((4 * entries + 255) & ~size_t(255));
+  const size_t res_bytes = off_coefs + sizeof(double2) * entries;
   const size_t extra = size_t(m0) * (sizeof(int32_t) + sizeof(double2)) +
-                       sizeof(double) * kEnergyStride + 2048;
+                       sizeof(double) * kEnergyStride + res_bytes + 4096;
   rc = EnsureArena(ctx, probe.off + sizeof(SigIter) + extra);
+  if (rc) return rc;
+  rc = EnsureHostStage(ctx, res_bytes);
   if (rc) return rc;
   Carve cv{ctx->arena};
   SigIter *d_it = cv.take<SigIter>(1);
@@ -2856,6 +2973,7 @@ int IterateImpl(mpsft_ctx *ctx, const mpsft_signal *sig,
   double *d_energy = cv.take<double>(kEnergyStride);
   const void **d_xs = cv.take<const void *>(1);
   int64_t *d_ns = cv.take<int64_t>(1);
+  unsigned char *d_res = cv.take<unsigned char>(res_bytes);
   Transform tf;
   int32_t q[kMaxTrials];
   if (tf_in) {
@@ -2871,6 +2989,11 @@ int IterateImpl(mpsft_ctx *ctx, const mpsft_signal *sig,
   SetThresholdCopies(&it);
   it.win_thr = opt->window_threshold;
   cudaStream_t st = ctx->stream;
+  BeginTables(ctx);
+  const bool new_phases = UsePhases(ctx, &it);
+  // the mode table is cleared and filled while the host waits for the energy
+  MPSFT_CUDA(ctx, cudaMemcpyAsync(d_it, &it, sizeof(it), cudaMemcpyHostToDevice,
+                                  st));
   std::vector<double> energy(1, 0.0);
   if (!fp64) {
     const void *h_x = sig->d_x;
@@ -2880,17 +3003,9 @@ int IterateImpl(mpsft_ctx *ctx, const mpsft_signal *sig,
     MPSFT_CUDA(ctx, cudaMemcpyAsync(d_ns, &h_n, sizeof(h_n),
                                     cudaMemcpyHostToDevice, st));
     LaunchEnergy(d_xs, d_ns, 1, sig->dtype == MPSFT_C128, d_energy, st, kPolicySample);
-    rc = ReadEnergy(ctx, d_energy, 1, &energy);
-    if (rc) return rc;
   }
-  SetNearTie(&it, fp64, opt->near_tie_margin, bins,
-             !fp64 && PolicyForcesFP64(opt->near_tie_margin, bins, energy[0],
-                                       opt->bin_threshold, opt->sv_threshold));
-  MPSFT_CUDA(ctx, cudaMemcpyAsync(d_it, &it, sizeof(it), cudaMemcpyHostToDevice,
-                                  st));
-  LaunchPhaseTables(d_it, 1, PhaseTableEntries(n), st);
-  rc = ClearTable(ctx, it, ctl);
-  if (rc) return rc;
+  if (new_phases) LaunchPhaseTables(d_it, 1, PhaseTableEntries(n), st);
+  LaunchClearTables(d_it, 1, it.tab_cap, st);
   if (m0 > 0) {
     MPSFT_CUDA(ctx, cudaMemcpyAsync(d_k0, mm_k, sizeof(int32_t) * m0,
                                     cudaMemcpyHostToDevice, st));
@@ -2898,33 +3013,57 @@ int IterateImpl(mpsft_ctx *ctx, const mpsft_signal *sig,
                                     cudaMemcpyHostToDevice, st));
     LaunchTableInsert(d_it, d_k0, d_coef, m0, st);
   }
+  if (!fp64) {
+    rc = ReadEnergy(ctx, d_energy, 1, &energy);
+    if (rc) return rc;
+  }
+  SetNearTie(&it, fp64, opt->near_tie_margin, bins,
+             !fp64 && PolicyForcesFP64(opt->near_tie_margin, bins, energy[0],
+                                       opt->bin_threshold, opt->sv_threshold));
+  // window and Bluestein tables of the kernels that will run: the context's
+  const bool f64 = fp64 || it.force_fp64;
+  bool fresh = UseBluestein(ctx, &it, f64, !f64);
+  if (f64) {
+    fresh |= UseWindow(ctx, &it, opt->window_delta, kTabWin64);
+    it.wtff = nullptr;  // (the near-tie re-binning's, not of these kernels)
+  } else {
+    fresh |= UseWindow(ctx, &it, opt->window_delta, kTabWin32);
+    fresh |= UseWindow(ctx, &it, opt->window_delta, kTabWinFF);
+  }
+  MPSFT_CUDA(ctx, cudaMemcpyAsync(d_it, &it, sizeof(it), cudaMemcpyHostToDevice,
+                                  st));
   std::vector<SigIter> h_its(1, it);
   BinTimer timer{ctx};
   rc = LaunchIteration(ctx, d_it, 1, h_its, sig->dtype == MPSFT_C128, fp64,
-                       &timer);
+                       &timer, nullptr, 0, !fresh);
   if (rc) return rc;
-  int32_t h_ctl[kCtlWords];
-  MPSFT_CUDA(ctx, cudaMemcpyAsync(h_ctl, ctl, sizeof(h_ctl),
-                                  cudaMemcpyDeviceToHost, st));
+  // the control words and the table, sorted by k0, with one wait
+  int32_t *head = reinterpret_cast<int32_t *>(d_res);
+  LaunchExportTables(d_it, 1, it.tab_cap, reinterpret_cast<int32_t *>(d_res + off_keys),
+                     reinterpret_cast<double2 *>(d_res + off_coefs), head + kCtlWords,
+                     head + kCtlWords + 1, st);
+  MPSFT_CUDA(ctx, cudaMemcpyAsync(head, ctl, sizeof(int32_t) * kCtlWords,
+                                  cudaMemcpyDeviceToDevice, st));
+  MPSFT_CUDA(ctx, cudaMemcpyAsync(ctx->h_stage, d_res, res_bytes, cudaMemcpyDeviceToHost,
+                                  st));
   MPSFT_CUDA(ctx, cudaStreamSynchronize(st));
+  CommitTables(ctx);
+  const int32_t *h_ctl = reinterpret_cast<const int32_t *>(ctx->h_stage);
   if (h_ctl[1] & kStatusCapacity) {
     return Fail(ctx, MPSFT_ERR_CAPACITY, "mode table full");
   }
   if (h_ctl[1] & kStatusNonFinite) {
     return Fail(ctx, MPSFT_ERR_NONFINITE, "non-finite values in the bins");
   }
-  std::vector<std::pair<int32_t, double2>> modes;
-  rc = DownloadTable(ctx, it, &modes);
-  if (rc) return rc;
-  if (int64_t(modes.size()) > mm_cap) {
+  // (at most m0 + bins entries, so the table is never more than half full and
+  // always exported sorted)
+  const int32_t size = h_ctl[kCtlWords];
+  if (size > mm_cap) {
     return Fail(ctx, MPSFT_ERR_CAPACITY, "mode map capacity too small");
   }
-  for (size_t j = 0; j < modes.size(); ++j) {
-    mm_k[j] = modes[j].first;
-    mm_c[2 * j] = modes[j].second.x;
-    mm_c[2 * j + 1] = modes[j].second.y;
-  }
-  *mm_size = int32_t(modes.size());
+  std::memcpy(mm_k, ctx->h_stage + off_keys, sizeof(int32_t) * size_t(size));
+  std::memcpy(mm_c, ctx->h_stage + off_coefs, sizeof(double2) * size_t(size));
+  *mm_size = size;
   *found = h_ctl[0] ? 1 : 0;
   return MPSFT_OK;
 }

@@ -170,6 +170,22 @@ struct mpsft_ctx {
   // for the next calls of that length
   double2 *ph_cache = nullptr;
   int64_t ph_cache_n = 0;
+  // tables of the single-signal calls (bins, estimates, Iterate), kept like FFT
+  // plans under what they depend on (CtxTable): bounded, least recently used
+  // out first, freed with the context
+  struct Table {
+    int kind;
+    int32_t bins;
+    int64_t n;
+    double delta;
+    unsigned char *ptr;
+    size_t bytes;
+    uint64_t used;  // the last call that asked for it
+    bool built;     // its builder's call has completed
+  };
+  std::vector<Table> tables;
+  size_t table_bytes = 0;
+  uint64_t table_call = 0;
   size_t win_bytes = 0;
   double win_delta = 0.0;
   int32_t win_bmin = 0, win_bmax = 0;

@@ -686,3 +686,49 @@ def test_bin_in_freq_modes_per_bin(ctx, port, count, bits):
     got = ctx.bin_in_freq(u, n, bins, bits, 1e-5, 1, 0, 77, 991, k, coef)
     want = port.bin_in_freq(u, n, bins, bits, 1e-5, 1, 0, 77, 991, k, coef)
     assert rel_err(got, want) < 1e-12
+
+
+def test_single_call_tables(ctx):
+    """The tables a context keeps for single calls (per bins, delta, n and
+    precision; the least recently used leave when there are too many): calls in
+    an order that reuses, evicts and rebuilds them give the same bits as
+    contexts that have just been made."""
+    rng = np.random.default_rng(5)
+    n = 1 << 14
+    x = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    k0 = rng.choice(n, 9, replace=False).astype(np.int32)
+    g = rng.standard_normal(9) + 1j * rng.standard_normal(9)
+
+    def call(c, sig, i):
+        bins, delta = 51 + 2 * (i % 50), (1e-5, 1e-6)[i % 3 == 0]
+        prec = PRECS[i % 2]
+        out = [c.bin_in_time(sig, bins, 6, delta, 77, 5, 9, 31, precision=prec)]
+        su = c.estimate_setup(bins, 6, delta, 77, 5, 9, [31])
+        nn = (n, 8191, 65537)[i % 3]
+        out.append(c.adjoint(nn, su, k0 % nn, g))
+        out.append(c.bin_in_freq(out[0], nn, bins, 6, delta, 77, 5, 9, 31, k0 % nn, g))
+        _, mm = c.iterate(sig, m.Rng(4 + i), bins, delta, precision=prec)
+        out.append(np.array([mm[k] for k in sorted(mm)]))
+        return out
+
+    kept = m.Context(0)
+    sig = kept.upload(x)
+    order = list(range(50)) + [0, 49, 7, 7, 23, 0]
+    got = {}
+    for i in order:
+        out = call(kept, sig, i)
+        if i in got:
+            for a, b in zip(out, got[i]):
+                # (the adjoint adds by atomics in any order)
+                assert np.allclose(a, b, rtol=0, atol=1e-13 * max(1.0, np.abs(b).max()))
+            for j in (0, 2, 3):
+                assert np.array_equal(out[j], got[i][j])
+        got[i] = out
+    for i in (0, 7, 23, 49):
+        c = m.Context(0)
+        s = c.upload(x)
+        out = call(c, s, i)
+        for j in (0, 2, 3):
+            assert np.array_equal(out[j], got[i][j])
+        c.close()
+    kept.close()
