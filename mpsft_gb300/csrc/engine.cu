@@ -864,7 +864,8 @@ Maxima MaximaOf(const std::vector<SigIter> &h_its) {
 
 // The kernels of one iteration of every active signal, on stream s (and the
 // context's side stream, forked from and joined back into s). tables: the
-// window and Bluestein tables are in place (CtxTable).
+// window and Bluestein tables are in place (CtxTable). single: a call of one
+// iteration (not of a solve).
 // The fixed-bins phase's pipelined body: while this iteration decides, the
 // next one (descriptors its_ahead) is planned and gathered/folded on the
 // prefold stream, into the second fold buffer (only this iteration's row FFT
@@ -933,7 +934,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
                            const Maxima &mx, bool x_c128, bool fp64,
                            Forced forced, BinTimer *timer, int64_t *launched,
                            cudaStream_t s, const Ahead *ahead = nullptr,
-                           bool tables = false) {
+                           bool tables = false, bool single = false) {
   if (mx.bins == 0) return MPSFT_OK;
   if (forced == kAllForced && !fp64 && mx.m <= kMaxFFT64) {
     return LaunchForcedIteration(ctx, d_its, nsig, mx, x_c128, timer, launched, s, tables);
@@ -1007,7 +1008,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   }
   if (!ahead && !tables) MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_blue, 0));
   LaunchRowFFT(d_its, nsig, mx.rows, mx.trials, mx.m, fp64, ctx->tw32, ctx->tw64,
-               s);
+               s, false, single);
   MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join, 0));  // join
   // near ties of the FP32 pass: listed bins re-binned and re-decided in
   // FP64; signals that the precision policy sends to FP64 (and signals whose
@@ -1073,7 +1074,8 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
 int LaunchIteration(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
                     const std::vector<SigIter> &h_its, bool x_c128, bool fp64,
                     BinTimer *timer, int64_t *launched = nullptr,
-                    int32_t tune_bins = 0, bool tables = false) {
+                    int32_t tune_bins = 0, bool tables = false,
+                    bool single = false) {
   int active = 0, forced = 0;
   for (const SigIter &it : h_its) {
     active += it.active;
@@ -1084,7 +1086,7 @@ int LaunchIteration(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   const int rc = LaunchIterationKernels(
       ctx, d_its, nsig, mx, x_c128, fp64,
       forced == 0 ? kNoneForced : (forced < active ? kSomeForced : kAllForced), timer,
-      launched, ctx->stream, nullptr, tables);
+      launched, ctx->stream, nullptr, tables, single);
   if (rc != MPSFT_OK) return rc;
   // (in the solve graph, k_finish inserts the spilled candidates)
   LaunchInsertSpills(d_its, nsig, ctx->stream);
@@ -2560,7 +2562,8 @@ int BinInTimeImpl(mpsft_ctx *ctx, const mpsft_signal *sig, int32_t bins,
                 FoldShapeFor(ctx, bins, sig->n, 1, sig->dtype == MPSFT_C128));
   rc = timer.End();
   if (rc) return rc;
-  LaunchRowFFT(d_it, 1, it.rows, 1, it.fft_m, fp64, ctx->tw32, ctx->tw64, st);
+  LaunchRowFFT(d_it, 1, it.rows, 1, it.fft_m, fp64, ctx->tw32, ctx->tw64, st, false,
+               true);
   MPSFT_CUDA(ctx, cudaGetLastError());
   // (bins_cap = bins: the rows are adjacent)
   MPSFT_CUDA(ctx, cudaMemcpyAsync(
@@ -3035,7 +3038,7 @@ int IterateImpl(mpsft_ctx *ctx, const mpsft_signal *sig,
   std::vector<SigIter> h_its(1, it);
   BinTimer timer{ctx};
   rc = LaunchIteration(ctx, d_it, 1, h_its, sig->dtype == MPSFT_C128, fp64,
-                       &timer, nullptr, 0, !fresh);
+                       &timer, nullptr, 0, !fresh, true);
   if (rc) return rc;
   // the control words and the table, sorted by k0, with one wait
   int32_t *head = reinterpret_cast<int32_t *>(d_res);

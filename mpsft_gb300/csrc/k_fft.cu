@@ -261,42 +261,61 @@ __global__ void __launch_bounds__(kRowFftThreads)
   }
 }
 
-// The FP64 row transform with one row over a cluster of C blocks, for launches
-// of few rows (one signal's call): FP64 operations bound it, and a block per
-// row leaves most SMs' pipes idle. Block c holds the c-th of C slices of the
-// bit-reversed array, Ms = M / C elements. The first log2 C forward stages need
-// no exchange: every block reads the row's samples and evaluates its own
-// outputs of them (the upper half of the input is zero). The stages within a
-// slice run as in k_row_fft; the last log2 C inverse stages read the C
-// slices' element k through distributed shared memory, each block a C-th of
-// the k, and only the outputs below M/2. A transform too small to split
+// The row transform with one row over a cluster of C blocks, for launches of
+// few rows (one signal's call), which a block per row leaves on a few SMs:
+// there the FP64 transform is bound by those SMs' FP64 pipes and the FP32 one
+// by the latency of its passes over a long row. Block c holds the c-th of C
+// slices of the bit-reversed array, Ms = M / C elements. The first log2 C
+// forward stages need no exchange: every block reads the row's samples and
+// evaluates its own outputs of them (the upper half of the input is zero). The
+// stages within a slice run as in k_row_fft; the last log2 C inverse stages read
+// the C slices' element k through distributed shared memory, each block a C-th
+// of the k, and only the outputs below M/2. A transform too small to split
 // (M < kSplitMin C) runs whole on block 0.
-// 31 rows of 501 bins (M = 1024), cold: 37 us with a block per row, 21 us
-// with 4.
+// Cold, FP64, 31 rows of 501 bins (M = 1024): 37 us with a block per row, 21 us
+// with 4; FP32, 29 rows of 8001 bins (M = 16384): 87 us and 33 us
+// with 8 (31 rows of 501 bins: 15.5 and 13 us).
 constexpr int kSplitThreads = 256;
 constexpr int kSplitMin = 64;  // elements per slice at least
 
-// One row of one block of the cluster: fill, local stages, exchange, epilogue
-// (dst = row factor * output); returns the block's sum and maximum of |U|^2.
-template <int C>
+// Output j of the row's transform times the row factor: FP64 bins, FP32 bins
+// widened, or (solves and iterations) complex64 bins.
+__device__ __forceinline__ void StoreBin(const SigIter &it, int tr, int row, int j, double2 y,
+                                         float2, float2, double2 f) {
+  it.ubuf[(size_t(tr) * it.rows + row) * it.bins_cap + j] = vmul(f, y);
+}
+__device__ __forceinline__ void StoreBin(const SigIter &it, int tr, int row, int j, float2 y,
+                                         float2 bh, float2 bl, double2 f) {
+  const size_t o = (size_t(tr) * it.rows + row) * it.bins_cap + j;
+  if (it.ubuf32 != nullptr) {
+    it.ubuf32[o] = MulPhaseFF(y, bh, bl);
+  } else {
+    it.ubuf[o] = cmul(f, make_double2(y.x, y.y));
+  }
+}
+
+// One row of one block of the cluster: fill, local stages, exchange, epilogue;
+// adds this thread's share to the sum and the maximum of |U|^2.
+template <typename V, int C>
 __device__ __forceinline__ void SplitRow(const SigIter &it, int tr, int row, int c,
-                                         cooperative_groups::cluster_group cl,
-                                         double2 *a, const double2 *__restrict__ tw,
-                                         bool work, float *ss, float *mx) {
+                                         cooperative_groups::cluster_group cl, V *a,
+                                         const V *__restrict__ tw, bool work, float *ss,
+                                         float *mx) {
   constexpr int kLog = C == 8 ? 3 : (C == 4 ? 2 : (C == 2 ? 1 : 0));
   constexpr int H = C > 1 ? C / 2 : 1;  // slices of the lower half
+  constexpr bool kF64 = sizeof(V) == sizeof(double2);
   const int B = it.bins, L = it.fft_log2m, M = it.fft_m, Ms = M / C;
   const int tid = threadIdx.x, lg = L - kLog;
-  const double2 *__restrict__ chirp = it.chirp64;
+  const V *__restrict__ chirp = ChirpOf(it, (V *)nullptr);
   if (work) {
-    const double2 *__restrict__ src = reinterpret_cast<const double2 *>(it.fold) +
-                                      (size_t(tr) * it.rows + row) * it.bins_cap;
+    const V *__restrict__ src = reinterpret_cast<const V *>(it.fold) +
+                                (size_t(tr) * it.rows + row) * it.bins_cap;
     for (int k = tid; k < Ms; k += kSplitThreads) {
-      double2 v[H];
+      V v[H];
 #pragma unroll
       for (int m = 0; m < H; ++m) {
         const int j = k + m * Ms;
-        v[m] = make_double2(0.0, 0.0);
+        v[m] = vmake2(0.0, 0.0, (V *)nullptr);
         if (j < B) {
           v[m] = vmul(src[j], __ldg(&chirp[j]));
           if (C > 1 && (c & (C / 2))) v[m] = vmul(v[m], Twiddle(tw, L, j, false));
@@ -320,19 +339,24 @@ __device__ __forceinline__ void SplitRow(const SigIter &it, int tr, int row, int
     }
   }
   __syncthreads();
-  BlockConv(a, work ? Ms : 0, lg, StagesPerPass(Ms), it.chat64 + size_t(c) * Ms, tw, tid,
-            kSplitThreads);
+  // stages per pass: FP64 by its schedulers (StagesPerPass), FP32 three (fewer
+  // barriers) unless that leaves less than two warps
+  BlockConv(a, work ? Ms : 0, lg, kF64 ? StagesPerPass(Ms) : (Ms >= 512 ? 3 : 2),
+            ChatOf(it, (V *)nullptr) + size_t(c) * Ms, tw, tid, kSplitThreads);
   cl.sync();  // every slice is done
   if (work) {
-    const double inv_m = 1.0 / double(M);
-    const double2 bq = it.row_fac[tr * it.rows + row];
-    double2 *dst = it.ubuf + (size_t(tr) * it.rows + row) * it.bins_cap;
-    const double2 *part[C];
+    const double2 f = kF64 ? it.row_fac[tr * it.rows + row]
+                           : make_double2(it.bq_re[tr], it.bq_im[tr]);
+    const float2 bh = make_float2(__double2float_rn(f.x), __double2float_rn(f.y));
+    const float2 bl = make_float2(__double2float_rn(f.x - double(bh.x)),
+                                  __double2float_rn(f.y - double(bh.y)));
+    const decltype(a->x) inv_m = decltype(a->x)(1) / decltype(a->x)(M);
+    const V *part[C];
 #pragma unroll
     for (int i = 0; i < C; ++i) part[i] = C > 1 ? cl.map_shared_rank(a, i) : a;
     const int k1 = (c + 1) * (Ms / C);
     for (int k = c * (Ms / C) + tid; k < k1; k += kSplitThreads) {
-      double2 x[C];
+      V x[C];
 #pragma unroll
       for (int i = 0; i < C; ++i) x[i] = part[i][Pad(k)];
 #pragma unroll
@@ -341,8 +365,8 @@ __device__ __forceinline__ void SplitRow(const SigIter &it, int tr, int row, int
         for (int i = 0; i < C; ++i) {
           if ((i & (1 << s)) == 0) {
             const int e = k + (i & ((1 << s) - 1)) * Ms;
-            const double2 v = vmul(x[i + (1 << s)], Twiddle(tw, lg + s + 1, e, true));
-            const double2 u = x[i];
+            const V v = vmul(x[i + (1 << s)], Twiddle(tw, lg + s + 1, e, true));
+            const V u = x[i];
             x[i] = vadd(u, v);
             if (s + 1 < kLog) x[i + (1 << s)] = vsub(u, v);
           }
@@ -352,9 +376,11 @@ __device__ __forceinline__ void SplitRow(const SigIter &it, int tr, int row, int
       for (int i = 0; i < H; ++i) {
         const int j = k + i * Ms;
         if (j < B) {
-          const double2 y = cscale(vmul(x[i], __ldg(&chirp[j])), inv_m);
-          dst[j] = vmul(bq, y);
-          const double y2 = y.x * y.x + y.y * y.y;
+          V y = vmul(x[i], __ldg(&chirp[j]));
+          y.x *= inv_m;  // (a power of two: exact)
+          y.y *= inv_m;
+          StoreBin(it, tr, row, j, y, bh, bl, f);
+          const auto y2 = y.x * y.x + y.y * y.y;
           *ss += float(y2);
           *mx = fmaxf(*mx, float(sqrt(y2)));
         }
@@ -363,10 +389,9 @@ __device__ __forceinline__ void SplitRow(const SigIter &it, int tr, int row, int
   }
 }
 
-template <int C>
+template <typename V, int C>
 __global__ void __launch_bounds__(kSplitThreads)
-    k_row_fft_split(const SigIter *__restrict__ its, const double2 *__restrict__ tw,
-                    int cond) {
+    k_row_fft_split(const SigIter *__restrict__ its, const V *__restrict__ tw, int cond) {
   PdlEnter(its, kTraceRowFft);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float part_ss[C], part_mx[C];  // block 0's: every block's share
@@ -378,12 +403,12 @@ __global__ void __launch_bounds__(kSplitThreads)
   if (cond ? !RedoFP64(it) : it.force_fp64) return;
   cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
   const int c = int(cl.block_rank());
-  double2 *a = reinterpret_cast<double2 *>(smem_raw);
+  V *a = reinterpret_cast<V *>(smem_raw);
   float ss = 0.f, mx = 0.f;
   if (it.fft_m >= kSplitMin * C) {
-    SplitRow<C>(it, tr, row, c, cl, a, tw, true, &ss, &mx);
+    SplitRow<V, C>(it, tr, row, c, cl, a, tw, true, &ss, &mx);
   } else {
-    SplitRow<1>(it, tr, row, 0, cl, a, tw, c == 0, &ss, &mx);
+    SplitRow<V, 1>(it, tr, row, 0, cl, a, tw, c == 0, &ss, &mx);
   }
   // the row's largest magnitude and sum of |U|^2 in a fixed order: a shuffle
   // tree, the warps in order, the blocks in order
@@ -540,20 +565,36 @@ inline size_t SplitSlots(int max_m, int c) {
   return size_t(PadLen(std::max(max_m / c, kSplitMin * c)));
 }
 
-template <int C>
-void LaunchRowSplit(const SigIter *d_its, dim3 grid, int max_m, const double2 *tw,
-                    cudaStream_t s, bool cond) {
-  const size_t sm = SplitSlots(max_m, C) * sizeof(double2);
-  cudaFuncSetAttribute(k_row_fft_split<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+template <typename V, int C>
+void LaunchRowSplit(const SigIter *d_its, dim3 grid, int max_m, const V *tw, cudaStream_t s,
+                    bool cond) {
+  const size_t sm = SplitSlots(max_m, C) * sizeof(V);
+  cudaFuncSetAttribute(k_row_fft_split<V, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        int(sm));
   grid.x *= C;
-  LaunchCluster(k_row_fft_split<C>, grid, kSplitThreads, sm, s, C, d_its, tw,
+  LaunchCluster(k_row_fft_split<V, C>, grid, kSplitThreads, sm, s, C, d_its, tw,
                 cond ? 1 : 0);
+}
+
+// Rows over clusters of c blocks; false for c = 1.
+template <typename V>
+bool LaunchRowSplits(const SigIter *d_its, dim3 grid, int c, int max_m, const V *tw,
+                     cudaStream_t s, bool cond) {
+  if (c == 8) {
+    LaunchRowSplit<V, 8>(d_its, grid, max_m, tw, s, cond);
+  } else if (c == 4) {
+    LaunchRowSplit<V, 4>(d_its, grid, max_m, tw, s, cond);
+  } else if (c == 2) {
+    LaunchRowSplit<V, 2>(d_its, grid, max_m, tw, s, cond);
+  } else {
+    return false;
+  }
+  return true;
 }
 
 void LaunchRowFFT(const SigIter *d_its, int nsig, int max_rows,
                   int max_trials, int max_m, bool fp64, const float2 *tw32,
-                  const double2 *tw64, cudaStream_t s, bool cond) {
+                  const double2 *tw64, cudaStream_t s, bool cond, bool split32) {
   // rows per block: as many as the transform size allows, but no fewer
   // blocks than about two per SM (so that a single signal, or the FP64
   // pipes, still spread over the GPU); every transform of the launch has at
@@ -564,17 +605,19 @@ void LaunchRowFFT(const SigIter *d_its, int nsig, int max_rows,
     Launch(k_row_dft_small, g, 64 * kDirectRowsPerBlock, 0, s, d_its, cond ? 1 : 0);
     return;
   }
-  // FP64 with so few rows that they do not fill the SMs' FP64 pipes: a row over
-  // a cluster of as many blocks as leave an SM to each (two blocks on one SM
-  // share its pipes and gain nothing), slices of kSplitMin elements or more
+  // so few rows that a block each does not fill the SMs: a row over a cluster,
+  // slices of kSplitMin elements or more. FP64: as many blocks as leave an SM
+  // to each (two blocks on one SM share its pipes and gain nothing); FP32: up to
+  // two per SM
   const int64_t total = int64_t(max_rows) * max_trials * nsig;
-  if (fp64) {
+  if (fp64 || split32) {
     int c = 8;
-    while (c > 1 && (total * c > 152 || max_m < kSplitMin * c)) c /= 2;
+    while (c > 1 && (total * c > (fp64 ? 152 : 304) || max_m < kSplitMin * c)) c /= 2;
     const dim3 g(max_rows, max_trials, nsig);
-    if (c == 8) return LaunchRowSplit<8>(d_its, g, max_m, tw64, s, cond);
-    if (c == 4) return LaunchRowSplit<4>(d_its, g, max_m, tw64, s, cond);
-    if (c == 2) return LaunchRowSplit<2>(d_its, g, max_m, tw64, s, cond);
+    if (fp64 ? LaunchRowSplits(d_its, g, c, max_m, tw64, s, cond)
+             : LaunchRowSplits(d_its, g, c, max_m, tw32, s, cond)) {
+      return;
+    }
   }
   // (a power of two, so that a row's threads are whole shuffle segments)
   int rpb_cap = 1;
@@ -610,9 +653,10 @@ bool FftKernelsLaunchable() {
   // split rows: the largest transform over the smallest cluster
   int n3 = 0;
   const size_t sms = SplitSlots(kMaxFFT64, 2) * sizeof(double2);
-  cudaFuncSetAttribute(k_row_fft_split<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       int(sms));
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n3, k_row_fft_split<2>, kSplitThreads, sms);
+  cudaFuncSetAttribute(k_row_fft_split<double2, 2>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(sms));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n3, k_row_fft_split<double2, 2>,
+                                                kSplitThreads, sms);
   if (n3 == 0) return false;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n1, k_row_fft<float2>, 512, sm32);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n2, k_row_fft<double2>, 512, sm64);

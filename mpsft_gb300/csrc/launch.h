@@ -104,10 +104,14 @@ void LaunchBinFold(const SigIter *d_its, int nsig, int max_bins, int max_bits,
                    int max_trials, bool x_c128, bool fp64, cudaStream_t s,
                    bool cond = false, int shape = 0);
 
-// Size-B FFT of every folded row, times e^{2 pi i b q / n}, into ubuf.
+// Size-B FFT of every folded row, times its row factor, into ubuf. split32:
+// few FP32 rows may go over clusters of blocks (calls of one iteration or bin
+// matrix; the rounding differs from the transform of solves, whose batches
+// have rows enough).
 void LaunchRowFFT(const SigIter *d_its, int nsig, int max_rows,
                   int max_trials, int max_m, bool fp64, const float2 *tw32,
-                  const double2 *tw64, cudaStream_t s, bool cond = false);
+                  const double2 *tw64, cudaStream_t s, bool cond = false,
+                  bool split32 = false);
 
 // Per found mode: k1, bin, window response and the per-trial row-0 term
 // (FP32 terms on the FP32 path, FP64 terms on the FP64 path and for signals

@@ -146,7 +146,7 @@ extern "C" int mpsft_bin_in_time_noalloc(const void *x_device, int64_t n,
   }
   LaunchBluesteinSetup(d_it, 1, it.fft_m, fp64, tw32, tw64, st);
   LaunchBinFold(d_it, 1, bins, bits, 1, dtype == MPSFT_C128, fp64, st);
-  LaunchRowFFT(d_it, 1, it.rows, 1, it.fft_m, fp64, tw32, tw64, st);
+  LaunchRowFFT(d_it, 1, it.rows, 1, it.fft_m, fp64, tw32, tw64, st, false, true);
   if (cudaGetLastError() != cudaSuccess) return MPSFT_ERR_CUDA;
   return MPSFT_OK;
 }
