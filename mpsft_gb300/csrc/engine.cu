@@ -224,12 +224,14 @@ void SetNearTie(SigIter *it, bool fp64, double margin, int32_t bins,
 // mean |x|^2 of the signals (device values, one synchronisation)
 int ReadEnergy(mpsft_ctx *ctx, const double *d_energy, int nsig,
                std::vector<double> *out) {
-  out->assign(nsig, 0.0);
-  MPSFT_CUDA(ctx, cudaMemcpy2DAsync(out->data(), sizeof(double), d_energy,
-                                    sizeof(double) * kEnergyStride,
-                                    sizeof(double), nsig,
-                                    cudaMemcpyDeviceToHost, ctx->stream));
+  std::vector<double> parts(size_t(nsig) * kEnergyStride);
+  MPSFT_CUDA(ctx, cudaMemcpyAsync(parts.data(), d_energy, sizeof(double) * parts.size(),
+                                  cudaMemcpyDeviceToHost, ctx->stream));
   MPSFT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  out->assign(nsig, 0.0);
+  for (int i = 0; i < nsig; ++i) {
+    for (int b = 0; b < kEnergyParts; ++b) (*out)[i] += parts[i * kEnergyStride + b];
+  }
   return MPSFT_OK;
 }
 

@@ -297,97 +297,40 @@ namespace mpsft {
 
 namespace {
 
-// Deterministic mean |x|^2: block b of signal s sums a fixed share in a
-// fixed tree order, then one block adds the partials in order. per_block = 0:
-// every sample (grid stride); otherwise block b sums the per_block samples
-// from n b / kEnergyBlocks on (an estimate from kEnergyBlocks evenly spread
-// runs).
-template <typename TX>
-__global__ void k_energy_partial(const void *const *__restrict__ xs,
-                                 const int64_t *__restrict__ ns,
-                                 double *__restrict__ energy, int per_block) {
-  __shared__ double red[256];
-  const int sig = blockIdx.y;
-  const TX *x = reinterpret_cast<const TX *>(xs[sig]);
-  const int64_t n = ns[sig];
-  // per-thread sums in FP32 (a few thousand terms), combined in FP64
-  float acc = 0.f;
-  const int64_t run = per_block > 0 ? min(int64_t(per_block), n / kEnergyBlocks) : 0;
-  if (run > 0) {
-    const int64_t start = n * blockIdx.x / kEnergyBlocks;
-    for (int64_t i = threadIdx.x; i < run; i += blockDim.x) {
-      const TX v = x[start + i];
-      const float re = float(v.x), im = float(v.y);
-      acc = fmaf(re, re, fmaf(im, im, acc));
-    }
-  } else {
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += int64_t(gridDim.x) * blockDim.x) {
-      const TX v = x[i];
-      const float re = float(v.x), im = float(v.y);
-      acc = fmaf(re, re, fmaf(im, im, acc));
-    }
-  }
-  red[threadIdx.x] = double(acc);
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) energy[size_t(sig) * kEnergyStride + 1 + blockIdx.x] = red[0];
-}
-
-__global__ void k_energy_final(const int64_t *__restrict__ ns,
-                               double *__restrict__ energy, int per_block) {
-  __shared__ double red[kEnergyBlocks];
-  const int sig = blockIdx.x;
-  double *e = energy + size_t(sig) * kEnergyStride;
-  red[threadIdx.x] = e[1 + threadIdx.x];
-  __syncthreads();
-  for (int o = kEnergyBlocks / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  const int64_t n = ns[sig];
-  const int64_t run = per_block > 0 ? min(int64_t(per_block), n / kEnergyBlocks) : 0;
-  if (threadIdx.x == 0) e[0] = red[0] / double(run > 0 ? run * kEnergyBlocks : n);
-}
-
-// The estimate alone (per_block > 0): one block per signal, thread t taking
-// sample t of every run, then the block's fixed tree; a signal shorter than
-// kEnergyBlocks runs of per_block samples is summed whole.
-// Bound by memory latency: one block reads 512 KB (256 runs of 2 KB). A
-// thread's kEnergyBatch loads are issued together and added in run order, so
-// the sum is that of one load at a time; a load per round trip took 139 us
-// cold, and one FP32 Iterate (n = 2^22, 1001 bins) 369 us, now 288.
-constexpr int kEnergyBatch = 32;
-static_assert(kEnergyBlocks % kEnergyBatch == 0, "whole batches of runs");
+// Estimate of mean |x|^2: kEnergyParts blocks per signal, block b taking
+// kEnergyBatch of the kEnergyBlocks runs, thread t sample t of each, then the
+// block's fixed tree; energy[sig * kEnergyStride + b] = the block's share of
+// the mean. A signal shorter than kEnergyBlocks samples is summed whole by
+// block 0.
+// Bound by memory latency (512 KB in runs of 2 KB, each on a page of its own):
+// a thread's kEnergyBatch loads are issued together. One block with a load per
+// round trip took 139 us cold, one block of 8 batches 45 us, 6 us now.
+constexpr int kEnergyBatch = kEnergyBlocks / kEnergyParts;
 template <typename TX>
 __global__ void __launch_bounds__(256)
     k_energy_sample(const void *const *__restrict__ xs, const int64_t *__restrict__ ns,
                     double *__restrict__ energy, int per_block) {
   __shared__ double red[256];
-  const int sig = blockIdx.x;
+  const int sig = blockIdx.y;
   const TX *x = reinterpret_cast<const TX *>(xs[sig]);
   const int64_t n = ns[sig];
   const int64_t run = min(int64_t(per_block), n / kEnergyBlocks);
   float acc = 0.f;
   if (run > 0) {
+    const int r0 = blockIdx.x * kEnergyBatch;
     for (int64_t i = threadIdx.x; i < run; i += blockDim.x) {
-      for (int r0 = 0; r0 < kEnergyBlocks; r0 += kEnergyBatch) {
-        TX v[kEnergyBatch];
+      TX v[kEnergyBatch];
 #pragma unroll
-        for (int u = 0; u < kEnergyBatch; ++u) {
-          v[u] = x[n * (r0 + u) / kEnergyBlocks + i];
-        }
+      for (int u = 0; u < kEnergyBatch; ++u) {
+        v[u] = x[n * (r0 + u) / kEnergyBlocks + i];
+      }
 #pragma unroll
-        for (int u = 0; u < kEnergyBatch; ++u) {
-          const float re = float(v[u].x), im = float(v[u].y);
-          acc = fmaf(re, re, fmaf(im, im, acc));
-        }
+      for (int u = 0; u < kEnergyBatch; ++u) {
+        const float re = float(v[u].x), im = float(v[u].y);
+        acc = fmaf(re, re, fmaf(im, im, acc));
       }
     }
-  } else {
+  } else if (blockIdx.x == 0) {
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
       const TX v = x[i];
       const float re = float(v.x), im = float(v.y);
@@ -401,7 +344,8 @@ __global__ void __launch_bounds__(256)
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    energy[size_t(sig) * kEnergyStride] = red[0] / double(run > 0 ? run * kEnergyBlocks : n);
+    energy[size_t(sig) * kEnergyStride + blockIdx.x] =
+        red[0] / double(run > 0 ? run * kEnergyBlocks : n);
   }
 }
 
@@ -409,21 +353,12 @@ __global__ void __launch_bounds__(256)
 
 void LaunchEnergy(const void *const *x, const int64_t *n, int nsig, bool c128,
                   double *energy, cudaStream_t s, int per_block) {
-  if (per_block > 0) {
-    if (c128) {
-      k_energy_sample<double2><<<nsig, 256, 0, s>>>(x, n, energy, per_block);
-    } else {
-      k_energy_sample<float2><<<nsig, 256, 0, s>>>(x, n, energy, per_block);
-    }
-    return;
-  }
-  dim3 grid(kEnergyBlocks, nsig);
+  const dim3 grid(kEnergyParts, nsig);
   if (c128) {
-    k_energy_partial<double2><<<grid, 256, 0, s>>>(x, n, energy, 0);
+    k_energy_sample<double2><<<grid, 256, 0, s>>>(x, n, energy, per_block);
   } else {
-    k_energy_partial<float2><<<grid, 256, 0, s>>>(x, n, energy, 0);
+    k_energy_sample<float2><<<grid, 256, 0, s>>>(x, n, energy, per_block);
   }
-  k_energy_final<<<nsig, kEnergyBlocks, 0, s>>>(n, energy, 0);
 }
 
 bool WindowKernelsLaunchable() {

@@ -130,13 +130,14 @@ void LaunchExportTables(const SigIter *d_its, int nsig, int max_cap,
                         int32_t *keys, double2 *coefs, int32_t *counts,
                         int32_t *sorted, cudaStream_t s);
 
-// mean |x|^2 of each signal into energy[sig * kEnergyStride] (two
-// deterministic passes): over every sample (per_block = 0), or estimated
-// from kEnergyBlocks evenly spread runs of per_block samples.
+// Estimate of each signal's mean |x|^2 from kEnergyBlocks evenly spread runs of
+// per_block samples: the sum of energy[sig * kEnergyStride + b] over its
+// kEnergyParts entries (deterministic).
 constexpr int kEnergyBlocks = 256;
-constexpr int kEnergyStride = kEnergyBlocks + 1;
+constexpr int kEnergyParts = 8;
+constexpr int kEnergyStride = kEnergyParts;
 void LaunchEnergy(const void *const *x, const int64_t *n, int nsig, bool c128,
-                  double *energy, cudaStream_t s, int per_block = 0);
+                  double *energy, cudaStream_t s, int per_block);
 
 // Lists of table slots per bin (counting sort by bin); prep: the mode
 // preparation of LaunchModePrep first, in the same kernel.
