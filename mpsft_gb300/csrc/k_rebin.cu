@@ -19,15 +19,17 @@
 //
 // The samples x[(a (tau_r + t) + c) mod n] come from the stash the FP32 fold
 // wrote when it stashed the row (StashRows: every row when the fold gathers
-// from few sectors, else row 0), read in order, and are gathered from x
-// again otherwise (random accesses, at the random-gather rate).
+// from few sectors, else row 0), read in order; where only row 0 is stashed, a
+// chunk of another row whose window lies within row 0's (sample t of the row at
+// offset off is row 0's sample t + off) reads row 0's. The others are gathered
+// from x again (random accesses, at the random-gather rate).
 //
 // Work item = (signal, listed bin, trial, listed row, chunk of the support;
 // RebinChunks(p) chunks),
 // one warp each; the 32 lanes split the chunk into consecutive runs; lane sums
-// are combined by a fixed shuffle tree and the chunk partials are added in
-// chunk order by whichever warp finishes a row's last chunk (so the result
-// does not depend on the scheduling).
+// are combined by a fixed shuffle tree and the chunk partials by another in
+// whichever warp finishes a row's last chunk (so the result does not depend on
+// the scheduling).
 #include "common.cuh"
 #include "launch.h"
 #include "rebin.cuh"
@@ -35,6 +37,8 @@
 namespace mpsft {
 
 namespace {
+
+static_assert(kRebinChunks <= 32, "a lane per chunk partial");
 
 // x*y + u*v in float-float: exact products of the high parts (FMA), two-sum
 // of those, the cross terms in the low word, then renormalisation.
@@ -189,7 +193,10 @@ __global__ void __launch_bounds__(256, 2)
   __syncthreads();
   float4 *pw = pw_s[warp];
   const int64_t total = items_end[nsig - 1];
-  for (int64_t w = int64_t(blockIdx.x) * 8 + warp; w < total;
+  // (a row's chunks go to as many blocks: rows that are not listed leave gaps
+  // in the items, and with a row's chunks on the warps of a few blocks some SMs
+  // had three times the work of others)
+  for (int64_t w = int64_t(warp) * gridDim.x + blockIdx.x; w < total;
        w += int64_t(gridDim.x) * 8) {
     int sig = 0;
     while (w >= items_end[sig]) ++sig;
@@ -249,9 +256,11 @@ __global__ void __launch_bounds__(256, 2)
     const TX *__restrict__ sx = nullptr;
     if (it.stash != nullptr && __ldcg(reinterpret_cast<const int32_t *>(it.stash)) == 1) {
       const int srows = StashRows(it);
+      const TX *s0 = reinterpret_cast<const TX *>(it.stash + kStashHeader) + it.p2;
       if (r < srows) {
-        sx = reinterpret_cast<const TX *>(it.stash + kStashHeader) +
-             (size_t(t) * srows + r) * it.p + it.p2;
+        sx = s0 + (size_t(t) * srows + r) * it.p;
+      } else if (srows == 1 && c0 + off >= -int64_t(it.p2) && c1 - 1 + off <= it.p2) {
+        sx = s0 + size_t(t) * it.p + off;
       }
     }
     if (t0 < t1) {
@@ -285,15 +294,17 @@ __global__ void __launch_bounds__(256, 2)
       __threadfence();
       last = atomicAdd(&it.esc_cnt[etr], 1) == nch - 1;
     }
-    if (__shfl_sync(0xffffffffu, last, 0) && lane == 0) {
+    if (__shfl_sync(0xffffffffu, last, 0)) {
+      // one chunk per lane, then a fixed shuffle tree
       __threadfence();
-      double2 s = __ldcg(&it.esc_part[etr * kRebinChunks]);
-      for (int cc = 1; cc < nch; ++cc) {
-        const double2 p = __ldcg(&it.esc_part[etr * kRebinChunks + cc]);
-        s.x += p.x;
-        s.y += p.y;
+      double2 s = make_double2(0.0, 0.0);
+      if (lane < nch) s = __ldcg(&it.esc_part[etr * kRebinChunks + lane]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
       }
-      it.esc_sum[etr] = s;
+      if (lane == 0) it.esc_sum[etr] = s;
     }
   }
 }
