@@ -295,17 +295,29 @@ __host__ __device__ inline int64_t PosMod(int64_t v, int64_t n) {
   return v < 0 ? v + n : v;
 }
 
-// The fixed-point constants that depend on n and the bins only (n, bins and
-// erf_d set).
-__host__ __device__ inline void SetBinsFixedPoint(SigIter *it) {
+// The fixed-point constants that depend on n only (n set).
+__host__ __device__ inline void SetLengthFixedPoint(SigIter *it) {
   const uint64_t n = uint64_t(it->n);
   const bool pow2 = (n & (n - 1)) == 0;
   it->n_inv = pow2 ? 0 : uint64_t(((unsigned __int128)1 << 64) / n);
-  const uint64_t twoB = 2 * uint64_t(it->bins);
-  it->psi = uint64_t((((unsigned __int128)1 << 64) + twoB / 2) / twoB);
   it->n_fix = n > 1 ? uint64_t((((unsigned __int128)1 << 64) + n / 2) / n) : 0;
-  it->wf_scale = float(it->erf_d / (4.0 * double(n) * double(it->bins)));
-  it->xi_scale = 1.0 / (2.0 * double(n) * double(it->bins));
+}
+
+// psi = round(2^64 / (2 bins)) without a 128-bit division: with
+// 2^64 = q 2B + r, it is q + floor((r + B) / 2B).
+__host__ __device__ inline uint64_t PsiOf(int32_t bins) {
+  const uint64_t twoB = 2 * uint64_t(bins);
+  const uint64_t q = ~uint64_t(0) / twoB, r = ~uint64_t(0) - q * twoB + 1;
+  return q + (r + twoB / 2) / twoB;
+}
+
+// The fixed-point constants that depend on n and the bins only (n, bins and
+// erf_d set).
+__host__ __device__ inline void SetBinsFixedPoint(SigIter *it) {
+  SetLengthFixedPoint(it);
+  it->psi = PsiOf(it->bins);
+  it->wf_scale = float(it->erf_d / (4.0 * double(it->n) * double(it->bins)));
+  it->xi_scale = 1.0 / (2.0 * double(it->n) * double(it->bins));
 }
 
 // phi_b = round(2^64 (b mod n) / n) (n and b set); for n = 2^k it is exactly

@@ -1236,6 +1236,7 @@ int GraphLoop(mpsft_ctx *ctx, const mpsft_signal *const *sigs,
       while ((int64_t(1) << k) < sigs[i]->n) ++k;
       it.phase_shift = 32 - k;
     }
+    SetLengthFixedPoint(&it);
     it.trials = opts[i].trials;
     it.active = 0;
     it.trace = i == 0 ? ctx->trace : nullptr;

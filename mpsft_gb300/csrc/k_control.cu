@@ -2,7 +2,7 @@
 // src/demo1.cc:36-59), so that a whole solve runs as one CUDA graph whose
 // iteration body sits under a conditional while node.
 //
-// k_plan (before each iteration, one thread per signal) computes what the
+// k_plan (before each iteration, one warp per signal) computes what the
 // reference computes on the host at the start of Iterate: the number of bins
 // B = max(2 (k - found) + 1, min_bins), NumBits, the window scalars
 // (src/window.cc:28-51, with explicitly rounded FP64 operations so that they
@@ -49,6 +49,13 @@ __device__ inline int32_t NextBins(const SolveCtl &c, const SigIter &it) {
   return bins;
 }
 
+// One warp per signal. A new number of bins takes eight FP64 divisions and a
+// square root (about 700 cycles each on this part's FP64 pipes, whatever the
+// number of lanes): the divisions run in three stages, the independent ones of a
+// stage on different lanes, without 128-bit divisions (one thread after the
+// other: one recovery of 1000 modes 1.008x, 24 uneven ones 1.005x slower).
+// Lane 0 stores.
+//
 // max_bins: signals needing more bins wait (the launch shapes of this body
 // do not cover them). ahead = 1 plans iteration iter + 1 of a signal in the
 // fixed-bins state while iteration iter runs (bins = min_bins; the flags,
@@ -56,20 +63,53 @@ __device__ inline int32_t NextBins(const SolveCtl &c, const SigIter &it) {
 __global__ void k_plan(SolveCtl *__restrict__ ctl, SigIter *__restrict__ its,
                        int nsig, int32_t max_bins, int ahead) {
   PdlEnter(its, kTracePlan);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= nsig) return;
   SolveCtl &c = ctl[i];
   SigIter &it = its[i];
   const int local = c.iter + ahead - c.draw_base;
   if (c.done || local >= c.draws_avail) {
-    it.active = 0;
+    if (lane == 0) it.active = 0;
     return;
   }
   const int32_t bins = ahead ? c.min_bins : NextBins(c, it);
   if (bins > max_bins) {
-    it.active = 0;
+    if (lane == 0) it.active = 0;
     return;
   }
+  // Everything that depends on the bins only (and on the signal's constants)
+  // stays from the previous iteration when the bins repeat (most late
+  // iterations).
+  const bool same_bins = it.bins == bins;
+  const double B = double(bins), n = double(it.n), sigma = c.sigma;
+  double width = 0, sigma_f = 0, xi_scale = 0, sigma_t = 0, bin_thr = 0, sv_thr = 0;
+  double erf_d = 0, folds = 0, wf_scale = 0;
+  if (!same_bins) {
+    // Window scalars in the reference's operation order, no contraction.
+    const double sq = c.sqrt_c_delta;
+    const double rb = __dsqrt_rn(B);
+    // each lane one quotient of the stage (0, 1 or the rest)
+    auto div3 = [lane](double n0, double d0, double n1, double d1, double n2, double d2,
+                       double *q0, double *q1, double *q2) {
+      const double q = __ddiv_rn(lane == 0 ? n0 : (lane == 1 ? n1 : n2),
+                                 lane == 0 ? d0 : (lane == 1 ? d1 : d2));
+      *q0 = __shfl_sync(0xffffffffu, q, 0);
+      *q1 = __shfl_sync(0xffffffffu, q, 1);
+      *q2 = __shfl_sync(0xffffffffu, q, 2);
+    };
+    div3(1.0, __dmul_rn(2.0, B), 0.5,
+         __dmul_rn(__dmul_rn(__dmul_rn(B, 2.0), M_SQRT2), sq), 1.0,
+         __dmul_rn(__dmul_rn(2.0, n), B), &width, &sigma_f, &xi_scale);
+    div3(1.0, __dmul_rn(2.0 * M_PI, sigma_f), __dmul_rn(3.0, sigma), rb, sigma, rb,
+         &sigma_t, &bin_thr, &sv_thr);
+    const double tmp =
+        __dadd_rn(__dmul_rn(__dmul_rn(2.0 * M_SQRT2, sigma_t), sq), 1.0);
+    erf_d = __dmul_rn(M_SQRT2 * M_PI, sigma_t);
+    double unused;
+    div3(tmp, B, erf_d, __dmul_rn(__dmul_rn(4.0, n), B), 0.0, 1.0, &folds, &wf_scale,
+         &unused);
+  }
+  if (lane != 0) return;
   if (ahead && it.fold_alt != nullptr) {
     // the planned iteration folds (and stashes its samples) into the
     // buffers this one's row transforms and re-binning do not read
@@ -80,23 +120,8 @@ __global__ void k_plan(SolveCtl *__restrict__ ctl, SigIter *__restrict__ its,
     it.stash = it.stash_alt;
     it.stash_alt = st;
   }
-  // Everything that depends on the bins only (and on the signal's constants)
-  // stays from the previous iteration when the bins repeat (most late
-  // iterations): the window scalars, fixed-point constants and thresholds
-  // are a chain of FP64 divisions, square roots and 128-bit divisions, each a
-  // long sequence on this part.
-  const bool same_bins = it.bins == bins;
-  const double B = double(bins);
   if (!same_bins) {
-    // Window scalars in the reference's operation order, no contraction.
-    const double width = __ddiv_rn(1.0, __dmul_rn(2.0, B));
-    const double sq = c.sqrt_c_delta;
-    const double sigma_f =
-        __ddiv_rn(0.5, __dmul_rn(__dmul_rn(__dmul_rn(B, 2.0), M_SQRT2), sq));
-    const double sigma_t = __ddiv_rn(1.0, __dmul_rn(2.0 * M_PI, sigma_f));
-    const double tmp =
-        __dadd_rn(__dmul_rn(__dmul_rn(2.0 * M_SQRT2, sigma_t), sq), 1.0);
-    int32_t f = int32_t(ceil(__ddiv_rn(tmp, B)));
+    int32_t f = int32_t(ceil(folds));
     if (f % 2 == 0) ++f;
     const int32_t bits = NumBitsDev(it.n, bins);
     it.bins = bins;
@@ -107,11 +132,12 @@ __global__ void k_plan(SolveCtl *__restrict__ ctl, SigIter *__restrict__ its,
     it.p2 = (it.p - 1) / 2;
     it.width = width;
     it.sigma_f = sigma_f;
-    it.erf_d = __dmul_rn(M_SQRT2 * M_PI, sigma_t);
-    SetBinsFixedPoint(&it);
-    const double rb = __dsqrt_rn(B);
-    it.bin_thr = __ddiv_rn(__dmul_rn(3.0, c.sigma), rb);
-    it.sv_thr = __ddiv_rn(c.sigma, rb);
+    it.erf_d = erf_d;
+    it.psi = PsiOf(bins);
+    it.wf_scale = float(wf_scale);
+    it.xi_scale = xi_scale;
+    it.bin_thr = bin_thr;
+    it.sv_thr = sv_thr;
     SetThresholdCopies(&it);
     int l = 0;
     while ((1 << l) < 2 * bins - 1) ++l;
@@ -283,7 +309,8 @@ void LaunchDelay(unsigned long long ns, cudaStream_t s) {
 
 void LaunchPlan(SolveCtl *ctl, SigIter *its, int nsig, int32_t max_bins,
                 cudaStream_t s, bool ahead) {
-  Launch(k_plan, (nsig + 127) / 128, 128, 0, s, ctl, its, nsig, max_bins, ahead ? 1 : 0);
+  // a warp per signal and block: its FP64 operations get a scheduler
+  Launch(k_plan, nsig, 32, 0, s, ctl, its, nsig, max_bins, ahead ? 1 : 0);
 }
 
 void LaunchFinish(SolveCtl *ctl, SigIter *its, int nsig,
