@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 && TMAX == 1) ? 6 : 1)
 // (k_decide_listed).
 constexpr int kListedBlocks = 8;
 
-__device__ void MergeBin(const SigIter &it, int beta);
+__device__ void MergeBin(const SigIter &it, int beta, bool go);
 
 // FP64 mode subtraction of the listed bins, beside their re-binning: one
 // block of W warps per listed bin. The bin's found modes get their FP64
@@ -375,11 +375,12 @@ __global__ void __launch_bounds__(256)
     if (!redo && blockIdx.x == 0 && threadIdx.x == 0) {
       atomicOr(&it.flags[1], kStatusUnresolved);
     }
-    if (merge && threadIdx.x == 0) {
+    if (merge && threadIdx.x < 32) {
       for (int e = blockIdx.x; e < it.esc_cap; e += kListedBlocks) {
         const int beta = it.esc_list[e];
-        it.cand_valid[beta] -= kCandListed;
-        MergeBin(it, beta);
+        if (threadIdx.x == 0) it.cand_valid[beta] -= kCandListed;
+        __syncwarp();
+        MergeBin(it, beta, threadIdx.x < 2);
       }
     }
     return;
@@ -426,39 +427,50 @@ __global__ void __launch_bounds__(256)
                                -1);
     }
     // the bin's candidate (written by lane 0 above) into the table
-    if (merge && lane == 0) MergeBin(it, beta);
+    if (merge) {
+      __syncwarp();
+      MergeBin(it, beta, lane < 2);
+    }
   }
 }
 
 // ---------------------------------------------------------------- merge
-// Candidate of bin beta -> table. A pending candidate is finished here in
-// FP64 (src/iterate.cc:139-171): the window response at
-// xi0 = k1/n - (beta + 1/2)/B and its threshold, the average over the
-// T (1 + 2L) values, k0 = a^-1 (k1 - b) mod n, the factor e^{-2 pi i c k0/n}
-// and the division by the window response.
-__device__ void MergeBin(const SigIter &it, int beta) {
-  const int v = it.cand_valid[beta];
-  if (!v) return;
-  int32_t k0 = it.cand_k0[beta];
-  double2 coef = it.cand_coef[beta];
-  double err = it.cand_err[beta];
+// Candidate of bin beta -> table, by a pair of neighbouring lanes (go: this
+// lane's bin has one to merge; every lane of the warp calls). A pending
+// candidate is finished here in FP64 (src/iterate.cc:139-171): the window
+// response at xi0 = k1/n - (beta + 1/2)/B and its threshold, the average over
+// the T (1 + 2L) values, k0 = a^-1 (k1 - b) mod n, the factor e^{-2 pi i c k0/n}
+// and the division by the window response. The response's two erf, about 100
+// FP64 instructions each of 64 cycles, are much of what a merge waits for: one
+// on each lane of the pair (one recovery of 1000 modes 1055 -> 1032 us).
+__device__ void MergeBin(const SigIter &it, int beta, bool go) {
+  const int half = threadIdx.x & 1;
+  const int v = go ? it.cand_valid[beta] : 0;
+  go = v == 1 || v == 2;
+  if (!__any_sync(0xffffffffu, go)) return;
+  int32_t k0 = go ? it.cand_k0[beta] : 0;
   const ModN mod{uint32_t(it.n), it.n_inv};
   // k1 of the candidate (pending: cand_k0 holds it), and whether it lies in
   // this bin's range
   const int64_t k1 = v == 2 ? int64_t(k0) : int64_t(mod(int64_t(it.a) * k0 + it.b));
   const bool own = int64_t(mod.quot(k1 * int64_t(it.bins))) == beta;
+  // xi0 = k1/n - (beta + 1/2)/B from its exact integer numerator
+  // (|num| < 2^53) and 1/(2nB)
+  const int64_t num =
+      2 * int64_t(it.bins) * k1 - (2 * int64_t(beta) + 1) * int64_t(it.n);
+  const double xi = double(num) * it.xi_scale, c = 0.5 * it.width;
+  const double e = erf((half ? xi - c : xi + c) * it.erf_d);
+  const double wf = 0.5 * (e - __shfl_xor_sync(0xffffffffu, e, 1));
+  if (!go || half) return;
+  double2 coef = it.cand_coef[beta];
+  double err = it.cand_err[beta];
   if (v == 2) {
-    const int64_t n = it.n;
-    const int B = it.bins;
-    // xi0 = k1/n - (beta + 1/2)/B from its exact integer numerator
-    // (|num| < 2^53) and 1/(2nB); one FP64 division per candidate (each is a
-    // long sequence on this part's FP64 pipes)
-    const int64_t num = 2 * int64_t(B) * k1 - (2 * int64_t(beta) + 1) * n;
-    const double wf = WindowInFreq(it, double(num) * it.xi_scale);
     if (fabs(wf) < it.win_thr) {
       it.cand_valid[beta] = 0;
       return;
     }
+    // one FP64 division per candidate (each is a long sequence on this part's
+    // FP64 pipes)
     const double m = double(it.trials * (1 + 2 * it.bits));
     const double scale = 1.0 / (m * wf);  // the average and the window
     k0 = int32_t(mod(int64_t(it.a_inv) * mod(k1 - it.b)));
@@ -496,16 +508,14 @@ __global__ void k_insert_spills(const SigIter *__restrict__ its, int nsig) {
   if (it.active && it.flags[4] > 0) InsertSpills(it);
 }
 
-// Candidates -> table, one thread per bin; bins held back for their FP64
+// Candidates -> table, two lanes per bin; bins held back for their FP64
 // near-tie decision (cand_valid >= kCandListed) are merged by that decision.
-__global__ void k_merge(const SigIter *__restrict__ its) {
+__global__ void __launch_bounds__(32) k_merge(const SigIter *__restrict__ its) {
   PdlEnter(its, kTraceMerge);
   const SigIter &it = its[blockIdx.y];
   if (!it.active) return;
-  const int beta = blockIdx.x * blockDim.x + threadIdx.x;
-  if (beta >= it.bins) return;
-  if (it.cand_valid[beta] >= kCandListed) return;
-  MergeBin(it, beta);
+  const int beta = blockIdx.x * 16 + (threadIdx.x >> 1);
+  MergeBin(it, beta, beta < it.bins);
 }
 
 __global__ void k_table_insert(const SigIter *__restrict__ it,
@@ -704,9 +714,9 @@ void LaunchListedTerms(const SigIter *d_its, int nsig, int max_trials, cudaStrea
 
 void LaunchMerge(const SigIter *d_its, int nsig, int max_bins,
                  cudaStream_t s) {
-  // a warp per block: a candidate's two FP64 erf and its division bind the
-  // SM's FP64 pipes (1001 bins of one signal: 19 us on 4 SMs of 256 threads)
-  dim3 grid((max_bins + 31) / 32, nsig);
+  // a warp per block: a candidate's FP64 operations bind the SM's FP64 pipes
+  // (1001 bins of one signal: 19 us on 4 SMs of 256 threads)
+  dim3 grid((max_bins + 15) / 16, nsig);
   Launch(k_merge, grid, 32, 0, s, d_its);
 }
 
