@@ -329,6 +329,22 @@ void CarveSignal(Carve &cv, const Shape &s, SigIter *it, int32_t **ctl) {
   it->bins_cap = s.bins_cap;
 }
 
+// The host inputs of a single-signal call (its descriptor, modes, gradients)
+// gathered for one copy to the device. Lives until the call's wait.
+struct Inputs {
+  std::vector<unsigned char> bytes;
+  static size_t Up(size_t v) { return (v + 255) & ~size_t(255); }
+  // reserves room and returns its offset (Put fills it)
+  size_t Room(size_t n) {
+    const size_t off = Up(bytes.size());
+    bytes.resize(off + n);
+    return off;
+  }
+  void Put(size_t off, const void *src, size_t n) {
+    if (n > 0) std::memcpy(bytes.data() + off, src, n);
+  }
+};
+
 int EnsureArena(mpsft_ctx *ctx, size_t bytes) {
   if (ctx->arena_size >= bytes) return MPSFT_OK;
   if (ctx->arena) {
@@ -2489,6 +2505,19 @@ int BinInTimeImpl(mpsft_ctx *ctx, const mpsft_signal *sig, int32_t bins,
   const Transform tf{a, b, c, InverseMod(a, n)};
   FillIter(&it, sig, bins, bits, w, tf, &q, 1);
   cudaStream_t st = ctx->stream;
+  // the row transform writes the caller's device buffer itself when it may:
+  // this device's memory, aligned for whole bins (bins_cap = bins: the rows are
+  // adjacent)
+  bool in_place = false;
+  if (out_on_device && !direct && reinterpret_cast<uintptr_t>(out) % sizeof(double2) == 0) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, out) == cudaSuccess) {
+      in_place = at.type == cudaMemoryTypeDevice && at.device == ctx->device;
+    } else {
+      cudaGetLastError();
+    }
+    if (in_place) it.ubuf = reinterpret_cast<double2 *>(out);
+  }
   // the window and Bluestein tables: the context's, evaluated on the device
   // when they are new, or (window) the caller's uploaded
   bool new_window = true, new_blue = true;
@@ -2568,11 +2597,12 @@ int BinInTimeImpl(mpsft_ctx *ctx, const mpsft_signal *sig, int32_t bins,
   LaunchRowFFT(d_it, 1, it.rows, 1, it.fft_m, fp64, ctx->tw32, ctx->tw64, st, false,
                true);
   MPSFT_CUDA(ctx, cudaGetLastError());
-  // (bins_cap = bins: the rows are adjacent)
-  MPSFT_CUDA(ctx, cudaMemcpyAsync(
-                      out, it.ubuf, sizeof(double2) * size_t(bins) * it.rows,
-                      out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
-                      st));
+  if (!in_place) {
+    MPSFT_CUDA(ctx, cudaMemcpyAsync(
+                        out, it.ubuf, sizeof(double2) * size_t(bins) * it.rows,
+                        out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
+                        st));
+  }
   MPSFT_CUDA(ctx, cudaStreamSynchronize(st));
   CommitTables(ctx);
   if (ctx->profiling) {
@@ -2632,15 +2662,17 @@ int BinInFreqImpl(mpsft_ctx *ctx, int32_t n, int32_t bins, int32_t bits,
   SigIter it{};
   int32_t *ctl;
   CarveSignal(probe, s, &it, &ctl);
-  const size_t extra = size_t(m) * (sizeof(int32_t) + sizeof(double2)) + 1024;
-  rc = EnsureArena(ctx, probe.off + sizeof(SigIter) + extra);
+  // one copy: the descriptor and the modes
+  Inputs in;
+  const size_t o_it = in.Room(sizeof(SigIter)), o_k0 = in.Room(sizeof(int32_t) * size_t(m)),
+               o_coef = in.Room(sizeof(double2) * size_t(m));
+  rc = EnsureArena(ctx, probe.off + in.bytes.size() + 1024);
   if (rc) return rc;
   Carve cv{ctx->arena};
-  SigIter *d_it = cv.take<SigIter>(1);
+  unsigned char *d_in = cv.take<unsigned char>(in.bytes.size());
+  SigIter *d_it = reinterpret_cast<SigIter *>(d_in + o_it);
   std::memset(&it, 0, sizeof(it));
   CarveSignal(cv, s, &it, &ctl);
-  int32_t *d_k0 = cv.take<int32_t>(size_t(m));
-  double2 *d_coef = cv.take<double2>(size_t(m));
   const Transform tf{a, b, c, 0};
   mpsft_signal fake;
   fake.n = n;
@@ -2652,45 +2684,32 @@ int BinInFreqImpl(mpsft_ctx *ctx, int32_t n, int32_t bins, int32_t bits,
   cudaStream_t st = ctx->stream;
   BeginTables(ctx);
   const bool new_phases = UsePhases(ctx, &it);
-  MPSFT_CUDA(ctx, cudaMemcpyAsync(d_it, &it, sizeof(it), cudaMemcpyHostToDevice,
-                                  st));
-  if (new_phases) LaunchPhaseTables(d_it, 1, PhaseTableEntries(n), st);
-  LaunchClearTables(d_it, 1, it.tab_cap, st);
-  if (m > 0) {
-    MPSFT_CUDA(ctx, cudaMemcpyAsync(d_k0, k0, sizeof(int32_t) * m,
-                                    cudaMemcpyHostToDevice, st));
-    std::vector<double> wc;
-    const double *src = coef;
-    if (wf) {
-      // wf * coef, the reference's first product (src/binner.cc:580)
-      wc.resize(2 * size_t(m));
-      for (int64_t i = 0; i < m; ++i) {
-        wc[2 * i] = coef[2 * i] * wf[i];
-        wc[2 * i + 1] = coef[2 * i + 1] * wf[i];
-      }
-      src = wc.data();
+  in.Put(o_it, &it, sizeof(it));
+  in.Put(o_k0, k0, sizeof(int32_t) * size_t(m));
+  in.Put(o_coef, coef, sizeof(double2) * size_t(m));
+  if (wf) {
+    // wf * coef, the reference's first product (src/binner.cc:580)
+    double *wc = reinterpret_cast<double *>(in.bytes.data() + o_coef);
+    for (int64_t i = 0; i < m; ++i) {
+      wc[2 * i] = coef[2 * i] * wf[i];
+      wc[2 * i + 1] = coef[2 * i + 1] * wf[i];
     }
-    MPSFT_CUDA(ctx, cudaMemcpyAsync(d_coef, src, sizeof(double2) * m,
-                                    cudaMemcpyHostToDevice, st));
-    LaunchTableInsert(d_it, d_k0, d_coef, m, st);
-    // the pageable source must outlive the copy
-    if (wf) MPSFT_CUDA(ctx, cudaStreamSynchronize(st));
   }
+  MPSFT_CUDA(ctx, cudaMemcpyAsync(d_in, in.bytes.data(), in.bytes.size(),
+                                  cudaMemcpyHostToDevice, st));
+  if (new_phases) LaunchPhaseTables(d_it, 1, PhaseTableEntries(n), st);
+  LaunchTableLoad(d_it, reinterpret_cast<const int32_t *>(d_in + o_k0),
+                  reinterpret_cast<const double2 *>(d_in + o_coef), m, st);
   // (bins_cap = bins: the rows are adjacent)
   const size_t u_bytes = sizeof(double2) * size_t(bins) * it.rows;
   MPSFT_CUDA(ctx, cudaMemcpyAsync(it.ubuf, inout, u_bytes, cudaMemcpyHostToDevice, st));
   LaunchBucket(d_it, 1, bins, s.tab_cap, st, true);
   LaunchDecide(d_it, 1, bins, 1, false, true, st);
   MPSFT_CUDA(ctx, cudaGetLastError());
+  // (the table has two slots per mode at least: it cannot fill up)
   MPSFT_CUDA(ctx, cudaMemcpyAsync(inout, it.ubuf, u_bytes, cudaMemcpyDeviceToHost, st));
-  int32_t h_ctl[kCtlWords];
-  MPSFT_CUDA(ctx, cudaMemcpyAsync(h_ctl, ctl, sizeof(h_ctl),
-                                  cudaMemcpyDeviceToHost, st));
   MPSFT_CUDA(ctx, cudaStreamSynchronize(st));
   CommitTables(ctx);
-  if (h_ctl[1] & kStatusCapacity) {
-    return Fail(ctx, MPSFT_ERR_CAPACITY, "mode table full");
-  }
   return MPSFT_OK;
 }
 
@@ -2738,12 +2757,14 @@ int mpsft_bin_in_freq_wf(mpsft_ctx *ctx, int32_t n, int32_t bins, int32_t bits,
 namespace {
 
 // Shared setup of mpsft_estimate / mpsft_adjoint: validates, carves one
-// signal's buffers plus `extra` bytes, fills and uploads the descriptor, and
+// signal's buffers plus `extra` bytes, fills and uploads the descriptor, the m
+// k0 and (adjoint) g in one copy (in, kept by the caller until its wait), and
 // builds the modulated window and what the context does not hold yet of the
 // FP64 window, Bluestein and unit-phase tables.
 int EstimateSetup(mpsft_ctx *ctx, int32_t n, const void *x,
-                  const mpsft_estimate_setup *su, size_t extra, Carve *cv,
-                  SigIter *it, SigIter **d_it) {
+                  const mpsft_estimate_setup *su, const int32_t *k0, int64_t m,
+                  const double *g, size_t extra, Inputs *in, Carve *cv, SigIter *it,
+                  SigIter **d_it, const int32_t **d_k0, const double2 **d_g) {
   if (!su) return Fail(ctx, MPSFT_ERR_INVALID, "null setup");
   int rc = CheckN(ctx, n);
   if (rc) return rc;
@@ -2769,10 +2790,16 @@ int EstimateSetup(mpsft_ctx *ctx, int32_t n, const void *x,
   SigIter tmp{};
   int32_t *ctl;
   CarveSignal(probe, s, &tmp, &ctl);
-  rc = EnsureArena(ctx, probe.off + sizeof(SigIter) + extra + 4096);
+  const size_t o_it = in->Room(sizeof(SigIter)),
+               o_k0 = in->Room(sizeof(int32_t) * size_t(m)),
+               o_g = in->Room(g ? sizeof(double2) * size_t(m) : 0);
+  rc = EnsureArena(ctx, probe.off + in->bytes.size() + extra + 4096);
   if (rc) return rc;
   *cv = Carve{ctx->arena};
-  *d_it = cv->take<SigIter>(1);
+  unsigned char *d_in = cv->take<unsigned char>(in->bytes.size());
+  *d_it = reinterpret_cast<SigIter *>(d_in + o_it);
+  *d_k0 = reinterpret_cast<const int32_t *>(d_in + o_k0);
+  if (d_g) *d_g = reinterpret_cast<const double2 *>(d_in + o_g);
   std::memset(it, 0, sizeof(*it));
   CarveSignal(*cv, s, it, &ctl);
   mpsft_signal fake{};
@@ -2786,7 +2813,10 @@ int EstimateSetup(mpsft_ctx *ctx, int32_t n, const void *x,
   const bool new_phases = UsePhases(ctx, it);
   const bool new_window = UseWindow(ctx, it, su->window_delta, kTabWin64);
   const bool new_blue = UseBluestein(ctx, it, true, false);
-  MPSFT_CUDA(ctx, cudaMemcpyAsync(*d_it, it, sizeof(SigIter),
+  in->Put(o_it, it, sizeof(SigIter));
+  in->Put(o_k0, k0, sizeof(int32_t) * size_t(m));
+  if (g) in->Put(o_g, g, sizeof(double2) * size_t(m));
+  MPSFT_CUDA(ctx, cudaMemcpyAsync(d_in, in->bytes.data(), in->bytes.size(),
                                   cudaMemcpyHostToDevice, st));
   if (new_phases) LaunchPhaseTables(*d_it, 1, PhaseTableEntries(n), st);
   LaunchWindowMod(*d_it, 1, su->bins, new_window, false, st);
@@ -2819,21 +2849,18 @@ int mpsft_estimate(mpsft_ctx *ctx, const mpsft_signal *sig,
   Carve cv{nullptr};
   SigIter it;
   SigIter *d_it = nullptr;
-  const size_t extra = size_t(m) * (sizeof(int32_t) + sizeof(double2)) + 1024;
-  rc = EstimateSetup(ctx, int32_t(sig->n), sig->d_x, setup, extra, &cv, &it, &d_it);
+  Inputs in;
+  const int32_t *d_k0 = nullptr;
+  rc = EstimateSetup(ctx, int32_t(sig->n), sig->d_x, setup, k0, m, nullptr,
+                     size_t(m) * sizeof(double2), &in, &cv, &it, &d_it, &d_k0, nullptr);
   if (rc) return rc;
-  int32_t *d_k0 = cv.take<int32_t>(size_t(m));
   double2 *d_coef = cv.take<double2>(size_t(m));
   cudaStream_t st = ctx->stream;
   LaunchBinFold(d_it, 1, it.bins, it.bits, it.trials, sig->dtype == MPSFT_C128,
                 true, st);
   LaunchRowFFT(d_it, 1, it.rows, it.trials, it.fft_m, true, ctx->tw32, ctx->tw64,
                st);
-  if (m > 0) {
-    MPSFT_CUDA(ctx, cudaMemcpyAsync(d_k0, k0, sizeof(int32_t) * m,
-                                    cudaMemcpyHostToDevice, st));
-    LaunchEstimate(d_it, d_k0, m, d_coef, st);
-  }
+  LaunchEstimate(d_it, d_k0, m, d_coef, st);
   MPSFT_CUDA(ctx, cudaGetLastError());
   if (m > 0) {
     MPSFT_CUDA(ctx, cudaMemcpyAsync(coef, d_coef, sizeof(double2) * m,
@@ -2852,23 +2879,18 @@ int mpsft_adjoint(mpsft_ctx *ctx, int32_t n, const mpsft_estimate_setup *setup,
   Carve cv{nullptr};
   SigIter it;
   SigIter *d_it = nullptr;
-  const size_t extra = size_t(m) * (sizeof(int32_t) + sizeof(double2)) +
-                       sizeof(double2) * size_t(n) + 1024;
-  int rc = EstimateSetup(ctx, n, nullptr, setup, extra, &cv, &it, &d_it);
+  Inputs in;
+  const int32_t *d_k0 = nullptr;
+  const double2 *d_g = nullptr;
+  int rc = EstimateSetup(ctx, n, nullptr, setup, k0, m, g,
+                         sizeof(double2) * size_t(n > 0 ? n : 0), &in, &cv, &it, &d_it,
+                         &d_k0, &d_g);
   if (rc) return rc;
-  int32_t *d_k0 = cv.take<int32_t>(size_t(m));
-  double2 *d_g = cv.take<double2>(size_t(m));
   double2 *d_dx = cv.take<double2>(size_t(n));
   cudaStream_t st = ctx->stream;
   const int64_t cells = int64_t(it.trials) * it.rows * it.bins_cap;
   MPSFT_CUDA(ctx, cudaMemsetAsync(it.fold, 0, sizeof(double2) * cells, st));
   MPSFT_CUDA(ctx, cudaMemsetAsync(d_dx, 0, sizeof(double2) * size_t(n), st));
-  if (m > 0) {
-    MPSFT_CUDA(ctx, cudaMemcpyAsync(d_k0, k0, sizeof(int32_t) * m,
-                                    cudaMemcpyHostToDevice, st));
-    MPSFT_CUDA(ctx, cudaMemcpyAsync(d_g, g, sizeof(double2) * m,
-                                    cudaMemcpyHostToDevice, st));
-  }
   LaunchAdjointSpread(d_it, d_k0, d_g, m, st);
   // inverse DFT of every row as conj(DFT(conj(G)))
   LaunchRowFFT(d_it, 1, it.rows, it.trials, it.fft_m, true, ctx->tw32, ctx->tw64,
@@ -2964,21 +2986,23 @@ int IterateImpl(mpsft_ctx *ctx, const mpsft_signal *sig,
   const size_t entries = size_t(m0) + size_t(bins);
   const size_t off_keys = 256, off_coefs = off_keys + ((4 * entries + 255) & ~size_t(255));
   const size_t res_bytes = off_coefs + sizeof(double2) * entries;
-  const size_t extra = size_t(m0) * (sizeof(int32_t) + sizeof(double2)) +
-                       sizeof(double) * kEnergyStride + res_bytes + 4096;
-  rc = EnsureArena(ctx, probe.off + sizeof(SigIter) + extra);
+  // one copy: the descriptor, the signal's pointer and length, the modes
+  Inputs in;
+  const size_t o_it = in.Room(sizeof(SigIter)), o_xs = in.Room(sizeof(void *)),
+               o_ns = in.Room(sizeof(int64_t)),
+               o_k0 = in.Room(sizeof(int32_t) * size_t(m0)),
+               o_coef = in.Room(sizeof(double2) * size_t(m0));
+  rc = EnsureArena(ctx, probe.off + in.bytes.size() + sizeof(double) * kEnergyStride +
+                            res_bytes + 4096);
   if (rc) return rc;
   rc = EnsureHostStage(ctx, res_bytes);
   if (rc) return rc;
   Carve cv{ctx->arena};
-  SigIter *d_it = cv.take<SigIter>(1);
+  unsigned char *d_in = cv.take<unsigned char>(in.bytes.size());
+  SigIter *d_it = reinterpret_cast<SigIter *>(d_in + o_it);
   std::memset(&it, 0, sizeof(it));
   CarveSignal(cv, s, &it, &ctl);
-  int32_t *d_k0 = cv.take<int32_t>(size_t(m0));
-  double2 *d_coef = cv.take<double2>(size_t(m0));
   double *d_energy = cv.take<double>(kEnergyStride);
-  const void **d_xs = cv.take<const void *>(1);
-  int64_t *d_ns = cv.take<int64_t>(1);
   unsigned char *d_res = cv.take<unsigned char>(res_bytes);
   Transform tf;
   int32_t q[kMaxTrials];
@@ -2998,27 +3022,24 @@ int IterateImpl(mpsft_ctx *ctx, const mpsft_signal *sig,
   BeginTables(ctx);
   const bool new_phases = UsePhases(ctx, &it);
   // the mode table is cleared and filled while the host waits for the energy
-  MPSFT_CUDA(ctx, cudaMemcpyAsync(d_it, &it, sizeof(it), cudaMemcpyHostToDevice,
-                                  st));
+  const void *h_x = sig->d_x;
+  const int64_t h_n = sig->n;
+  in.Put(o_it, &it, sizeof(it));
+  in.Put(o_xs, &h_x, sizeof(h_x));
+  in.Put(o_ns, &h_n, sizeof(h_n));
+  in.Put(o_k0, mm_k, sizeof(int32_t) * size_t(m0));
+  in.Put(o_coef, mm_c, sizeof(double2) * size_t(m0));
+  MPSFT_CUDA(ctx, cudaMemcpyAsync(d_in, in.bytes.data(), in.bytes.size(),
+                                  cudaMemcpyHostToDevice, st));
   std::vector<double> energy(1, 0.0);
   if (!fp64) {
-    const void *h_x = sig->d_x;
-    const int64_t h_n = sig->n;
-    MPSFT_CUDA(ctx, cudaMemcpyAsync(d_xs, &h_x, sizeof(h_x),
-                                    cudaMemcpyHostToDevice, st));
-    MPSFT_CUDA(ctx, cudaMemcpyAsync(d_ns, &h_n, sizeof(h_n),
-                                    cudaMemcpyHostToDevice, st));
-    LaunchEnergy(d_xs, d_ns, 1, sig->dtype == MPSFT_C128, d_energy, st, kPolicySample);
+    LaunchEnergy(reinterpret_cast<const void *const *>(d_in + o_xs),
+                 reinterpret_cast<const int64_t *>(d_in + o_ns), 1,
+                 sig->dtype == MPSFT_C128, d_energy, st, kPolicySample);
   }
   if (new_phases) LaunchPhaseTables(d_it, 1, PhaseTableEntries(n), st);
-  LaunchClearTables(d_it, 1, it.tab_cap, st);
-  if (m0 > 0) {
-    MPSFT_CUDA(ctx, cudaMemcpyAsync(d_k0, mm_k, sizeof(int32_t) * m0,
-                                    cudaMemcpyHostToDevice, st));
-    MPSFT_CUDA(ctx, cudaMemcpyAsync(d_coef, mm_c, sizeof(double2) * m0,
-                                    cudaMemcpyHostToDevice, st));
-    LaunchTableInsert(d_it, d_k0, d_coef, m0, st);
-  }
+  LaunchTableLoad(d_it, reinterpret_cast<const int32_t *>(d_in + o_k0),
+                  reinterpret_cast<const double2 *>(d_in + o_coef), m0, st);
   if (!fp64) {
     rc = ReadEnergy(ctx, d_energy, 1, &energy);
     if (rc) return rc;

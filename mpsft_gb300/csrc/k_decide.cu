@@ -518,12 +518,22 @@ __global__ void __launch_bounds__(32) k_merge(const SigIter *__restrict__ its) {
   MergeBin(it, beta, beta < it.bins);
 }
 
-__global__ void k_table_insert(const SigIter *__restrict__ it,
-                               const int32_t *__restrict__ k0,
-                               const double2 *__restrict__ coef, int64_t m) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  InsertMode(*it, k0[i], coef[i], 0.0);
+// One signal's mode table emptied, its control words cleared and the given
+// (k0, coef) pairs added to it, by one block: the pairs wait only for the
+// block's barrier, not for a kernel of their own.
+__global__ void __launch_bounds__(1024) k_table_load(const SigIter *__restrict__ its,
+                                                     const int32_t *__restrict__ k0,
+                                                     const double2 *__restrict__ coef,
+                                                     int64_t m) {
+  const SigIter &it = *its;
+  for (int i = threadIdx.x; i < it.tab_cap; i += blockDim.x) {
+    it.tab_key[i] = kEmptyKey;
+    it.tab_coef[i] = make_double2(0.0, 0.0);
+    it.tab_err[i] = 0.0;
+  }
+  if (threadIdx.x < kCtlWords) it.flags[threadIdx.x] = 0;
+  __syncthreads();
+  for (int64_t i = threadIdx.x; i < m; i += blockDim.x) InsertMode(it, k0[i], coef[i], 0.0);
 }
 
 __global__ void k_pencil(const double2 *__restrict__ u3, int64_t count,
@@ -724,10 +734,9 @@ void LaunchInsertSpills(const SigIter *d_its, int nsig, cudaStream_t s) {
   Launch(k_insert_spills, (nsig + 127) / 128, 128, 0, s, d_its, nsig);
 }
 
-void LaunchTableInsert(const SigIter *d_it, const int32_t *k0,
-                       const double2 *coef, int64_t m, cudaStream_t s) {
-  if (m <= 0) return;
-  k_table_insert<<<unsigned((m + 255) / 256), 256, 0, s>>>(d_it, k0, coef, m);
+void LaunchTableLoad(const SigIter *d_it, const int32_t *k0, const double2 *coef,
+                     int64_t m, cudaStream_t s) {
+  k_table_load<<<1, 1024, 0, s>>>(d_it, k0, coef, m);
 }
 
 void LaunchPencil(const double2 *u3, int64_t count, double *sigma,

@@ -179,9 +179,10 @@ void LaunchListedTerms(const SigIter *d_its, int nsig, int max_trials, cudaStrea
 // iterations that no k_finish follows.
 void LaunchInsertSpills(const SigIter *d_its, int nsig, cudaStream_t s);
 
-// Inserts / accumulates explicit (k0, coef) pairs into one signal's table.
-void LaunchTableInsert(const SigIter *d_it, const int32_t *k0,
-                       const double2 *coef, int64_t m, cudaStream_t s);
+// One signal's table emptied, its control words cleared and m (k0, coef) pairs
+// added to it.
+void LaunchTableLoad(const SigIter *d_it, const int32_t *k0, const double2 *coef,
+                     int64_t m, cudaStream_t s);
 
 // Device-side control of a solve: iteration planning and the stop rule
 // (sets the while condition of the solve graph when set_condition).

@@ -732,3 +732,46 @@ def test_single_call_tables(ctx):
             assert np.array_equal(out[j], got[i][j])
         c.close()
     kept.close()
+
+
+@pytest.mark.parametrize("count", [1, 1023, 1025, 4096, 4097, 9000])
+def test_bin_in_freq_many_modes(ctx, port, count):
+    """The modes' sort by bin with fewer and more modes than a block's threads
+    and than its threads keep at hand, against the oracle (1e-12 of max|U|)."""
+    n, bins, bits = 1 << 18, 501, 3
+    rng = np.random.default_rng(count)
+    k = rng.choice(n, count, replace=False).astype(np.int32)
+    coef = rng.standard_normal(count) + 1j * rng.standard_normal(count)
+    u = rng.standard_normal((1 + 2 * bits, bins)) * (1 + 0.5j)
+    got = ctx.bin_in_freq(u, n, bins, bits, 1e-5, 77777, 5, 9, 991, k, coef)
+    want = port.bin_in_freq(u, n, bins, bits, 1e-5, 77777, 5, 9, 991, k, coef)
+    assert rel_err(got, want) < 1e-12
+
+
+@pytest.mark.parametrize("prec", PRECS, ids=PREC_IDS)
+@pytest.mark.parametrize("bins", [51, 501])
+def test_bins_on_the_device(ctx, prec, bins):
+    """Bins left on the device, written in place (aligned) or copied (a buffer
+    that is not aligned for whole bins), equal those returned to the host bit
+    for bit, and nothing around the buffer changes."""
+    import ctypes
+
+    import torch
+
+    n, bits = 1 << 14, 6
+    rng = np.random.default_rng(bins)
+    x = (rng.standard_normal(n) + 1j * rng.standard_normal(n)).astype(np.complex64)
+    sig = ctx.upload(x)
+    want = ctx.bin_in_time(sig, bins, bits, 1e-5, 77, 5, 9, 31, precision=prec)
+    size = 2 * want.size
+    for skip in (2, 1):
+        buf = torch.full((size + 8,), 7.25, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        rc = m.load_library().mpsft_bin_in_time(
+            ctx._h, sig._h, bins, bits, 1e-5, 77, 5, 9, 31, prec,
+            ctypes.c_void_p(buf.data_ptr() + 8 * skip), 1)
+        assert rc == m.OK
+        got = buf.cpu().numpy()
+        assert np.array_equal(got[skip:skip + size], want.view(np.float64).ravel())
+        assert (got[:skip] == 7.25).all() and (got[skip + size:] == 7.25).all()
+    sig.free()
