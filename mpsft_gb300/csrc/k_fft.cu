@@ -48,8 +48,10 @@ __device__ __forceinline__ float2 MulPhaseFF(float2 y, float2 bh, float2 bl) {
                      DotRound(y.x, bh.y, y.y, bh.x, bl.y, bl.x));
 }
 
-// cond: only signals whose iteration is redone in FP64 take part. Also
-// records the largest |U| of each row (used by the FP32 near-tie bound).
+// cond: only signals whose iteration is redone in FP64 take part. The FP32
+// transform also records the mean |U|^2 and the largest |U| of each row (for the
+// near-tie bound; an FP64 square root per output and what goes with it were a
+// seventh of the FP64 transform's operations).
 //
 // Rows per block: small transforms share a block, RowsPerBlock(M) rows side by
 // side (M/8 threads each for the radix-8 passes), so that late iterations
@@ -212,10 +214,14 @@ __global__ void __launch_bounds__(kRowFftThreads)
       }
     }
   } else if (live) {
+    // FP64 (row factor, power-of-two scale and all in FP64 operations, the
+    // fewest: no magnitudes, which only the FP32 near-tie bound reads), or FP32
+    // bins widened
     const double inv_m = 1.0 / double(M);
-    const double2 bq = sizeof(V) == sizeof(double2)
-                           ? it.row_fac[tr * it.rows + row]
-                           : make_double2(it.bq_re[tr], it.bq_im[tr]);
+    const double2 f = sizeof(V) == sizeof(double2)
+                          ? it.row_fac[tr * it.rows + row]
+                          : make_double2(it.bq_re[tr], it.bq_im[tr]);
+    const double2 bq = cscale(f, inv_m);
     double2 *dst = it.ubuf + (size_t(tr) * it.rows + row) * it.bins_cap;
     for (int k0 = tid; k0 < B; k0 += 8 * nth) {
       V w[8];
@@ -228,36 +234,42 @@ __global__ void __launch_bounds__(kRowFftThreads)
       for (int u = 0; u < 8; ++u) {
         const int k = k0 + u * nth;
         if (k < B) {
-          const double2 y = cscale(to_d2(vmul(conv_out(k), w[u])), inv_m);
-          dst[k] = vmul(bq, y);
-          const double y2 = y.x * y.x + y.y * y.y;
-          ss += float(y2);
-          mx = fmaxf(mx, float(sqrt(y2)));
+          if constexpr (sizeof(V) == sizeof(double2)) {
+            dst[k] = vmul(bq, vmul(conv_out(k), w[u]));
+          } else {
+            const double2 y = cscale(to_d2(vmul(conv_out(k), w[u])), inv_m);
+            dst[k] = vmul(f, y);
+            const double y2 = y.x * y.x + y.y * y.y;
+            ss += float(y2);
+            mx = fmaxf(mx, float(sqrt(y2)));
+          }
         }
       }
     }
   }
-  // the row's sum of |U|^2 in a fixed order: a shuffle tree over segments of
-  // min(nth, 32) threads (a row's threads are consecutive, nth a power of
-  // two), then the row's segments in order
-  __shared__ float seg_ss[kRowFftThreads / 8];
-  const int seg = nth < 32 ? nth : 32;
-  for (int o = seg >> 1; o > 0; o >>= 1) {
-    ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  }
-  if ((threadIdx.x & (seg - 1)) == 0) {
-    seg_ss[threadIdx.x / seg] = ss;
-    // non-negative floats order like their bit patterns
-    if (live) atomicMax(&row_max_bits[lr], __float_as_uint(mx));
-  }
-  __syncthreads();  // (rows past the last only reach the barriers)
-  if (live && tid == 0 && it.row_max != nullptr) {
-    it.row_max[tr * it.rows + row] = __uint_as_float(row_max_bits[lr]);
-    const int nseg = nth / seg;
-    float t = 0.f;
-    for (int j = 0; j < nseg; ++j) t += seg_ss[lr * nseg + j];
-    it.row_ms[tr * it.rows + row] = t / float(B);
+  if constexpr (sizeof(V) == sizeof(float2)) {
+    // the row's sum of |U|^2 in a fixed order: a shuffle tree over segments of
+    // min(nth, 32) threads (a row's threads are consecutive, nth a power of
+    // two), then the row's segments in order
+    __shared__ float seg_ss[kRowFftThreads / 8];
+    const int seg = nth < 32 ? nth : 32;
+    for (int o = seg >> 1; o > 0; o >>= 1) {
+      ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if ((threadIdx.x & (seg - 1)) == 0) {
+      seg_ss[threadIdx.x / seg] = ss;
+      // non-negative floats order like their bit patterns
+      if (live) atomicMax(&row_max_bits[lr], __float_as_uint(mx));
+    }
+    __syncthreads();  // (rows past the last only reach the barriers)
+    if (live && tid == 0 && it.row_max != nullptr) {
+      it.row_max[tr * it.rows + row] = __uint_as_float(row_max_bits[lr]);
+      const int nseg = nth / seg;
+      float t = 0.f;
+      for (int j = 0; j < nseg; ++j) t += seg_ss[lr * nseg + j];
+      it.row_ms[tr * it.rows + row] = t / float(B);
+    }
   }
 }
 
@@ -278,8 +290,8 @@ __global__ void __launch_bounds__(kRowFftThreads)
 constexpr int kSplitThreads = 256;
 constexpr int kSplitMin = 64;  // elements per slice at least
 
-// Output j of the row's transform times the row factor: FP64 bins, FP32 bins
-// widened, or (solves and iterations) complex64 bins.
+// Output j of the row's transform times the row factor: FP64 bins (f scaled by
+// 1 / M), FP32 bins widened, or (solves and iterations) complex64 bins.
 __device__ __forceinline__ void StoreBin(const SigIter &it, int tr, int row, int j, double2 y,
                                          float2, float2, double2 f) {
   it.ubuf[(size_t(tr) * it.rows + row) * it.bins_cap + j] = vmul(f, y);
@@ -295,7 +307,7 @@ __device__ __forceinline__ void StoreBin(const SigIter &it, int tr, int row, int
 }
 
 // One row of one block of the cluster: fill, local stages, exchange, epilogue;
-// adds this thread's share to the sum and the maximum of |U|^2.
+// FP32 adds this thread's share to the sum and the maximum of |U|^2.
 template <typename V, int C>
 __device__ __forceinline__ void SplitRow(const SigIter &it, int tr, int row, int c,
                                          cooperative_groups::cluster_group cl, V *a,
@@ -345,12 +357,12 @@ __device__ __forceinline__ void SplitRow(const SigIter &it, int tr, int row, int
             ChatOf(it, (V *)nullptr) + size_t(c) * Ms, tw, tid, kSplitThreads);
   cl.sync();  // every slice is done
   if (work) {
-    const double2 f = kF64 ? it.row_fac[tr * it.rows + row]
+    const double2 f = kF64 ? cscale(it.row_fac[tr * it.rows + row], 1.0 / double(M))
                            : make_double2(it.bq_re[tr], it.bq_im[tr]);
     const float2 bh = make_float2(__double2float_rn(f.x), __double2float_rn(f.y));
     const float2 bl = make_float2(__double2float_rn(f.x - double(bh.x)),
                                   __double2float_rn(f.y - double(bh.y)));
-    const decltype(a->x) inv_m = decltype(a->x)(1) / decltype(a->x)(M);
+    const float inv_m = 1.f / float(M);
     const V *part[C];
 #pragma unroll
     for (int i = 0; i < C; ++i) part[i] = C > 1 ? cl.map_shared_rank(a, i) : a;
@@ -377,12 +389,16 @@ __device__ __forceinline__ void SplitRow(const SigIter &it, int tr, int row, int
         const int j = k + i * Ms;
         if (j < B) {
           V y = vmul(x[i], __ldg(&chirp[j]));
-          y.x *= inv_m;  // (a power of two: exact)
-          y.y *= inv_m;
-          StoreBin(it, tr, row, j, y, bh, bl, f);
-          const auto y2 = y.x * y.x + y.y * y.y;
-          *ss += float(y2);
-          *mx = fmaxf(*mx, float(sqrt(y2)));
+          if constexpr (kF64) {
+            StoreBin(it, tr, row, j, y, bh, bl, f);
+          } else {
+            y.x *= inv_m;  // (a power of two: exact)
+            y.y *= inv_m;
+            StoreBin(it, tr, row, j, y, bh, bl, f);
+            const float y2 = y.x * y.x + y.y * y.y;
+            *ss += y2;
+            *mx = fmaxf(*mx, sqrtf(y2));
+          }
         }
       }
     }
@@ -410,34 +426,38 @@ __global__ void __launch_bounds__(kSplitThreads)
   } else {
     SplitRow<V, 1>(it, tr, row, 0, cl, a, tw, c == 0, &ss, &mx);
   }
-  // the row's largest magnitude and sum of |U|^2 in a fixed order: a shuffle
-  // tree, the warps in order, the blocks in order
+  if constexpr (sizeof(V) == sizeof(double2)) {
+    cl.sync();  // no block reads another's slice any more
+  } else {
+    // the row's largest magnitude and sum of |U|^2 in a fixed order: a shuffle
+    // tree, the warps in order, the blocks in order
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    warp_ss[threadIdx.x >> 5] = ss;
-    warp_mx[threadIdx.x >> 5] = mx;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < kSplitThreads / 32; ++w) {
-      ss += warp_ss[w];
-      mx = fmaxf(mx, warp_mx[w]);
+    for (int o = 16; o > 0; o >>= 1) {
+      ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     }
-    *cl.map_shared_rank(&part_ss[c], 0) = ss;
-    *cl.map_shared_rank(&part_mx[c], 0) = mx;
-  }
-  cl.sync();  // the shares are in block 0, and no block reads another's slice any more
-  if (c == 0 && threadIdx.x == 0 && it.row_max != nullptr) {
-    for (int i = 1; i < C; ++i) {
-      ss += part_ss[i];
-      mx = fmaxf(mx, part_mx[i]);
+    if ((threadIdx.x & 31) == 0) {
+      warp_ss[threadIdx.x >> 5] = ss;
+      warp_mx[threadIdx.x >> 5] = mx;
     }
-    it.row_max[tr * it.rows + row] = mx;
-    it.row_ms[tr * it.rows + row] = ss / float(it.bins);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < kSplitThreads / 32; ++w) {
+        ss += warp_ss[w];
+        mx = fmaxf(mx, warp_mx[w]);
+      }
+      *cl.map_shared_rank(&part_ss[c], 0) = ss;
+      *cl.map_shared_rank(&part_mx[c], 0) = mx;
+    }
+    cl.sync();  // the shares are in block 0, and no block reads another's slice any more
+    if (c == 0 && threadIdx.x == 0 && it.row_max != nullptr) {
+      for (int i = 1; i < C; ++i) {
+        ss += part_ss[i];
+        mx = fmaxf(mx, part_mx[i]);
+      }
+      it.row_max[tr * it.rows + row] = mx;
+      it.row_ms[tr * it.rows + row] = ss / float(it.bins);
+    }
   }
 }
 
