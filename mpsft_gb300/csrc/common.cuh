@@ -532,7 +532,10 @@ __device__ inline double WindowInFreq(const SigIter &it, double xi) {
 // slot s (k1 and its bin given) into mode_base (BinInFreqV1::Run,
 // src/binner.cc:565-591).
 __device__ inline void ModeTerms64(const SigIter &it, int s, int64_t k1, int bin) {
-  const double xi = (double(bin) + 0.5) / double(it.bins) - double(k1) / double(it.n);
+  // xi = (bin + 1/2)/B - k1/n from its exact numerator (|num| < 2^53): no FP64
+  // division, and no cancellation
+  const int64_t num = (2 * int64_t(bin) + 1) * it.n - 2 * int64_t(it.bins) * k1;
+  const double xi = double(num) * it.xi_scale;
   const double2 wc =
       it.unit_wf ? it.tab_coef[s] : cscale(it.tab_coef[s], WindowInFreq(it, xi));
   const int32_t key = it.tab_key[s];

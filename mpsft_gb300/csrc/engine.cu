@@ -901,20 +901,20 @@ struct Ahead {
 int LaunchForcedIteration(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
                           const Maxima &mx, bool x_c128, BinTimer *timer,
                           int64_t *launched, cudaStream_t s, bool tables) {
-  // side stream: mode preparation and bucketing (the decisions wait for them);
-  // low-priority stream: the Bluestein tables (the row transforms do)
+  // side stream (ahead of the binning's blocks): the Bluestein tables (the row
+  // transforms wait for them; behind the binning, on the lowest priority, they
+  // held the first transforms of 2000 modes up by 160 us), mode preparation and
+  // bucketing (the decisions do)
   MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_fork, s));
   MPSFT_CUDA(ctx, cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
+  if (!tables) {
+    LaunchBluesteinSetup(d_its, nsig, mx.m, true, ctx->tw32, ctx->tw64, ctx->side, true);
+  }
+  MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_blue, ctx->side));
   LaunchModePrep(d_its, nsig, mx.cap, ctx->side, true);
   LaunchBucket(d_its, nsig, mx.bins, mx.cap, ctx->side, false);
   MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_join, ctx->side));
-  MPSFT_CUDA(ctx, cudaStreamWaitEvent(ctx->side64, ctx->ev_fork, 0));
-  if (!tables) {
-    LaunchBluesteinSetup(d_its, nsig, mx.m, true, ctx->tw32, ctx->tw64, ctx->side64, true);
-  }
-  MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_blue, ctx->side64));
-  if (!tables) LaunchWindow64(d_its, nsig, mx.p2, s);
-  LaunchWindowMod(d_its, nsig, mx.bins, false, true, s);
+  LaunchWindowMod(d_its, nsig, mx.bins, tables ? kWindowRead : kWindowNew, true, s);
   if (timer) {
     // (tag 0: the iteration's FP32 binning, which has no signal)
     int rc = timer->Begin();
@@ -939,7 +939,7 @@ int LaunchForcedIteration(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join, 0));
   LaunchDecide(d_its, nsig, mx.bins, mx.trials, false, false, s, true);
   LaunchMerge(d_its, nsig, mx.bins, s);
-  if (launched) *launched += tables ? 7 : 9;
+  if (launched) *launched += tables ? 7 : 8;
   MPSFT_CUDA(ctx, cudaGetLastError());
   return MPSFT_OK;
 }
@@ -997,8 +997,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
     MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_join64, ctx->side64));
   }
   if (fp64) {
-    if (!tables) LaunchWindow(d_its, nsig, mx.p2, s);
-    LaunchWindowMod(d_its, nsig, mx.bins, false, false, s);
+    LaunchWindowMod(d_its, nsig, mx.bins, tables ? kWindowRead : kWindowNew, false, s);
   } else if (!ahead && !tables) {
     LaunchWindow32(d_its, nsig, mx.p2, s);
   }
@@ -1039,8 +1038,8 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   // Bluestein setup, mode preparation with bucketing, window(s), fold, FFT,
   // decide (ahead: the next iteration's plan and fold, bucketing, FP64
   // window, FFT, decide)
-  // FP64: the modulated window instead of the second window table
-  if (launched) *launched += ahead ? 6 : (tables ? (fp64 ? 5 : 4) : 7);
+  // FP64: the modulated window instead of the two window tables
+  if (launched) *launched += ahead ? 6 : (tables ? (fp64 ? 5 : 4) : (fp64 ? 6 : 7));
   if (!fp64) {
     // side stream: the listed bins' FP64 mode terms (before any merge
     // changes a coefficient), then the merge of the other bins, beside the
@@ -1061,7 +1060,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
     if (redo) {
       LaunchModePrep(d_its, nsig, mx.cap, s, true);
       LaunchBluesteinSetup(d_its, nsig, mx.m, true, ctx->tw32, ctx->tw64, s, true);
-      LaunchWindowMod(d_its, nsig, mx.bins, false, true, s);
+      LaunchWindowMod(d_its, nsig, mx.bins, kWindowRead, true, s);
       if (timer && ctx->profiling) LaunchDelay(20000, s);
       if (timer) {
         int rc = timer->Begin(1);
@@ -2534,7 +2533,8 @@ int BinInTimeImpl(mpsft_ctx *ctx, const mpsft_signal *sig, int32_t bins,
     if (direct) {
       if (!wt) LaunchWindow(d_it, 1, it.p2, st);
     } else if (fp64) {
-      LaunchWindowMod(d_it, 1, bins, !wt && new_window, false, st);
+      LaunchWindowMod(d_it, 1, bins, !wt && new_window ? kWindowNew : kWindowRead, false,
+                      st);
     } else if (!wt && new_window) {
       LaunchWindow32(d_it, 1, it.p2, st);
     }
@@ -2819,7 +2819,7 @@ int EstimateSetup(mpsft_ctx *ctx, int32_t n, const void *x,
   MPSFT_CUDA(ctx, cudaMemcpyAsync(d_in, in->bytes.data(), in->bytes.size(),
                                   cudaMemcpyHostToDevice, st));
   if (new_phases) LaunchPhaseTables(*d_it, 1, PhaseTableEntries(n), st);
-  LaunchWindowMod(*d_it, 1, su->bins, new_window, false, st);
+  LaunchWindowMod(*d_it, 1, su->bins, new_window ? kWindowNew : kWindowRead, false, st);
   if (new_blue) {
     LaunchBluesteinSetup(*d_it, 1, it->fft_m, true, ctx->tw32, ctx->tw64, st);
   }

@@ -45,7 +45,9 @@ __device__ inline ModeSetup SetupMode(const SigIter &it, int32_t k0, int lane) {
   ModeSetup m;
   m.k1 = mod(int64_t(it.a) * k0 + it.b);
   m.beta = int(mod.quot(m.k1 * B));
-  const double xi0 = double(m.k1) / double(n) - (double(m.beta) + 0.5) / double(B);
+  // k1/n - (beta + 1/2)/B from its exact numerator (|num| < 2^53)
+  const double xi0 =
+      double(2 * B * m.k1 - (2 * int64_t(m.beta) + 1) * n) * it.xi_scale;
   const double h = 0.5 * it.width;
   const double e = erf((xi0 + ((lane & 1) ? -h : h)) * it.erf_d);
   const double wf = 0.5 * (__shfl_sync(0xffffffffu, e, 0) - __shfl_sync(0xffffffffu, e, 1));

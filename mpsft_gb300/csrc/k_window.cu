@@ -104,8 +104,8 @@ __device__ double2 UnitRoot64(int64_t m, int64_t n) {
 // lanes per clock), so a block covers only 8 r's and one signal's bins spread
 // over every SM (501 bins, 18537 window points evaluated: 18 us with 32 r's in
 // 16 blocks, 12.5 us with 8); the last block has the row factors. eval: the
-// window itself is evaluated here (and stored in wt64 when present), else
-// read from wt64.
+// window itself is evaluated here (and stored in wt64 when present) unless
+// the signal's tables stand, else read from wt64.
 constexpr int kModCols = 8, kModThreads = 128;
 constexpr int kModFolds = kFoldLanes * kMaxFoldsPerLane / 2 + 1;  // f = t / B
 static_assert(kModCols + kModFolds <= kModThreads, "a thread per phase");
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kModThreads)
       const int t = r + f * B;
       if (t > it.p2) break;
       double w;
-      if (eval) {
+      if (eval && !it.tables_valid) {
         w = Window64At(it, t);
         if (it.wt64 != nullptr) it.wt64[t] = w;
       } else {
@@ -259,10 +259,11 @@ void LaunchWindow(const SigIter *d_its, int nsig, int max_p2, cudaStream_t s) {
   Launch(k_window64, grid, 256, 0, s, d_its, 1);
 }
 
-void LaunchWindowMod(const SigIter *d_its, int nsig, int max_bins, bool eval, bool cond,
-                     cudaStream_t s) {
+void LaunchWindowMod(const SigIter *d_its, int nsig, int max_bins, WindowSource window,
+                     bool cond, cudaStream_t s) {
   dim3 grid((max_bins + kModCols - 1) / kModCols + 1, nsig);
-  Launch(k_window_mod, grid, kModThreads, 0, s, d_its, eval ? 1 : 0, cond ? 1 : 0);
+  Launch(k_window_mod, grid, kModThreads, 0, s, d_its, window == kWindowNew ? 1 : 0,
+         cond ? 1 : 0);
 }
 
 void LaunchWindow64(const SigIter *d_its, int nsig, int max_p2, cudaStream_t s) {

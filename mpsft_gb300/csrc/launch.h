@@ -73,11 +73,12 @@ void LaunchWindow(const SigIter *d_its, int nsig, int max_p2, cudaStream_t s);
 void LaunchWindow32(const SigIter *d_its, int nsig, int max_p2, cudaStream_t s);
 void LaunchWindow64(const SigIter *d_its, int nsig, int max_p2, cudaStream_t s);
 
-// The modulated window and row factors of the FP64 binning (wmod, row_fac).
-// eval: the window evaluated in the same kernel (into wt64 too when it is not
-// null); otherwise read from wt64.
-void LaunchWindowMod(const SigIter *d_its, int nsig, int max_bins, bool eval, bool cond,
-                     cudaStream_t s);
+// The modulated window and row factors of the FP64 binning (wmod, row_fac), from
+// wt64 (kWindowRead), or with the window evaluated in the same kernel, into
+// wt64 too when it is not null (kWindowNew; signals with tables_valid have it).
+enum WindowSource { kWindowRead = 0, kWindowNew = 1 };
+void LaunchWindowMod(const SigIter *d_its, int nsig, int max_bins, WindowSource window,
+                     bool cond, cudaStream_t s);
 
 // Bluestein chirp and FFT(conjugate chirp) of every active signal.
 // fp64 selects double tables.

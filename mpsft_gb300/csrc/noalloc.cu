@@ -140,7 +140,7 @@ extern "C" int mpsft_bin_in_time_noalloc(const void *x_device, int64_t n,
   k_noalloc_setup<<<1, 1024, 0, st>>>(it, d_it, tw32, tw64,
                                       reinterpret_cast<uint32_t *>(base + kOffReady));
   if (fp64) {
-    LaunchWindowMod(d_it, 1, bins, true, false, st);
+    LaunchWindowMod(d_it, 1, bins, kWindowNew, false, st);
   } else {
     LaunchWindow32(d_it, 1, it.p2, st);
   }
