@@ -1356,10 +1356,7 @@ int GraphLoop(mpsft_ctx *ctx, const mpsft_signal *const *sigs,
     cudaError_t ce = cudaSuccess;
     int64_t per_body = 1;
     // the captured kernels use programmatic dependent launch
-    struct PdlScope {
-      PdlScope() { g_launch_pdl = true; }
-      ~PdlScope() { g_launch_pdl = false; }
-    } pdl_scope;
+    const PdlScope pdl_scope;
     cudaGraphNode_t prev = nullptr;
     for (const Phase &ph : phases) {
       if (ph.pipelined) {
@@ -2504,6 +2501,7 @@ int BinInTimeImpl(mpsft_ctx *ctx, const mpsft_signal *sig, int32_t bins,
   const Transform tf{a, b, c, InverseMod(a, n)};
   FillIter(&it, sig, bins, bits, w, tf, &q, 1);
   cudaStream_t st = ctx->stream;
+  const PdlScope pdl_scope;
   // the row transform writes the caller's device buffer itself when it may:
   // this device's memory, aligned for whole bins (bins_cap = bins: the rows are
   // adjacent)
@@ -2682,6 +2680,7 @@ int BinInFreqImpl(mpsft_ctx *ctx, int32_t n, int32_t bins, int32_t bits,
   it.x = nullptr;
   it.unit_wf = wf ? 1 : 0;
   cudaStream_t st = ctx->stream;
+  const PdlScope pdl_scope;
   BeginTables(ctx);
   const bool new_phases = UsePhases(ctx, &it);
   in.Put(o_it, &it, sizeof(it));
@@ -2850,6 +2849,7 @@ int mpsft_estimate(mpsft_ctx *ctx, const mpsft_signal *sig,
   SigIter it;
   SigIter *d_it = nullptr;
   Inputs in;
+  const PdlScope pdl_scope;
   const int32_t *d_k0 = nullptr;
   rc = EstimateSetup(ctx, int32_t(sig->n), sig->d_x, setup, k0, m, nullptr,
                      size_t(m) * sizeof(double2), &in, &cv, &it, &d_it, &d_k0, nullptr);
@@ -2880,6 +2880,7 @@ int mpsft_adjoint(mpsft_ctx *ctx, int32_t n, const mpsft_estimate_setup *setup,
   SigIter it;
   SigIter *d_it = nullptr;
   Inputs in;
+  const PdlScope pdl_scope;
   const int32_t *d_k0 = nullptr;
   const double2 *d_g = nullptr;
   int rc = EstimateSetup(ctx, n, nullptr, setup, k0, m, g,
@@ -3019,6 +3020,7 @@ int IterateImpl(mpsft_ctx *ctx, const mpsft_signal *sig,
   SetThresholdCopies(&it);
   it.win_thr = opt->window_threshold;
   cudaStream_t st = ctx->stream;
+  const PdlScope pdl_scope;
   BeginTables(ctx);
   const bool new_phases = UsePhases(ctx, &it);
   // the mode table is cleared and filled while the host waits for the energy

@@ -66,6 +66,7 @@ __device__ inline ModeSetup SetupMode(const SigIter &it, int32_t k0, int lane) {
 __global__ void __launch_bounds__(32) k_estimate(const SigIter *__restrict__ its,
                                                  const int32_t *k0s, int64_t m,
                                                  double2 *coef) {
+  PdlEnter();
   const SigIter &it = *its;
   const int lane = threadIdx.x;
   for (int64_t i = blockIdx.x; i < m; i += gridDim.x) {
@@ -94,6 +95,7 @@ __global__ void __launch_bounds__(32) k_estimate(const SigIter *__restrict__ its
 __global__ void __launch_bounds__(32) k_adjoint_spread(const SigIter *__restrict__ its,
                                                        const int32_t *k0s,
                                                        const double2 *g, int64_t m) {
+  PdlEnter();
   const SigIter &it = *its;
   const int lane = threadIdx.x;
   double2 *G = reinterpret_cast<double2 *>(it.fold);
@@ -119,6 +121,7 @@ __global__ void __launch_bounds__(32) k_adjoint_spread(const SigIter *__restrict
 // 33 us at 401 bins and 25 rows, now 8 us.
 __global__ void __launch_bounds__(256) k_adjoint_scatter(const SigIter *__restrict__ its,
                                                          double2 *dx) {
+  PdlEnter();
   const SigIter &it = *its;
   const int tt = blockIdx.x * blockDim.x + threadIdx.x;
   const int r = blockIdx.y, t = blockIdx.z;
@@ -148,18 +151,18 @@ unsigned ModeBlocks(int64_t m) {
 void LaunchEstimate(const SigIter *d_it, const int32_t *k0, int64_t m,
                     double2 *coef, cudaStream_t s) {
   if (m <= 0) return;
-  k_estimate<<<ModeBlocks(m), 32, 0, s>>>(d_it, k0, m, coef);
+  Launch(k_estimate, ModeBlocks(m), 32, 0, s, d_it, k0, m, coef);
 }
 
 void LaunchAdjointSpread(const SigIter *d_it, const int32_t *k0, const double2 *g,
                          int64_t m, cudaStream_t s) {
-  if (m > 0) k_adjoint_spread<<<ModeBlocks(m), 32, 0, s>>>(d_it, k0, g, m);
+  if (m > 0) Launch(k_adjoint_spread, ModeBlocks(m), 32, 0, s, d_it, k0, g, m);
 }
 
 void LaunchAdjointScatter(const SigIter *d_it, int p, int rows, int trials, double2 *dx,
                           cudaStream_t s) {
   dim3 grid((p + 255) / 256, rows, trials);
-  k_adjoint_scatter<<<grid, 256, 0, s>>>(d_it, dx);
+  Launch(k_adjoint_scatter, grid, 256, 0, s, d_it, dx);
 }
 
 }  // namespace mpsft

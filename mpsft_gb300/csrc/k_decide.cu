@@ -525,6 +525,7 @@ __global__ void __launch_bounds__(1024) k_table_load(const SigIter *__restrict__
                                                      const int32_t *__restrict__ k0,
                                                      const double2 *__restrict__ coef,
                                                      int64_t m) {
+  PdlEnter();
   const SigIter &it = *its;
   for (int i = threadIdx.x; i < it.tab_cap; i += blockDim.x) {
     it.tab_key[i] = kEmptyKey;
@@ -568,6 +569,7 @@ __global__ void k_clear_tables(const SigIter *__restrict__ its) {
 __global__ void __launch_bounds__(1024)
     k_export_tables(const SigIter *__restrict__ its, int nsig, int32_t *keys,
                     double2 *coefs, int32_t *counts, int32_t *sorted) {
+  PdlEnter();
   extern __shared__ unsigned long long sk[];
   __shared__ long long s_base;
   const SigIter &it = its[blockIdx.x];
@@ -658,7 +660,7 @@ void LaunchExportTables(const SigIter *d_its, int nsig, int max_cap,
   const size_t sm = size_t(BucketKeys(max_cap)) * sizeof(unsigned long long);
   cudaFuncSetAttribute(k_export_tables, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        int(sm));
-  k_export_tables<<<nsig, 1024, sm, s>>>(d_its, nsig, keys, coefs, counts, sorted);
+  Launch(k_export_tables, nsig, 1024, sm, s, d_its, nsig, keys, coefs, counts, sorted);
 }
 
 void LaunchModePrep(const SigIter *d_its, int nsig, int max_cap, cudaStream_t s,
@@ -736,7 +738,7 @@ void LaunchInsertSpills(const SigIter *d_its, int nsig, cudaStream_t s) {
 
 void LaunchTableLoad(const SigIter *d_it, const int32_t *k0, const double2 *coef,
                      int64_t m, cudaStream_t s) {
-  k_table_load<<<1, 1024, 0, s>>>(d_it, k0, coef, m);
+  Launch(k_table_load, 1, 1024, 0, s, d_it, k0, coef, m);
 }
 
 void LaunchPencil(const double2 *u3, int64_t count, double *sigma,

@@ -7,11 +7,16 @@
 
 namespace mpsft {
 
-// True while the calling thread captures a solve graph: the iteration
-// kernels are then launched with programmatic stream serialization (each
-// starts with PdlEnter), so that a kernel's launch overlaps the end of the
-// kernel before it.
+// True while the calling thread captures a solve graph or launches a
+// single-signal call: the kernels are then launched with programmatic stream
+// serialization (each starts with PdlEnter), so that a kernel's launch overlaps
+// the end of the kernel before it.
 extern thread_local bool g_launch_pdl;
+struct PdlScope {
+  bool outer = g_launch_pdl;
+  PdlScope() { g_launch_pdl = true; }
+  ~PdlScope() { g_launch_pdl = outer; }
+};
 
 // A launch of clusters of `cluster` blocks along x (1: no clusters).
 template <typename... P, typename... A>
