@@ -415,6 +415,7 @@ struct ResultStage {
 // `est` entries (the last call's count and a quarter more), so that one wait
 // usually covers the results (FinishResults copies any rest).
 int LaunchResults(mpsft_ctx *ctx, const SigIter *d_its, const ResultStage &rs) {
+  const PdlScope pdl_scope;
   size_t *est = &rs.est;
   unsigned char *d = rs.dev;
   LaunchCopyMapped(ctx->d_solve_ctl, rs.at<SolveCtl>(d, rs.ctl),
@@ -499,6 +500,7 @@ int Upload(mpsft_ctx *ctx, void *dst, const void *src, size_t bytes,
   }
   std::memcpy(ctx->h_up + off, src, bytes);
   ctx->up_off = off + bytes;
+  const PdlScope pdl_scope;
   LaunchCopyMapped(ctx->d_up + off, dst, bytes, s);
   ++ctx->up_launches;
   MPSFT_CUDA(ctx, cudaGetLastError());
@@ -1672,10 +1674,13 @@ int SolveMany(mpsft_ctx *ctx, const mpsft_signal *const *sigs,
   // whole call)
   rc = Upload(ctx, d_its, its.data(), sizeof(SigIter) * nsig, ctx->stream);
   if (rc) return rc;
-  LaunchClearTables(d_its, nsig, max_cap, ctx->stream);
   bool any_phase = false;
   for (int i = 0; i < nsig; ++i) any_phase |= its[i].ph_build != 0;
-  if (any_phase) LaunchPhaseTables(d_its, nsig, phase_entries, ctx->stream);
+  {
+    const PdlScope pdl_scope;
+    LaunchClearTables(d_its, nsig, max_cap, ctx->stream);
+    if (any_phase) LaunchPhaseTables(d_its, nsig, phase_entries, ctx->stream);
+  }
   MPSFT_CUDA(ctx, cudaGetLastError());
   ctx->ph_cache_n = sigs[0]->n;  // the shared tables are built (or were)
   bool host_loop = ctx->profiling || ctx->graph_unavailable;

@@ -549,6 +549,7 @@ __global__ void k_pencil(const double2 *__restrict__ u3, int64_t count,
 
 // Empty tables and control words of every signal.
 __global__ void k_clear_tables(const SigIter *__restrict__ its) {
+  PdlEnter();
   const SigIter &it = its[blockIdx.y];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < it.tab_cap) {
@@ -651,7 +652,7 @@ void LaunchDecideP(const SigIter *d_its, int nsig, int max_bins, int max_trials,
 void LaunchClearTables(const SigIter *d_its, int nsig, int max_cap,
                        cudaStream_t s) {
   dim3 grid((std::max(max_cap, int(kCtlWords)) + 255) / 256, nsig);
-  k_clear_tables<<<grid, 256, 0, s>>>(d_its);
+  Launch(k_clear_tables, grid, 256, 0, s, d_its);
 }
 
 void LaunchExportTables(const SigIter *d_its, int nsig, int max_cap,

@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(kModThreads)
 // ph_lo[l] = e^{2 pi i l / n} for l < 2^ph_k and ph_hi[h] = e^{2 pi i h 2^ph_k / n}
 // for h <= (n - 1) >> ph_k, from exact integer phases.
 __global__ void k_phase_tables(const SigIter *__restrict__ its) {
+  PdlEnter();
   const SigIter &it = its[blockIdx.y];
   if (!it.ph_build) return;  // (tables shared with another signal, or cached)
   const int64_t n = it.n;
@@ -251,7 +252,7 @@ void LaunchTwiddles(float2 *tw32, double2 *tw64, cudaStream_t s) {
 void LaunchPhaseTables(const SigIter *d_its, int nsig, int64_t entries,
                        cudaStream_t s) {
   dim3 grid(unsigned((entries + 255) / 256), nsig);
-  k_phase_tables<<<grid, 256, 0, s>>>(d_its);
+  Launch(k_phase_tables, grid, 256, 0, s, d_its);
 }
 
 void LaunchWindow(const SigIter *d_its, int nsig, int max_p2, cudaStream_t s) {
@@ -311,6 +312,7 @@ template <typename TX>
 __global__ void __launch_bounds__(256)
     k_energy_sample(const void *const *__restrict__ xs, const int64_t *__restrict__ ns,
                     double *__restrict__ energy, int per_block) {
+  PdlEnter();
   __shared__ double red[256];
   const int sig = blockIdx.y;
   const TX *x = reinterpret_cast<const TX *>(xs[sig]);
@@ -356,9 +358,9 @@ void LaunchEnergy(const void *const *x, const int64_t *n, int nsig, bool c128,
                   double *energy, cudaStream_t s, int per_block) {
   const dim3 grid(kEnergyParts, nsig);
   if (c128) {
-    k_energy_sample<double2><<<grid, 256, 0, s>>>(x, n, energy, per_block);
+    Launch(k_energy_sample<double2>, grid, 256, 0, s, x, n, energy, per_block);
   } else {
-    k_energy_sample<float2><<<grid, 256, 0, s>>>(x, n, energy, per_block);
+    Launch(k_energy_sample<float2>, grid, 256, 0, s, x, n, energy, per_block);
   }
 }
 
