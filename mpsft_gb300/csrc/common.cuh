@@ -322,20 +322,26 @@ __host__ __device__ inline void SetBinsFixedPoint(SigIter *it) {
 
 // phi_b = round(2^64 (b mod n) / n) (n and b set); for n = 2^k it is exactly
 // (b mod n) 2^(64 - k), without the 128-bit division.
-__host__ __device__ inline void SetPhiB(SigIter *it) {
-  const uint64_t n = uint64_t(it->n);
-  const uint64_t bm = uint64_t(PosMod(it->b, int64_t(n)));
+// round(2^64 (b mod n) / n). A length that is no power of two takes two 64-bit
+// divisions by a 31-bit number (a 128-bit one is a call of several hundred
+// instructions, on the one thread that plans a signal).
+__host__ __device__ inline uint64_t PhiOf(int32_t b, int32_t n32) {
+  int32_t r32 = b % n32;
+  if (r32 < 0) r32 += n32;
+  const uint64_t n = uint64_t(n32), bm = uint64_t(r32);
   if ((n & (n - 1)) == 0) {
 #ifdef __CUDA_ARCH__
     const int k = 63 - __clzll(static_cast<long long>(n));
 #else
     const int k = __builtin_ctzll(n);
 #endif
-    it->phi_b = bm << (64 - k);
-  } else {
-    it->phi_b = uint64_t((((unsigned __int128)bm << 64) + n / 2) / n);
+    return k == 0 ? 0 : bm << (64 - k);
   }
+  const uint64_t hi = (bm << 32) / n;
+  const uint64_t rem = (bm << 32) - hi * n;
+  return (hi << 32) + ((rem << 32) + n / 2) / n;
 }
+__host__ __device__ inline void SetPhiB(SigIter *it) { it->phi_b = PhiOf(it->b, it->n); }
 
 // The fixed-point constants of an iteration (n, b, bins and erf_d set).
 __host__ __device__ inline void SetFixedPoint(SigIter *it) {

@@ -42,11 +42,9 @@ __device__ int32_t NumBitsDev(int32_t n, int32_t bins) {
   return out;
 }
 
-__device__ inline int32_t NextBins(const SolveCtl &c, const SigIter &it) {
-  const int32_t found = *it.tab_count;
-  int32_t bins = (c.k - found) * 2 + 1;
-  if (bins < c.min_bins) bins = c.min_bins;
-  return bins;
+__device__ inline int32_t NextBins(const SolveCtl &c, int32_t found) {
+  const int32_t bins = (c.k - found) * 2 + 1;
+  return bins < c.min_bins ? c.min_bins : bins;
 }
 
 // One warp per signal. A new number of bins takes eight FP64 divisions and a
@@ -54,7 +52,13 @@ __device__ inline int32_t NextBins(const SolveCtl &c, const SigIter &it) {
 // number of lanes): the divisions run in three stages, the independent ones of a
 // stage on different lanes, without 128-bit divisions (one thread after the
 // other: one recovery of 1000 modes 1.008x, 24 uneven ones 1.005x slower).
-// Lane 0 stores.
+// What is read through the descriptors (the number of modes, the draws, the
+// table cache's entries) is read by all lanes at once before anything is stored,
+// a draw per lane, so that the kernel waits for memory three times and not for
+// every trial again. Lane 0 stores the rest. (With k_finish, which does the same:
+// 6 us less of every iteration of 24 signals, 2 to 3 us of one signal's; a solve
+// of one signal 1117 -> 1081 us, of 24 signals 5611 -> 5494 us, of 24 uneven ones
+// 23.9 -> 23.4 ms.)
 //
 // max_bins: signals needing more bins wait (the launch shapes of this body
 // do not cover them). ahead = 1 plans iteration iter + 1 of a signal in the
@@ -65,18 +69,28 @@ __global__ void k_plan(SolveCtl *__restrict__ ctl, SigIter *__restrict__ its,
   PdlEnter(its, kTracePlan);
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= nsig) return;
-  SolveCtl &c = ctl[i];
+  const SolveCtl c = ctl[i];
   SigIter &it = its[i];
   const int local = c.iter + ahead - c.draw_base;
   if (c.done || local >= c.draws_avail) {
     if (lane == 0) it.active = 0;
     return;
   }
-  const int32_t bins = ahead ? c.min_bins : NextBins(c, it);
+  // a, b, c, a_inv, q_0 .. (lanes 0 .. 3 + trials) and re, im of every trial's
+  // row phase (lanes 0 .. 2 trials - 1)
+  const int32_t dv = lane < 4 + c.trials
+                         ? c.draws[size_t(local) * c.draw_stride + lane] : 0;
+  const double bv = lane < 2 * c.trials
+                        ? c.draw_bq[size_t(local) * (c.draw_stride - 4) * 2 + lane] : 0.0;
+  const int32_t bins = ahead ? c.min_bins : NextBins(c, *it.tab_count);
   if (bins > max_bins) {
     if (lane == 0) it.active = 0;
     return;
   }
+  const bool cached = c.win_base != nullptr && !c.force_fp64;
+  const int h = bins >> 1;
+  const int64_t win_base = cached ? c.win_base[h] : 0;
+  const int32_t win_valid = cached ? c.win_valid[h] : 0;
   // Everything that depends on the bins only (and on the signal's constants)
   // stays from the previous iteration when the bins repeat (most late
   // iterations).
@@ -108,6 +122,14 @@ __global__ void k_plan(SolveCtl *__restrict__ ctl, SigIter *__restrict__ its,
     double unused;
     div3(tmp, B, erf_d, __dmul_rn(__dmul_rn(4.0, n), B), 0.0, 1.0, &folds, &wf_scale,
          &unused);
+  }
+  const int32_t b = __shfl_sync(0xffffffffu, dv, 1);
+  const uint64_t phi_b = PhiOf(b, it.n);
+  const int32_t cc = __shfl_sync(0xffffffffu, dv, 2);
+  const int32_t a_inv = __shfl_sync(0xffffffffu, dv, 3);
+  if (lane >= 4 && lane < 4 + c.trials) it.q[lane - 4] = dv;
+  if (lane < 2 * c.trials) {
+    (lane & 1 ? it.bq_im : it.bq_re)[lane >> 1] = bv;
   }
   if (lane != 0) return;
   if (ahead && it.fold_alt != nullptr) {
@@ -152,35 +174,27 @@ __global__ void k_plan(SolveCtl *__restrict__ ctl, SigIter *__restrict__ its,
       it.eps_ms = 0.f;
     }
   }
-  const int32_t *d = c.draws + size_t(local) * c.draw_stride;
-  const double *bq = c.draw_bq + size_t(local) * (c.draw_stride - 4) * 2;
-  it.a = d[0];
-  it.b = d[1];
-  it.c = d[2];
-  it.a_inv = d[3];
+  it.a = dv;
+  it.b = b;
+  it.c = cc;
+  it.a_inv = a_inv;
   it.trials = c.trials;
-  SetPhiB(&it);
-  for (int t = 0; t < c.trials; ++t) {
-    it.q[t] = d[4 + t];
-    it.bq_re[t] = bq[2 * t];
-    it.bq_im[t] = bq[2 * t + 1];
-  }
+  it.phi_b = phi_b;
   it.win_thr = c.win_thr;
   it.force_fp64 = c.force_fp64;
   it.win_slot = -1;
-  if (c.win_base != nullptr && !c.force_fp64) {
+  if (cached) {
     // tables from the context's cache: built already, or built now by the
     // one signal of the batch that claims the block
-    const int h = bins >> 1;
     const WinBlock wb = WinBlockOf(it.p2, bins, it.fft_m);
-    unsigned char *blk = c.win_pool + c.win_base[h];
+    unsigned char *blk = c.win_pool + win_base;
     it.wt32 = reinterpret_cast<float *>(blk);
     it.wt64 = reinterpret_cast<double *>(blk + wb.wt64);
     it.wtff = reinterpret_cast<float2 *>(blk + wb.wtff);
     it.chirp32 = reinterpret_cast<float2 *>(blk + wb.chirp32);
     it.chat32 = reinterpret_cast<float2 *>(blk + wb.chat32);
     it.r2b64 = reinterpret_cast<double2 *>(blk + wb.r2b64);
-    const bool build = c.win_valid[h] == 0 && atomicCAS(&c.win_claim[h], 0, 1) == 0;
+    const bool build = win_valid == 0 && atomicCAS(&c.win_claim[h], 0, 1) == 0;
     it.tables_valid = build ? 0 : 1;
     if (build) it.win_slot = h;
   } else {
@@ -207,45 +221,65 @@ __global__ void __launch_bounds__(1024)
   PdlEnter(its, kTraceFinish);
   int any = 0;
   for (int i = threadIdx.x; i < nsig; i += blockDim.x) {
-    SolveCtl &c = ctl[i];
-    SigIter &it = its[i];
-    if (it.active) {
+    // everything read before anything is stored: two waits for memory, not one
+    // at every counter
+    const SolveCtl c = ctl[i];
+    const SigIter &it = its[i];
+    int32_t *const fl = it.flags;
+    int32_t found = *it.tab_count;
+    const int32_t progress = fl[0], near_ties = fl[2], spills = fl[4];
+    int32_t bits = fl[1], max_found = fl[3];
+    const int32_t active = it.active, bins = it.bins, win_slot = it.win_slot;
+    const bool forced = it.force_fp64 != 0, f64 = c.fp64_path || forced;
+    const int64_t gathers = BinGathers(it, f64), bytes = BinBytesOf(it, f64);
+    const int64_t tab_cap = it.tab_cap;
+    int32_t iter = c.iter, done = c.done;
+    if (active) {
       // this iteration's spilled candidates, after all others (InsertSpills)
-      if (it.flags[4] > 0) InsertSpills(it);
-      const int32_t *fl = it.flags;
-      c.iter += 1;
-      c.near_ties += fl[2];
-      if (fl[1] & kStatusUnresolved) c.unresolved += 1;
-      c.fp64_iters += it.force_fp64;
-      const bool f64 = c.fp64_path || it.force_fp64;
-      c.gathers += BinGathers(it, f64);
-      c.bin_bytes += BinBytesOf(it, f64);
-      if (fl[1] & kStatusCapacity) {
-        c.status = kSolveCapacity;
-      } else if (fl[1] & kStatusNonFinite) {
-        c.status = kSolveNonFinite;
-      } else if (int64_t(fl[3]) * 2 > it.tab_cap) {
-        c.status = kSolveCapacity;
+      if (spills > 0) {
+        InsertSpills(it);
+        found = *it.tab_count;
+        bits = fl[1];
+        max_found = fl[3];
       }
-      if (!fl[0]) c.stale += 1;
-      if (c.status == 0 && c.stale < c.max_stale && c.iter >= c.max_iter) {
-        c.status = kSolveIterCap;
+      SolveCtl &o = ctl[i];
+      iter += 1;
+      int32_t stale = c.stale, status = c.status;
+      if (bits & kStatusCapacity) {
+        status = kSolveCapacity;
+      } else if (bits & kStatusNonFinite) {
+        status = kSolveNonFinite;
+      } else if (int64_t(max_found) * 2 > tab_cap) {
+        status = kSolveCapacity;
       }
-      if (c.status != 0 || c.stale >= c.max_stale) c.done = 1;
-      c.last_bins = it.bins;
+      if (!progress) stale += 1;
+      if (status == 0 && stale < c.max_stale && iter >= c.max_iter) {
+        status = kSolveIterCap;
+      }
+      if (status != 0 || stale >= c.max_stale) done = 1;
+      o.iter = iter;
+      o.near_ties = c.near_ties + near_ties;
+      if (bits & kStatusUnresolved) o.unresolved = c.unresolved + 1;
+      o.fp64_iters = c.fp64_iters + forced;
+      o.gathers = c.gathers + gathers;
+      o.bin_bytes = c.bin_bytes + bytes;
+      o.stale = stale;
+      o.status = status;
+      o.done = done;
+      o.last_bins = bins;
       // the tables this signal built are complete (every table kernel of
       // the iteration has run)
-      if (it.win_slot >= 0) c.win_valid[it.win_slot] = 1;
-      it.active = 0;
+      if (win_slot >= 0) c.win_valid[win_slot] = 1;
+      its[i].active = 0;
     }
     if (its_ahead != nullptr) {
-      if (c.done) its_ahead[i].active = 0;
-      it.flags[0] = 0;
-      it.flags[1] = 0;
-      it.flags[2] = 0;
+      if (done) its_ahead[i].active = 0;
+      fl[0] = 0;
+      fl[1] = 0;
+      fl[2] = 0;
     }
-    if (!c.done && c.iter - c.draw_base < c.draws_avail) {
-      const int32_t nb = NextBins(c, it);
+    if (!done && iter - c.draw_base < c.draws_avail) {
+      const int32_t nb = NextBins(c, found);
       if (nb > cond_lo && nb <= cond_hi && !(exclude_fixed && nb <= c.min_bins)) {
         any = 1;
       }
