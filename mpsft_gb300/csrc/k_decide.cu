@@ -207,8 +207,7 @@ __global__ void __launch_bounds__(1024) k_bucket(const SigIter *__restrict__ its
 template <typename T, int TMAX>
 __global__ void __launch_bounds__(256, (sizeof(T) == 4 && TMAX == 1) ? 6 : 1)
     k_decide(const SigIter *__restrict__ its, int mode, int cond, int mark) {
-  PdlEnter(its, kTraceDecide);
-  const SigIter &it = its[blockIdx.y];
+  const SigIter &it = PdlEnterLoaded(its, blockIdx.y, kTraceDecide);
   if (!it.active) return;
   if (cond ? !RedoFP64(it) : it.force_fp64) return;
   const int beta = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -255,11 +254,10 @@ __device__ void MergeBin(const SigIter &it, int beta, bool go);
 // marked unresolved (k_decide_listed).
 template <int TMAX, int W, int G>
 __global__ void __launch_bounds__(32 * W) k_listed_terms(const SigIter *__restrict__ its) {
-  PdlEnter(its, kTraceListedTerms);
+  const SigIter &it = PdlEnterLoaded(its, blockIdx.y, kTraceListedTerms);
   __shared__ double2 s_p0[W][TMAX];
   __shared__ double2 s_pp[W][32][TMAX];
   __shared__ double2 s_pm[W][32][TMAX];
-  const SigIter &it = its[blockIdx.y];
   if (!it.active || it.force_fp64 || it.esc_mask == nullptr) return;
   const int nf = *(volatile int32_t *)&it.flags[2];
   if (nf > it.esc_cap) return;
@@ -366,8 +364,7 @@ __global__ void __launch_bounds__(32 * W) k_listed_terms(const SigIter *__restri
 template <int TMAX>
 __global__ void __launch_bounds__(256)
     k_decide_listed(const SigIter *__restrict__ its, int redo, int merge) {
-  PdlEnter(its, kTraceDecideListed);
-  const SigIter &it = its[blockIdx.y];
+  const SigIter &it = PdlEnterLoaded(its, blockIdx.y, kTraceDecideListed);
   if (!it.active) return;
   if (it.force_fp64) return;
   const int nf = *(volatile int32_t *)&it.flags[2];
@@ -511,8 +508,7 @@ __global__ void k_insert_spills(const SigIter *__restrict__ its, int nsig) {
 // Candidates -> table, two lanes per bin; bins held back for their FP64
 // near-tie decision (cand_valid >= kCandListed) are merged by that decision.
 __global__ void __launch_bounds__(32) k_merge(const SigIter *__restrict__ its) {
-  PdlEnter(its, kTraceMerge);
-  const SigIter &it = its[blockIdx.y];
+  const SigIter &it = PdlEnterLoaded(its, blockIdx.y, kTraceMerge);
   if (!it.active) return;
   const int beta = blockIdx.x * 16 + (threadIdx.x >> 1);
   MergeBin(it, beta, beta < it.bins);

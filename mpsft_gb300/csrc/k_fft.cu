@@ -70,10 +70,9 @@ template <typename V>
 __global__ void __launch_bounds__(kRowFftThreads)
     k_row_fft(const SigIter *__restrict__ its, int max_trials,
               const V *__restrict__ tw, int cond, int rpb_cap) {
-  PdlEnter(its, kTraceRowFft);
+  const SigIter &it = PdlEnterLoaded(its, blockIdx.z, kTraceRowFft);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned row_max_bits[kRowsMax];
-  const SigIter &it = its[blockIdx.z];
   if (!it.active) return;
   if (cond ? !RedoFP64(it) : it.force_fp64) return;
   const int tr = blockIdx.y;
@@ -408,11 +407,10 @@ __device__ __forceinline__ void SplitRow(const SigIter &it, int tr, int row, int
 template <typename V, int C>
 __global__ void __launch_bounds__(kSplitThreads)
     k_row_fft_split(const SigIter *__restrict__ its, const V *__restrict__ tw, int cond) {
-  PdlEnter(its, kTraceRowFft);
+  const SigIter &it = PdlEnterLoaded(its, blockIdx.z, kTraceRowFft);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float part_ss[C], part_mx[C];  // block 0's: every block's share
   __shared__ float warp_ss[kSplitThreads / 32], warp_mx[kSplitThreads / 32];
-  const SigIter &it = its[blockIdx.z];
   const int row = blockIdx.x / C, tr = blockIdx.y;
   // (the same for every block of a cluster)
   if (!it.active || tr >= it.trials || row >= it.rows) return;
@@ -475,12 +473,11 @@ constexpr int kDirectRowsPerBlock = 4;  // two warps per row
 
 __global__ void __launch_bounds__(64 * kDirectRowsPerBlock)
     k_row_dft_small(const SigIter *__restrict__ its, int cond) {
-  PdlEnter(its, kTraceRowFft);
+  const SigIter &it = PdlEnterLoaded(its, blockIdx.z, kTraceRowFft);
   __shared__ float2 roots[kDirectMaxBins];
   __shared__ float2 rows[kDirectRowsPerBlock][kDirectMaxBins];
   __shared__ float wmax[2 * kDirectRowsPerBlock];
   __shared__ float wss[2 * kDirectRowsPerBlock];
-  const SigIter &it = its[blockIdx.z];
   if (!it.active) return;
   if (cond ? !RedoFP64(it) : it.force_fp64) return;
   const int tr = blockIdx.y;

@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(256) k_rebin_prep(const SigIter *__restrict__ 
 template <typename TX>
 __global__ void __launch_bounds__(256, 2)
     k_rebin_ff(const SigIter *__restrict__ its, int nsig) {
-  PdlEnter(its, kTraceRebin);
+  const SigIter &first = PdlEnterLoaded(its, 0, kTraceRebin);
   __shared__ int64_t items_end[kRebinMaxSignals];
   __shared__ float4 pw_s[8][kPowLen];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(256, 2)
       const int s = s0 + lane;
       int64_t items = 0;
       if (s < nsig) {
-        const SigIter &q = its[s];
+        const SigIter &q = s == 0 ? first : its[s];
         if (q.active && !q.force_fp64) {
           const int nf = *(volatile int32_t *)&q.flags[2];
           if (nf <= q.esc_cap) items = int64_t(nf) * q.trials * q.rows * RebinChunks(q.p);
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(256, 2)
     // (a signal's items: at most kMaxListed * kMaxTrials * rows * chunks,
     // far below 2^32, so the decode divides in 32 bits)
     uint32_t local = uint32_t(w - (sig > 0 ? items_end[sig - 1] : 0));
-    const SigIter &it = its[sig];
+    const SigIter &it = sig == 0 ? first : its[sig];
     const int nch = RebinChunks(it.p);
     const int c = int(local % uint32_t(nch));
     local /= uint32_t(nch);
