@@ -512,8 +512,9 @@ __device__ int DecideBin(const SigIter &it, int beta, const Src &src,
   int listed = -1;  // list position when this bin is listed as a near tie
 
   // ---- row 0 and its mode subtraction (the bin's modes are in increasing k0).
-  // The first 32 modes are loaded once, one per lane, and shared by shuffles
-  // (the common case); further modes are read directly.
+  // 32 modes at a time are loaded, one per lane, and shared by shuffles (read
+  // mode after mode, those past the first 32 took two dependent misses each, the
+  // longest warps of iterations with 20 modes per bin on average).
   V u0[TMAX];
 #pragma unroll
   for (int t = 0; t < TMAX; ++t) {
@@ -534,26 +535,30 @@ __device__ int DecideBin(const SigIter &it, int beta, const Src &src,
   V pre_base[TMAX];
   float mode_err = 0.f;  // FP32 error carried into this bin by the found modes
   int pre_k1 = 0;  // k1 of the lane's mode (row factors below)
-  if (lane < npre) {
-    const int sl = it.bkt_list[st + lane];
-    O::template terms<TMAX>(it, sl, pre_base);
-    pre_k1 = it.mode_k1[sl];
-    if (fp32) mode_err = it.mode_errw[sl];
-  }
+  // the lane's mode of those from i0 on
+  auto load_modes = [&](int i0, float *errw) {
+    if (i0 + lane < nm) {
+      const int sl = it.bkt_list[st + i0 + lane];
+      O::template terms<TMAX>(it, sl, pre_base);
+      pre_k1 = it.mode_k1[sl];
+      if (fp32 && errw) *errw = it.mode_errw[sl];
+    }
+  };
+  if (npre > 0) load_modes(0, &mode_err);
+  float errw = 0.f;
   for (int i = 0; i < (kSums ? 0 : nm); ++i) {
+    if (i > 0 && (i & 31) == 0) load_modes(i, &errw);
     V bs[TMAX];
-    if (i < 32) {
 #pragma unroll
-      for (int t = 0; t < TMAX; ++t) {
-        if (t < TR) {
-          bs[t].x = __shfl_sync(0xffffffffu, pre_base[t].x, i);
-          bs[t].y = __shfl_sync(0xffffffffu, pre_base[t].y, i);
-        }
+    for (int t = 0; t < TMAX; ++t) {
+      if (t < TR) {
+        bs[t].x = __shfl_sync(0xffffffffu, pre_base[t].x, i & 31);
+        bs[t].y = __shfl_sync(0xffffffffu, pre_base[t].y, i & 31);
       }
-    } else {
-      const int sl = it.bkt_list[st + i];
-      O::template terms<TMAX>(it, sl, bs);
-      if (fp32 && lane == 0) mode_err += it.mode_errw[sl];
+    }
+    if (i >= 32) {
+      const float e = __shfl_sync(0xffffffffu, errw, i & 31);
+      if (lane == 0) mode_err += e;
     }
 #pragma unroll
     for (int t = 0; t < TMAX; ++t) {
@@ -654,31 +659,27 @@ __device__ int DecideBin(const SigIter &it, int beta, const Src &src,
     }
   }
   for (int i0 = 0; i0 < (kSums ? 0 : nm); i0 += 4) {
+    if (nm > 32 && (i0 & 31) == 0) load_modes(i0, nullptr);
     V fac[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int i = i0 + u;
-      if (i < nm) {
-        const int64_t k1 = i < 32 ? __shfl_sync(0xffffffffu, pre_k1, i)
-                                  : it.mode_k1[it.bkt_list[st + i]];
-        if (has_bit) fac[u] = O::phase(it, off * k1);
-      }
+      // (on every lane and for every u: a branch around each keeps the four
+      // from running side by side)
+      const int64_t k1 =
+          __shfl_sync(0xffffffffu, pre_k1, min(i0 + u, nm - 1) & 31);
+      fac[u] = O::phase(it, off * k1);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int i = i0 + u;
       if (i < nm) {
         V bs[TMAX];
-        if (i < 32) {
 #pragma unroll
-          for (int t = 0; t < TMAX; ++t) {
-            if (t < TR) {
-              bs[t].x = __shfl_sync(0xffffffffu, pre_base[t].x, i);
-              bs[t].y = __shfl_sync(0xffffffffu, pre_base[t].y, i);
-            }
+        for (int t = 0; t < TMAX; ++t) {
+          if (t < TR) {
+            bs[t].x = __shfl_sync(0xffffffffu, pre_base[t].x, i & 31);
+            bs[t].y = __shfl_sync(0xffffffffu, pre_base[t].y, i & 31);
           }
-        } else {
-          O::template terms<TMAX>(it, it.bkt_list[st + i], bs);
         }
         if (has_bit) {
 #pragma unroll
