@@ -405,24 +405,26 @@ __device__ __forceinline__ void PdlEnter(const SigIter *its, int32_t id) {
 }
 
 // PdlEnter for the kernels in the middle of an iteration: signal sig's
-// descriptor is copied to shared memory while the kernel before still runs, and
-// read from there. Every block otherwise starts by walking from the descriptor
+// descriptor is copied to shared memory while the kernel before still runs (Early;
+// else after the wait, its lines at once), and read from there. Every block otherwise starts by walking from the descriptor
 // through its pointers to the data, some 900 cycles a step, and its eight lines
 // came one after the other. The descriptor does not change between the plan (or
 // the upload) and the end of the iteration; a kernel launched early starts when
 // the one before has passed its own wait, so what the kernels before that one
 // wrote is complete. The kernel right behind a writer of descriptors must not
-// use it. Called by the whole block. (A load before the wait without the copy
+// copy early. Called by the whole block. (A load before the wait without the copy
 // gained nothing: the wait drops the L1 lines.) One recovery of 1000 modes 906 ->
 // 843 us, 64 signals 5532 -> 5455 us, an FP64 iteration at 101 bins 109 -> 106 us.
+template <bool Early = true>
 __device__ __forceinline__ const SigIter &PdlEnterLoaded(const SigIter *__restrict__ its,
                                                          unsigned sig, int32_t id) {
+  if (!Early) PdlEnter();
   constexpr unsigned kWords = sizeof(SigIter) / sizeof(unsigned long long);
   static_assert(sizeof(SigIter) % sizeof(unsigned long long) == 0, "whole words");
   __shared__ unsigned long long words[kWords];
   const unsigned long long *src = reinterpret_cast<const unsigned long long *>(its + sig);
   for (unsigned i = threadIdx.x; i < kWords; i += blockDim.x) words[i] = __ldcg(src + i);
-  PdlEnter();
+  if (Early) PdlEnter();
   __syncthreads();
   const SigIter &it = *reinterpret_cast<const SigIter *>(words);
   if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {

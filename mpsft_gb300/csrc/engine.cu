@@ -914,7 +914,7 @@ int LaunchForcedIteration(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   }
   MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_blue, ctx->side));
   LaunchModePrep(d_its, nsig, mx.cap, ctx->side, true);
-  LaunchBucket(d_its, nsig, mx.bins, mx.cap, ctx->side, false);
+  LaunchBucket(d_its, nsig, mx.bins, mx.cap, ctx->side, kBucketOnly);
   MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_join, ctx->side));
   LaunchWindowMod(d_its, nsig, mx.bins, tables ? kWindowRead : kWindowNew, true, s);
   if (timer) {
@@ -987,13 +987,21 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
     LaunchBluesteinSetup(d_its, nsig, mx.m, fp64, ctx->tw32, ctx->tw64, ctx->side);
     MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_blue, ctx->side));
   }
-  // mode preparation and bucketing in one kernel
-  LaunchBucket(d_its, nsig, mx.bins, mx.cap, ctx->side, true);
+  // mode preparation and bucketing in one kernel; ahead, where no fold stands
+  // before the decisions, the modes' terms beside it (with them the bucketing
+  // takes 10 us, the row transforms 4)
+  if (ahead) {
+    MPSFT_CUDA(ctx, cudaStreamWaitEvent(ctx->side64, ctx->ev_fork, 0));
+    LaunchModeTerms32(d_its, nsig, mx.cap, ctx->side64);
+    MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_blue, ctx->side64));
+  }
+  LaunchBucket(d_its, nsig, mx.bins, mx.cap, ctx->side,
+               ahead ? kBucketBins : kBucketTerms);
   MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_join, ctx->side));
   // FP32 path: the FP64 window tables (for the near-tie re-binning and the
   // FP64 kernels) are built on the low-priority stream and joined only
   // before the re-binning; the binning uses an FP32 evaluation
-  if (!fp64 && !tables) {
+  if (!fp64 && !tables && !ahead) {
     MPSFT_CUDA(ctx, cudaStreamWaitEvent(ctx->side64, ctx->ev_fork, 0));
     LaunchWindow64(d_its, nsig, mx.p2, ctx->side64);
     MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_join64, ctx->side64));
@@ -1008,7 +1016,9 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
     // first), and its launch enqueued while a short delay kernel holds the
     // stream, so that its events time the kernel, not a host launch gap
     MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join, 0));
-    if (!fp64 && !tables) MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join64, 0));
+    if (!fp64 && !tables) {
+      MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join64, 0));
+    }
     LaunchDelay(20000, s);
   }
   if (timer) {
@@ -1029,6 +1039,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   LaunchRowFFT(d_its, nsig, mx.rows, mx.trials, mx.m, fp64, ctx->tw32, ctx->tw64,
                s, false, single);
   MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join, 0));  // join
+  if (ahead) MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_blue, 0));  // the terms
   // near ties of the FP32 pass: listed bins re-binned and re-decided in
   // FP64; signals that the precision policy sends to FP64 (and signals whose
   // near-tie list overflowed) run the FP64 kernels (redo). Without redo the
@@ -1054,7 +1065,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
       LaunchMerge(d_its, nsig, mx.bins, ctx->side);
       MPSFT_CUDA(ctx, cudaEventRecord(ctx->ev_join_m, ctx->side));
     }
-    if (!tables) MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join64, 0));
+    if (!tables && !ahead) MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join64, 0));
     LaunchRebin(d_its, nsig, kMaxListed, x_c128, false, s);
     MPSFT_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join_l, 0));
     LaunchDecideListed(d_its, nsig, mx.trials, redo, side_merge, s);
@@ -1362,22 +1373,28 @@ int GraphLoop(mpsft_ctx *ctx, const mpsft_signal *const *sigs,
     cudaGraphNode_t prev = nullptr;
     for (const Phase &ph : phases) {
       if (ph.pipelined) {
-        // prologue: plan, fold and Bluestein tables of the phase's first
-        // iteration
+        // prologue: plan, fold and tables of the phase's first iteration (the
+        // FP64 window beside the fold)
         cudaGraph_t pg = nullptr;
         MPSFT_CUDA(ctx, cudaGraphCreate(&pg, 0));
         ce = cudaStreamBeginCaptureToGraph(ctx->cap, pg, nullptr, nullptr, 0,
                                            cudaStreamCaptureModeThreadLocal);
         if (ce == cudaSuccess) {
           LaunchPlan(ctx->d_solve_ctl, d_its, nsig, ph.plan_max, ctx->cap);
+          ce = cudaEventRecord(ctx->ev_fork, ctx->cap);
+          if (ce == cudaSuccess) ce = cudaStreamWaitEvent(ctx->side64, ctx->ev_fork, 0);
+          LaunchWindow64(d_its, nsig, ph.shape.p2, ctx->side64);
+          if (ce == cudaSuccess) ce = cudaEventRecord(ctx->ev_join64, ctx->side64);
           LaunchWindow32(d_its, nsig, ph.shape.p2, ctx->cap);
           LaunchBinFold(d_its, nsig, ph.shape.bins, ph.shape.bits, ph.shape.trials,
                         x_c128, false, ctx->cap, false,
                         FoldShapeFor(ctx, ph.shape.bins, ph.shape.n, nsig, x_c128));
           LaunchBluesteinSetup(d_its, nsig, ph.shape.m, false, ctx->tw32, ctx->tw64,
                                ctx->cap);
+          if (ce == cudaSuccess) ce = cudaStreamWaitEvent(ctx->cap, ctx->ev_join64, 0);
           cudaGraph_t captured = nullptr;
-          ce = cudaStreamEndCapture(ctx->cap, &captured);
+          const cudaError_t ee = cudaStreamEndCapture(ctx->cap, &captured);
+          if (ce == cudaSuccess) ce = ee;
         }
         cudaGraphNode_t child = nullptr;
         if (ce == cudaSuccess) {
@@ -2707,7 +2724,7 @@ int BinInFreqImpl(mpsft_ctx *ctx, int32_t n, int32_t bins, int32_t bits,
   // (bins_cap = bins: the rows are adjacent)
   const size_t u_bytes = sizeof(double2) * size_t(bins) * it.rows;
   MPSFT_CUDA(ctx, cudaMemcpyAsync(it.ubuf, inout, u_bytes, cudaMemcpyHostToDevice, st));
-  LaunchBucket(d_it, 1, bins, s.tab_cap, st, true);
+  LaunchBucket(d_it, 1, bins, s.tab_cap, st, kBucketTerms);
   LaunchDecide(d_it, 1, bins, 1, false, true, st);
   MPSFT_CUDA(ctx, cudaGetLastError());
   // (the table has two slots per mode at least: it cannot fill up)

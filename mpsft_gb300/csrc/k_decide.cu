@@ -32,14 +32,14 @@ namespace mpsft {
 namespace {
 
 // ---------------------------------------------------------------- prep
-// Per occupied slot (the table's insertion list): k1 = (a k0 + b)
-// mod n and the mode's bin for the bucketing, and the row-0 term
+// Per occupied slot (the table's insertion list): k1 = (a k0 + b) mod n and the
+// mode's bin for the bucketing, and the row-0 term
 // wf c e^{2 pi i (q_t k1 + c k0)/n} of every trial (BinInFreqV1::Run,
-// src/binner.cc:565-591) in FP64 (unit phases from the FP64 tables). The
-// FP32 path also gets FP32 terms, computed in FP32, together with the error
-// the mode carries into its bin: the coefficient's bound tab_err |wf| plus
-// 8 eps_rel |wf c| for the FP32 window response, phase, rounding and
-// subtraction (each a few 2^-24 relative).
+// src/binner.cc:565-591) in FP64 (ModeTerms64; unit phases from the FP64
+// tables), or on the FP32 path in FP32, together with the error the mode carries
+// into its bin: the coefficient's bound tab_err |wf| plus 8 eps_rel |wf c| for the
+// FP32 window response, phase, rounding and subtraction (each a few 2^-24
+// relative).
 __device__ inline float WindowInFreq32(const SigIter &it, int64_t k1, int bin) {
   // xi +- 1/(4B) with xi = (bin + 1/2)/B - k1/n, as exact integers over 4nB
   const int64_t n = it.n, B4 = 4 * int64_t(it.bins);
@@ -48,32 +48,32 @@ __device__ inline float WindowInFreq32(const SigIter &it, int64_t k1, int bin) {
   return 0.5f * (erff(float(np) * it.wf_scale) - erff(float(nm) * it.wf_scale));
 }
 
-// One occupied slot s of k_mode_prep.
-__device__ void ModePrepSlot(const SigIter &it, int s, int cond) {
-  const int32_t key = it.tab_key[s];
-  const int64_t n = it.n;
-  const int B = it.bins;
-  const ModN mod{uint32_t(n), it.n_inv};
+__device__ inline int64_t ModeK1(const SigIter &it, int32_t key, int *bin) {
+  const ModN mod{uint32_t(it.n), it.n_inv};
   const int64_t k1 = mod(int64_t(it.a) * key + it.b);
-  const int bin = int(mod.quot(k1 * B));
-  it.mode_k1[s] = int32_t(k1);
-  it.mode_bin[s] = bin;
-  const bool fp32 = it.eps_rel > 0.f && !it.force_fp64 && !cond;
-  if (fp32) {
-    const float wf = WindowInFreq32(it, k1, bin);
-    const double2 cd = it.tab_coef[s];
-    const float2 wc = make_float2(float(cd.x) * wf, float(cd.y) * wf);
-    for (int t = 0; t < it.trials; ++t) {
-      const int64_t ph = int64_t(it.q[t]) * k1 + int64_t(it.c) * key;
-      it.mode_base32[size_t(s) * it.trials + t] = cmulf(wc, Phase32(it, ph));
-    }
-    it.mode_errw[s] = float(it.tab_err[s]) * fabsf(wf) +
-                      8.f * it.eps_rel * sqrtf(wc.x * wc.x + wc.y * wc.y);
-  } else {
-    ModeTerms64(it, s, k1, bin);
-  }
+  *bin = int(mod.quot(k1 * it.bins));
+  return k1;
 }
 
+__device__ inline void ModeTerms32(const SigIter &it, int s, int32_t key, int64_t k1,
+                                   int bin) {
+  const double2 cd = it.tab_coef[s];
+  const double err = it.tab_err[s];
+  const float wf = WindowInFreq32(it, k1, bin);
+  const float2 wc = make_float2(float(cd.x) * wf, float(cd.y) * wf);
+  for (int t = 0; t < it.trials; ++t) {
+    const int64_t ph = int64_t(it.q[t]) * k1 + int64_t(it.c) * key;
+    it.mode_base32[size_t(s) * it.trials + t] = cmulf(wc, Phase32(it, ph));
+  }
+  it.mode_errw[s] = float(err) * fabsf(wf) +
+                    8.f * it.eps_rel * sqrtf(wc.x * wc.x + wc.y * wc.y);
+}
+
+__device__ inline bool TermsIn32(const SigIter &it) {
+  return it.eps_rel > 0.f && !it.force_fp64;
+}
+
+// FP64 terms with k1 and bin (the bucketing after it sorts by them).
 __global__ void k_mode_prep(const SigIter *__restrict__ its, int cond) {
   PdlEnter(its, kTraceModePrep);
   const SigIter &it = its[blockIdx.y];
@@ -85,7 +85,27 @@ __global__ void k_mode_prep(const SigIter *__restrict__ its, int cond) {
   const int count = *it.tab_count;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count;
        i += gridDim.x * blockDim.x) {
-    ModePrepSlot(it, it.occ_list[i], cond);
+    const int s = it.occ_list[i];
+    int bin;
+    const int64_t k1 = ModeK1(it, it.tab_key[s], &bin);
+    it.mode_k1[s] = int32_t(k1);
+    it.mode_bin[s] = bin;
+    ModeTerms64(it, s, k1, bin);
+  }
+}
+
+// FP32 terms alone, beside the bucketing (kBucketBins), which evaluates k1 and
+// the bins itself.
+__global__ void __launch_bounds__(64) k_mode_terms32(const SigIter *__restrict__ its) {
+  const SigIter &it = PdlEnterLoaded<false>(its, blockIdx.y, kTraceModePrep);
+  if (!it.active || !TermsIn32(it)) return;
+  const int count = *it.tab_count;
+  for (int i = blockIdx.x * 64 + threadIdx.x; i < count; i += gridDim.x * 64) {
+    const int s = it.occ_list[i];
+    const int32_t key = it.tab_key[s];
+    int bin;
+    const int64_t k1 = ModeK1(it, key, &bin);
+    ModeTerms32(it, s, key, k1, bin);
   }
 }
 
@@ -112,46 +132,78 @@ __device__ void BitonicSort(unsigned long long *keys, int m) {
 
 // Sorts the occupied slots by (bin, k0): a counting sort by bin (per-bin
 // counts, their exclusive scan, then each slot's key k0 << 20 | slot placed
-// in its bin's run), then each bin's run sorted by k0 by one thread
-// (insertion sort; a run holds the few modes of one bin). The subtraction
-// later walks each bin's modes in increasing k0, an order that does not
-// depend on the table layout. Thread 0 also evaluates this iteration's FP32
-// error scale eps. Shared memory: the keys (half the table, BucketKeys),
-// then the bins' counts and fill positions.
-__global__ void __launch_bounds__(1024) k_bucket(const SigIter *__restrict__ its,
-                                                 int max_bins, int prep) {
-  PdlEnter(its, kTraceBucket);
+// in its bin's run), then a key's place in its run is the number of smaller keys
+// there (a run holds the few modes of one bin). The subtraction later walks each
+// bin's modes in increasing k0, an order that does not depend on the table layout.
+// Shared memory: the keys (half the table, BucketKeys), then the bins' counts and
+// fill positions.
+// prep: kBucketOnly sorts by the bins k_mode_prep left, kBucketBins evaluates k1
+// and the bins itself, kBucketTerms the modes' row-0 terms too.
+// One block per signal, on the decisions' critical path, bound by the latency of
+// its steps: each thread holds the slot, key and bin of its first kHeld modes in
+// registers through all of them (51 bins and 1000 modes with their terms: 10 us,
+// of which 4.7 us the terms; 3 us without them and with the modes held). Solves in
+// the fixed-bins phase evaluate the terms beside it (k_mode_terms32): one recovery
+// of 1000 modes 1110 -> 1065 us, 64 signals 5378 -> 5338 us.
+constexpr int kBucketThreads = 1024, kHeld = 2;
+__global__ void __launch_bounds__(kBucketThreads) k_bucket(const SigIter *__restrict__ its,
+                                                           int max_bins, int prep) {
+  const SigIter &it = PdlEnterLoaded<false>(its, blockIdx.x, kTraceBucket);
   extern __shared__ unsigned long long keys[];
-  const SigIter &it = its[blockIdx.x];
   if (!it.active) return;
   const int B = it.bins;
   const int occ = *it.tab_count;
-  if (prep) {
-    // the mode preparation of k_mode_prep for this signal's slots first
-    // (one kernel fewer at the start of an iteration)
-    for (int i = threadIdx.x; i < occ; i += blockDim.x) {
-      ModePrepSlot(it, it.occ_list[i], 0);
-    }
-    __syncthreads();  // their bins are visible to the whole block
-  }
   int *cnt = reinterpret_cast<int *>(keys + BucketKeys(it.tab_cap));
   int *fill = cnt + max_bins;
+  const bool terms32 = TermsIn32(it);
+  int h_slot[kHeld], h_bin[kHeld];
+  int32_t h_key[kHeld];
+  for (int b = threadIdx.x; b < B; b += kBucketThreads) cnt[b] = 0;
+  auto read = [&](int i, int *slot, int32_t *key, int *bin) {
+    *slot = it.occ_list[i];
+    *key = it.tab_key[*slot];
+    if (prep == kBucketOnly) {
+      *bin = it.mode_bin[*slot];
+      return;
+    }
+    const int64_t k1 = ModeK1(it, *key, bin);
+    it.mode_k1[*slot] = int32_t(k1);
+    it.mode_bin[*slot] = *bin;
+    if (prep == kBucketTerms) {
+      if (terms32) {
+        ModeTerms32(it, *slot, *key, k1, *bin);
+      } else {
+        ModeTerms64(it, *slot, k1, *bin);
+      }
+    }
+  };
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u) {
+    const int i = threadIdx.x + u * kBucketThreads;
+    if (i < occ) read(i, &h_slot[u], &h_key[u], &h_bin[u]);
+  }
   // shared keys were sized for half the table (BucketKeys); more occupied
   // slots end the solve with a capacity status instead of overflowing
   if (occ > BucketKeys(it.tab_cap)) {
     if (threadIdx.x == 0) atomicOr(&it.flags[1], kStatusCapacity);
     return;
   }
-  for (int b = threadIdx.x; b < B; b += blockDim.x) cnt[b] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < occ; i += blockDim.x) {
-    atomicAdd(&cnt[it.mode_bin[it.occ_list[i]]], 1);
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u) {
+    if (threadIdx.x + u * kBucketThreads < occ) atomicAdd(&cnt[h_bin[u]], 1);
+  }
+  for (int i = threadIdx.x + kHeld * kBucketThreads; i < occ; i += kBucketThreads) {
+    int sl, bin;
+    int32_t key;
+    read(i, &sl, &key, &bin);
+    atomicAdd(&cnt[bin], 1);
   }
   __syncthreads();
   // exclusive scan of the counts: each thread a contiguous chunk, then the
-  // chunk totals by warp shuffles and one pass over the warps' totals
-  __shared__ int warp_tot[32];
-  const int per = (B + blockDim.x - 1) / blockDim.x;
+  // chunk totals by warp shuffles, and the warps' totals by every warp's
+  __shared__ int warp_tot[kBucketThreads / 32];
+  const int per = (B + kBucketThreads - 1) / kBucketThreads;
   const int b0 = threadIdx.x * per;
   int local = 0;
   for (int b = b0; b < b0 + per && b < B; ++b) local += cnt[b];
@@ -164,16 +216,10 @@ __global__ void __launch_bounds__(1024) k_bucket(const SigIter *__restrict__ its
   }
   if (lane == 31) warp_tot[warp] = incl;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int w = 0; w < int(blockDim.x >> 5); ++w) {
-      const int t = warp_tot[w];
-      warp_tot[w] = acc;
-      acc += t;
-    }
-  }
-  __syncthreads();
-  int run = warp_tot[warp] + incl - local;
+  int before = lane < warp ? warp_tot[lane] : 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  int run = before + incl - local;
   for (int b = b0; b < b0 + per && b < B; ++b) {
     fill[b] = run;
     it.bkt_start[b] = run;
@@ -181,24 +227,36 @@ __global__ void __launch_bounds__(1024) k_bucket(const SigIter *__restrict__ its
     run += cnt[b];
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < occ; i += blockDim.x) {
+  auto place = [&](int sl, int32_t key, int bin) {
+    keys[atomicAdd(&fill[bin], 1)] =
+        (static_cast<unsigned long long>(uint32_t(key)) << 20) |
+        static_cast<unsigned long long>(sl);
+  };
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u) {
+    if (threadIdx.x + u * kBucketThreads < occ) place(h_slot[u], h_key[u], h_bin[u]);
+  }
+  for (int i = threadIdx.x + kHeld * kBucketThreads; i < occ; i += kBucketThreads) {
     const int sl = it.occ_list[i];
-    const int pos = atomicAdd(&fill[it.mode_bin[sl]], 1);
-    keys[pos] = (static_cast<unsigned long long>(uint32_t(it.tab_key[sl])) << 20) |
-                static_cast<unsigned long long>(sl);
+    place(sl, it.tab_key[sl], it.mode_bin[sl]);
   }
   __syncthreads();
-  // each bin's run in increasing k0 (keys are distinct: one slot per k0): a
-  // key's place in its run is the number of smaller keys in the run, every
-  // key ranked by its own thread (runs are a bin's few modes)
-  for (int i = threadIdx.x; i < occ; i += blockDim.x) {
-    const unsigned long long k = keys[i];
-    // the run holding position i: the bin whose [start, fill) contains it
-    const int bin = it.mode_bin[int(k & 0xFFFFFu)];
-    const int st = fill[bin] - cnt[bin], en = fill[bin];
-    int rank = 0;
-    for (int j = st; j < en; ++j) rank += keys[j] < k ? 1 : 0;
-    it.bkt_list[st + rank] = int32_t(k & 0xFFFFFu);
+  // keys are distinct: one slot per k0; fill is now every run's end
+  auto rank = [&](int sl, int32_t key, int bin) {
+    const unsigned long long k = (static_cast<unsigned long long>(uint32_t(key)) << 20) |
+                                 static_cast<unsigned long long>(sl);
+    const int en = fill[bin], st = en - cnt[bin];
+    int r = st;
+    for (int j = st; j < en; ++j) r += keys[j] < k ? 1 : 0;
+    it.bkt_list[r] = sl;
+  };
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u) {
+    if (threadIdx.x + u * kBucketThreads < occ) rank(h_slot[u], h_key[u], h_bin[u]);
+  }
+  for (int i = threadIdx.x + kHeld * kBucketThreads; i < occ; i += kBucketThreads) {
+    const int sl = it.occ_list[i];
+    rank(sl, it.tab_key[sl], it.mode_bin[sl]);
   }
 }
 
@@ -670,6 +728,12 @@ void LaunchModePrep(const SigIter *d_its, int nsig, int max_cap, cudaStream_t s,
   Launch(k_mode_prep, grid, 64, 0, s, d_its, cond ? 1 : 0);
 }
 
+void LaunchModeTerms32(const SigIter *d_its, int nsig, int max_cap, cudaStream_t s) {
+  // a mode per thread up to 2048, in blocks small enough to spread
+  dim3 grid(std::min(32, std::max(1, max_cap / 2 / 64)), nsig);
+  Launch(k_mode_terms32, grid, 64, 0, s, d_its);
+}
+
 // Shared memory of k_bucket: the keys, then two ints per bin.
 inline size_t BucketSmem(int max_cap, int max_bins) {
   return size_t(BucketKeys(max_cap)) * sizeof(unsigned long long) +
@@ -677,11 +741,11 @@ inline size_t BucketSmem(int max_cap, int max_bins) {
 }
 
 void LaunchBucket(const SigIter *d_its, int nsig, int max_bins, int max_cap,
-                  cudaStream_t s, bool prep) {
+                  cudaStream_t s, BucketPrep prep) {
   const size_t sm = BucketSmem(max_cap, max_bins);
   cudaFuncSetAttribute(k_bucket, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        int(sm));
-  Launch(k_bucket, nsig, 1024, sm, s, d_its, max_bins, prep ? 1 : 0);
+  Launch(k_bucket, nsig, kBucketThreads, sm, s, d_its, max_bins, int(prep));
 }
 
 void LaunchDecide(const SigIter *d_its, int nsig, int max_bins, int max_trials,

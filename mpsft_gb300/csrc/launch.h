@@ -145,10 +145,14 @@ constexpr int kEnergyStride = kEnergyParts;
 void LaunchEnergy(const void *const *x, const int64_t *n, int nsig, bool c128,
                   double *energy, cudaStream_t s, int per_block);
 
-// Lists of table slots per bin (counting sort by bin); prep: the mode
-// preparation of LaunchModePrep first, in the same kernel.
+// Lists of table slots per bin (counting sort by bin), by the bins LaunchModePrep
+// left, with the bins evaluated in the same kernel, or with the modes' row-0 terms
+// too.
+enum BucketPrep { kBucketOnly, kBucketBins, kBucketTerms };
 void LaunchBucket(const SigIter *d_its, int nsig, int max_bins, int max_cap,
-                  cudaStream_t s, bool prep = false);
+                  cudaStream_t s, BucketPrep prep);
+// The FP32 row-0 terms alone, for kBucketBins.
+void LaunchModeTerms32(const SigIter *d_its, int nsig, int max_cap, cudaStream_t s);
 
 // Per-bin mode subtraction, energy test, pencil votes and coefficient
 // estimation (the bin loop of Iterate); writes the candidates. With

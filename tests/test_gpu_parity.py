@@ -775,3 +775,31 @@ def test_bins_on_the_device(ctx, prec, bins):
         assert np.array_equal(got[skip:skip + size], want.view(np.float64).ravel())
         assert (got[:skip] == 7.25).all() and (got[skip + size:] == 7.25).all()
     sig.free()
+
+
+@pytest.mark.parametrize("prec", PRECS, ids=PREC_IDS)
+@pytest.mark.parametrize("found", [2, 60, 93, 96, 99, 200])
+def test_iterate_found_modes_per_bin(ctx, port, prec, found):
+    """An iteration with about found / 3 known modes in each of three bins (fewer
+    and more than a warp's lanes) and one unknown mode: it is the one the oracle
+    finds, with its coefficient. FP32: a value of the bin carries at most
+    17 * 2^-24 of the largest magnitude (kEpsRms and friends), here below
+    found + 1, and the window response divides it by 0.1 or more."""
+    n, bins = 1 << 14, 3
+    rng = np.random.default_rng(found)
+    k = rng.choice(n, found + 1, replace=False)
+    c = np.exp(2j * np.pi * rng.random(found + 1))
+    spec = np.zeros(n, np.complex128)
+    spec[k] = c
+    x = (np.fft.ifft(spec) * n).astype(np.complex64).astype(np.complex128)
+    mm = {int(k[i]): complex(c[i]) for i in range(found)}
+    kw = dict(window_delta=1e-6, trials=1, bin_threshold=0.05, window_threshold=0.1,
+              mm=mm)
+    port.seed(11)
+    _, want = port.iterate(x, bins, **kw)
+    sig = ctx.upload(x.astype(np.complex64))
+    _, got = ctx.iterate(sig, m.Rng(11), bins, precision=prec, **kw)
+    sig.free()
+    assert sorted(got) == sorted(want)
+    tol = 17 * 2.0**-24 * (found + 1) / 0.1 if prec == m.FP32 else 1e-9
+    assert max(abs(got[q] - want[q]) for q in want) < tol
