@@ -546,23 +546,25 @@ __device__ int DecideBin(const SigIter &it, int beta, const Src &src,
   };
   if (npre > 0) load_modes(0, &mode_err);
   float errw = 0.f;
-  for (int i = 0; i < (kSums ? 0 : nm); ++i) {
-    if (i > 0 && (i & 31) == 0) load_modes(i, &errw);
-    V bs[TMAX];
+  for (int i0 = 0; i0 < (kSums ? 0 : nm); i0 += 32) {
+    if (i0 > 0) load_modes(i0, &errw);
+    const int m = min(nm - i0, 32);
+#pragma unroll 4
+    for (int i = 0; i < m; ++i) {
 #pragma unroll
-    for (int t = 0; t < TMAX; ++t) {
-      if (t < TR) {
-        bs[t].x = __shfl_sync(0xffffffffu, pre_base[t].x, i & 31);
-        bs[t].y = __shfl_sync(0xffffffffu, pre_base[t].y, i & 31);
+      for (int t = 0; t < TMAX; ++t) {
+        if (t < TR) {
+          V b;
+          b.x = __shfl_sync(0xffffffffu, pre_base[t].x, i);
+          b.y = __shfl_sync(0xffffffffu, pre_base[t].y, i);
+          u0[t] = vsub2(u0[t], b);
+        }
       }
     }
-    if (i >= 32) {
-      const float e = __shfl_sync(0xffffffffu, errw, i & 31);
+    // (the errors of the first 32 modes stay on their lanes)
+    for (int i = 0; i < (i0 > 0 ? m : 0); ++i) {
+      const float e = __shfl_sync(0xffffffffu, errw, i);
       if (lane == 0) mode_err += e;
-    }
-#pragma unroll
-    for (int t = 0; t < TMAX; ++t) {
-      if (t < TR) u0[t] = vsub2(u0[t], bs[t]);
     }
   }
   if (fp32) {

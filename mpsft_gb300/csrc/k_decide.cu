@@ -245,9 +245,16 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket(const SigIter *__rest
   auto rank = [&](int sl, int32_t key, int bin) {
     const unsigned long long k = (static_cast<unsigned long long>(uint32_t(key)) << 20) |
                                  static_cast<unsigned long long>(sl);
+    // (four keys' loads in flight: one after the other they took half the kernel)
     const int en = fill[bin], st = en - cnt[bin];
     int r = st;
-    for (int j = st; j < en; ++j) r += keys[j] < k ? 1 : 0;
+    for (int j = st; j < en; j += 4) {
+      unsigned long long q[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) q[u] = keys[min(j + u, en - 1)];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) r += j + u < en && q[u] < k ? 1 : 0;
+    }
     it.bkt_list[r] = sl;
   };
 #pragma unroll
