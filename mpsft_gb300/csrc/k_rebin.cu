@@ -25,11 +25,12 @@
 // from x again (random accesses, at the random-gather rate).
 //
 // Work item = (signal, listed bin, trial, listed row, chunk of the support;
-// RebinChunks(p) chunks),
-// one warp each; the 32 lanes split the chunk into consecutive runs; lane sums
-// are combined by a fixed shuffle tree and the chunk partials by another in
-// whichever warp finishes a row's last chunk (so the result does not depend on
-// the scheduling).
+// RebinChunks(p) chunks), by one warp: the 32 lanes split the chunk into
+// consecutive runs; lane sums are combined by a fixed shuffle tree and the chunk
+// partials by another in whichever warp finishes a row's last chunk (so the result
+// does not depend on the scheduling). A group of warps takes a listed bin's trial,
+// each every so manieth of its items with one evaluation of the bin's phase-step
+// powers: these are 40 of the 70 FP64 instructions of a single item, 64 cycles each.
 #include "common.cuh"
 #include "launch.h"
 #include "rebin.cuh"
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(256, 2)
   __shared__ int64_t items_end[kRebinMaxSignals];
   __shared__ float4 pw_s[8][kPowLen];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // the signals' work item counts and their inclusive prefix sums, by warp 0
+  // the signals' listed bins times trials and their inclusive prefix sums, by warp 0
   // (32 signals per step, a shuffle scan each)
   if (warp == 0) {
     int64_t carry = 0;
@@ -178,7 +179,7 @@ __global__ void __launch_bounds__(256, 2)
         const SigIter &q = s == 0 ? first : its[s];
         if (q.active && !q.force_fp64) {
           const int nf = *(volatile int32_t *)&q.flags[2];
-          if (nf <= q.esc_cap) items = int64_t(nf) * q.trials * q.rows * RebinChunks(q.p);
+          if (nf <= q.esc_cap) items = int64_t(nf) * q.trials;
         }
       }
 #pragma unroll
@@ -193,45 +194,33 @@ __global__ void __launch_bounds__(256, 2)
   __syncthreads();
   float4 *pw = pw_s[warp];
   const int64_t total = items_end[nsig - 1];
-  // (a row's chunks go to as many blocks: rows that are not listed leave gaps
-  // in the items, and with a row's chunks on the warps of a few blocks some SMs
-  // had three times the work of others)
-  for (int64_t w = int64_t(warp) * gridDim.x + blockIdx.x; w < total;
-       w += int64_t(gridDim.x) * 8) {
+  // warps per unit: all of them shared out, or with few for each, eight per unit
+  // and several units for a warp, so that no warp has much more than another. A
+  // unit's warps are on as many blocks.
+  const uint32_t units = uint32_t(total), warps = gridDim.x * 8;
+  uint32_t group = units > 0 ? warps / units : 1;
+  if (group < 4) group = 8;
+  for (uint32_t w = uint32_t(warp) * gridDim.x + blockIdx.x; w < units * group;
+       w += warps) {
+    uint32_t local = w / group;
+    const int g0 = int(w - local * group);
     int sig = 0;
-    while (w >= items_end[sig]) ++sig;
-    // (a signal's items: at most kMaxListed * kMaxTrials * rows * chunks,
-    // far below 2^32, so the decode divides in 32 bits)
-    uint32_t local = uint32_t(w - (sig > 0 ? items_end[sig - 1] : 0));
+    while (int64_t(local) >= items_end[sig]) ++sig;
+    local -= uint32_t(sig > 0 ? items_end[sig - 1] : 0);
     const SigIter &it = sig == 0 ? first : its[sig];
     const int nch = RebinChunks(it.p);
-    const int c = int(local % uint32_t(nch));
-    local /= uint32_t(nch);
-    const int r = int(local % uint32_t(it.rows));
-    local /= uint32_t(it.rows);
-    const int t = int(local % uint32_t(it.trials));
     const int e = int(local / uint32_t(it.trials));
-    // row not listed (a null mask lists every row)
-    if (r > 0 && it.esc_mask != nullptr &&
-        !((it.esc_mask[e] >> ((r - 1) >> 1)) & 1u)) {
-      continue;
-    }
+    const int t = int(local - uint32_t(e) * uint32_t(it.trials));
+    // the rows: 0, and those of the bits whose decisions were near (a null mask
+    // lists every row)
+    const uint32_t bits = it.esc_mask != nullptr ? it.esc_mask[e] : 0xffffffffu;
+    const uint32_t listed = it.bits < 32 ? bits & ((1u << it.bits) - 1u) : bits;
+    const int items = (1 + 2 * __popc(listed)) * nch;
+    if (g0 >= items) continue;
     const int beta = it.esc_list[e];
     const int64_t n = it.n;
     const int64_t B = it.bins;
     const ModN mod{uint32_t(n), it.n_inv};
-    int64_t off = 0;
-    if (r > 0) {
-      const int s = (r - 1) / 2;
-      off = (r & 1) ? (B << s) : -(B << s);
-    }
-    const int64_t tau = int64_t(it.q[t]) + off;
-    const int64_t chunk = (int64_t(it.p) + nch - 1) / nch;
-    const int64_t c0 = -int64_t(it.p2) + c * chunk;
-    const int64_t c1 = min(c0 + chunk, int64_t(it.p2) + 1);
-    const int64_t per = (chunk + 31) / 32;
-    const int64_t t0 = c0 + lane * per;
-    const int64_t t1 = min(t0 + per, c1);
     // the bin's phase-step powers s^k (k < 64) into shared memory and s^64
     // (StepPowers): from the per-bin tables its preparation filled, else
     // evaluated here
@@ -250,61 +239,80 @@ __global__ void __launch_bounds__(256, 2)
     pw[lane] = p0;
     pw[lane + 32] = p1;
     __syncwarp();
-    double tr = 0.0, ti = 0.0;
-    // the row's samples from the fold's stash when it wrote them (read in
-    // order), else gathered from x
-    const TX *__restrict__ sx = nullptr;
-    if (it.stash != nullptr && __ldcg(reinterpret_cast<const int32_t *>(it.stash)) == 1) {
-      const int srows = StashRows(it);
-      const TX *s0 = reinterpret_cast<const TX *>(it.stash + kStashHeader) + it.p2;
-      if (r < srows) {
-        sx = s0 + (size_t(t) * srows + r) * it.p;
-      } else if (srows == 1 && c0 + off >= -int64_t(it.p2) && c1 - 1 + off <= it.p2) {
-        sx = s0 + size_t(t) * it.p + off;
+    const int64_t chunk = (int64_t(it.p) + nch - 1) / nch;
+    for (int i = g0; i < items; i += int(group)) {
+      const int row = i / nch, c = i - row * nch;
+      int r = 0;
+      int64_t off = 0;
+      if (row > 0) {
+        uint32_t left = listed;
+        for (int k = (row - 1) >> 1; k > 0; --k) left &= left - 1;
+        const int s = __ffs(left) - 1;
+        r = 2 * s + 1 + ((row - 1) & 1);
+        off = (r & 1) ? (B << s) : -(B << s);
       }
-    }
-    if (t0 < t1) {
-      const int64_t twoB = 2 * B;
-      const int64_t u0 = mod(tau + t0);
-      uint32_t j = mod(int64_t(it.a) * u0 + it.c);
-      const uint32_t astep = mod(it.a);
-      const uint32_t nn = uint32_t(n);
-      const int64_t m0 = mod(int64_t(bm) * u0);
-      const int64_t r0 = PosMod(g * t0, twoB);
-      const double2 a0 = StepPhase(it, m0, r0);
-      // (only complex64 input has a stash)
-      if (sizeof(TX) == sizeof(float2) && sx != nullptr) {
-        SumRun<TX, true>(sx, 0u, 0u, 0u, it.wtff, pw, t0, t1, S, a0.x, a0.y, &tr, &ti);
-      } else {
-        SumRun<TX, false>(reinterpret_cast<const TX *>(it.x), j, astep, nn, it.wtff, pw,
-                          t0, t1, S, a0.x, a0.y, &tr, &ti);
+      const int64_t tau = int64_t(it.q[t]) + off;
+      const int64_t c0 = -int64_t(it.p2) + c * chunk;
+      const int64_t c1 = min(c0 + chunk, int64_t(it.p2) + 1);
+      const int64_t per = (chunk + 31) / 32;
+      const int64_t t0 = c0 + lane * per;
+      const int64_t t1 = min(t0 + per, c1);
+      double tr = 0.0, ti = 0.0;
+      // the row's samples from the fold's stash when it wrote them (read in
+      // order), else gathered from x
+      const TX *__restrict__ sx = nullptr;
+      if (it.stash != nullptr && __ldcg(reinterpret_cast<const int32_t *>(it.stash)) == 1) {
+        const int srows = StashRows(it);
+        const TX *s0 = reinterpret_cast<const TX *>(it.stash + kStashHeader) + it.p2;
+        if (r < srows) {
+          sx = s0 + (size_t(t) * srows + r) * it.p;
+        } else if (srows == 1 && c0 + off >= -int64_t(it.p2) && c1 - 1 + off <= it.p2) {
+          sx = s0 + size_t(t) * it.p + off;
+        }
       }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      tr += __shfl_xor_sync(0xffffffffu, tr, o);
-      ti += __shfl_xor_sync(0xffffffffu, ti, o);
-    }
-    // the warp that completes a (trial, row) adds its chunk partials in
-    // chunk order (the result does not depend on which warp that is)
-    const size_t etr = (size_t(e) * it.trials + t) * it.rows + r;
-    int last = 0;
-    if (lane == 0) {
-      it.esc_part[etr * kRebinChunks + c] = make_double2(tr, ti);
-      __threadfence();
-      last = atomicAdd(&it.esc_cnt[etr], 1) == nch - 1;
-    }
-    if (__shfl_sync(0xffffffffu, last, 0)) {
-      // one chunk per lane, then a fixed shuffle tree
-      __threadfence();
-      double2 s = make_double2(0.0, 0.0);
-      if (lane < nch) s = __ldcg(&it.esc_part[etr * kRebinChunks + lane]);
+      if (t0 < t1) {
+        const int64_t twoB = 2 * B;
+        const int64_t u0 = mod(tau + t0);
+        uint32_t j = mod(int64_t(it.a) * u0 + it.c);
+        const uint32_t astep = mod(it.a);
+        const uint32_t nn = uint32_t(n);
+        const int64_t m0 = mod(int64_t(bm) * u0);
+        const int64_t r0 = PosMod(g * t0, twoB);
+        const double2 a0 = StepPhase(it, m0, r0);
+        // (only complex64 input has a stash)
+        if (sizeof(TX) == sizeof(float2) && sx != nullptr) {
+          SumRun<TX, true>(sx, 0u, 0u, 0u, it.wtff, pw, t0, t1, S, a0.x, a0.y, &tr, &ti);
+        } else {
+          SumRun<TX, false>(reinterpret_cast<const TX *>(it.x), j, astep, nn, it.wtff, pw,
+                            t0, t1, S, a0.x, a0.y, &tr, &ti);
+        }
+      }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
-        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+        tr += __shfl_xor_sync(0xffffffffu, tr, o);
+        ti += __shfl_xor_sync(0xffffffffu, ti, o);
       }
-      if (lane == 0) it.esc_sum[etr] = s;
+      // the warp that completes a (trial, row) adds its chunk partials in
+      // chunk order (the result does not depend on which warp that is)
+      const size_t etr = (size_t(e) * it.trials + t) * it.rows + r;
+      int last = 0;
+      if (lane == 0) {
+        it.esc_part[etr * kRebinChunks + c] = make_double2(tr, ti);
+        __threadfence();
+        last = atomicAdd(&it.esc_cnt[etr], 1) == nch - 1;
+      }
+      if (__shfl_sync(0xffffffffu, last, 0)) {
+        // one chunk per lane, then a fixed shuffle tree
+        __threadfence();
+        double2 s = make_double2(0.0, 0.0);
+        if (lane < nch) s = __ldcg(&it.esc_part[etr * kRebinChunks + lane]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+          s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+        }
+        if (lane == 0) it.esc_sum[etr] = s;
+      }
     }
   }
 }
