@@ -803,3 +803,24 @@ def test_iterate_found_modes_per_bin(ctx, port, prec, found):
     assert sorted(got) == sorted(want)
     tol = 17 * 2.0**-24 * (found + 1) / 0.1 if prec == m.FP32 else 1e-9
     assert max(abs(got[q] - want[q]) for q in want) < tol
+
+
+@pytest.mark.parametrize("bits", [0, 3])
+@pytest.mark.parametrize("bins", [1, 3, 303, 305, 607, 609, 1217])
+def test_direct_bins_per_warp(ctx, port, bins, bits):
+    """The direct summation with fewer and more bins than warps to share out
+    among them, against the oracle within the FP64 bins' tolerance."""
+    n = 1 << 14
+    rng = np.random.default_rng(bins)
+    x = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    a, b, c, q = 4097, 77, 5, 4099
+    want = port.bin_in_time(x, bins, bits, 1e-5, a, b, c, q)
+    for dtype in (np.complex64, np.complex128):
+        xs = x.astype(dtype)
+        if dtype == np.complex64:
+            want32 = port.bin_in_time(xs.astype(np.complex128), bins, bits, 1e-5, a, b,
+                                      c, q)
+        sig = ctx.upload(xs)
+        u = ctx.bin_in_time(sig, bins, bits, 1e-5, a, b, c, q, precision=m.FP64_DIRECT)
+        sig.free()
+        assert rel_err(u, want32 if dtype == np.complex64 else want) < TOL_BINS[m.FP64]
