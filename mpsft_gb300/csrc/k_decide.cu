@@ -269,8 +269,8 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket(const SigIter *__rest
 
 // One warp per bin. cond: only signals whose iteration is redone in FP64
 // (more near-tie bins than their list holds) take part.
-template <typename T, int TMAX>
-__global__ void __launch_bounds__(256, (sizeof(T) == 4 && TMAX == 1) ? 6 : 1)
+template <typename T, int TMAX, int MINB>
+__global__ void __launch_bounds__(256, MINB)
     k_decide(const SigIter *__restrict__ its, int mode, int cond, int mark) {
   const SigIter &it = PdlEnterLoaded(its, blockIdx.y, kTraceDecide);
   if (!it.active) return;
@@ -693,7 +693,16 @@ void LaunchDecideT(const SigIter *d_its, int nsig, int max_bins, int mode,
   // blocks of eight, 21 us in blocks of one)
   const int w = sizeof(T) == 8 && int64_t(max_bins) * nsig <= 152 * 16 ? 1 : 8;
   dim3 grid((max_bins + w - 1) / w, nsig);
-  Launch(k_decide<T, TMAX>, grid, 32 * w, 0, s, d_its, mode, cond, mark);
+  // FP32, one trial: six blocks per SM (40 registers) while there are more than
+  // four for each, else four (64 registers: the row factors of four modes side by
+  // side). One recovery of 1000 modes 940 us with four throughout, 948 with six; 64
+  // signals 5185 and 5125 us.
+  constexpr bool kSix = sizeof(T) == 4 && TMAX == 1;
+  if (kSix && int64_t(max_bins) * nsig > 152 * 4 * 8) {
+    Launch(k_decide<T, TMAX, kSix ? 6 : 1>, grid, 32 * w, 0, s, d_its, mode, cond, mark);
+  } else {
+    Launch(k_decide<T, TMAX, kSix ? 4 : 1>, grid, 32 * w, 0, s, d_its, mode, cond, mark);
+  }
 }
 
 template <typename T>
@@ -828,8 +837,8 @@ bool DecideKernelsLaunchable() {
                        int(smb));
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e, k_export_tables, 1024, smb);
   a = a < e ? a : e;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_decide<double, kMaxTrials>, 256, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_decide<float, kMaxTrials>, 256, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_decide<double, kMaxTrials, 1>, 256, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_decide<float, kMaxTrials, 1>, 256, 0);
   int l = 0, l1 = 0, l5 = 0, d = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&l, k_listed_terms<kMaxTrials, 2, 1>, 64, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&l1, k_listed_terms<1, 8, 4>, 256, 0);
