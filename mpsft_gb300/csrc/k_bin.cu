@@ -204,14 +204,17 @@ __device__ void FoldClusterWarp(const SigIter &it, int tr, int beta, int sc,
 // 32-bit turns for sincospif. SPLIT, BATCH and CLUSTER (the row cluster on,
 // or every group folded pairwise) are the launch shape the autotuner picks
 // (FoldShapeOf); every shape computes the same sums up to FP32 rounding.
+// The descriptor is read from shared memory (after the wait: its writer stands
+// right before): a block's misses on it, one after the other, stood before its first
+// gather, and a small fold's blocks do little else (a binning of 2^22 samples in 501
+// bins 63.9 -> 55.9 us, of 2^26 in 8001 bins 171.7 -> 168.6 us).
 template <typename TX, int SPLIT, int BATCH, bool CLUSTER>
 __global__ void __launch_bounds__(256, 4)
     k_bin_fold32(const SigIter *__restrict__ its, int gmax) {
   constexpr int kFoldSplit = SPLIT;
   constexpr int kFoldBatch = BATCH;
   constexpr int kFoldBins = 256 / SPLIT;  // bins per CTA
-  PdlEnter(its, kTraceFold);
-  const SigIter &it = its[blockIdx.z];
+  const SigIter &it = PdlEnterLoaded<false>(its, blockIdx.z, kTraceFold);
   if (!it.active || it.force_fp64) return;
   const int B = it.bins;
   const int g = blockIdx.y % gmax;
