@@ -112,9 +112,8 @@ static_assert(kModCols + kModFolds <= kModThreads, "a thread per phase");
 
 __global__ void __launch_bounds__(kModThreads)
     k_window_mod(const SigIter *__restrict__ its, int eval, int cond) {
-  PdlEnter();
+  const SigIter &it = PdlEnterLoaded<false>(its, blockIdx.y, kTraceWindow64);
   __shared__ double2 zr[kModCols], zf[kModFolds];
-  const SigIter &it = its[blockIdx.y];
   if (!it.active) return;
   if (cond ? !RedoFP64(it) : it.force_fp64) return;
   const int B = it.bins;
