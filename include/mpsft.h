@@ -192,7 +192,7 @@ int mpsft_bin_in_time_wt(mpsft_ctx *ctx, const mpsft_signal *sig, int32_t bins,
  * and out_device ((1 + 2*bits) x bins complex128, row-major) are the caller's
  * device memory, and the work runs asynchronously on stream (a cudaStream_t;
  * NULL = the legacy default stream). Scratch is one fixed array of about
- * 2.5 MiB compiled into the library and held on every GPU that loads it.
+ * 2.7 MiB compiled into the library and held on every GPU that loads it.
  * Limits: bins <= 2047, bits <= 20, window folds p/bins <= 80; larger sizes
  * return MPSFT_ERR_CAPACITY. n must be prime or a power of two, as for
  * mpsft_bin_in_time (MPSFT_ERR_UNSUPPORTED_N otherwise). Every call resolves
