@@ -109,24 +109,63 @@ __global__ void __launch_bounds__(64) k_mode_terms32(const SigIter *__restrict__
   }
 }
 
+// Compare-exchange of the keys a at index i (lane or lane + 32 of a run of 64) at
+// a distance within the warp.
+__device__ __forceinline__ unsigned long long ExchangeLanes(unsigned long long a, int i,
+                                                            int size, int stride) {
+  const unsigned long long b = __shfl_xor_sync(0xffffffffu, a, stride);
+  return ((i & stride) == 0) == ((i & size) == 0) ? min(a, b) : max(a, b);
+}
+
 // Ascending bitonic sort of keys[0..m) in shared memory (m a power of two),
-// by the whole block; ends with a barrier.
+// by the whole block; ends with a barrier. The steps at distances below 64 run in
+// registers, a warp on 64 keys: a barrier per step (66 of them at 2048 keys, 21
+// now) was what the export of a table cost.
 __device__ void BitonicSort(unsigned long long *keys, int m) {
-  for (int size = 2; size <= m; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < m; i += blockDim.x) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const bool up = (i & size) == 0;
-          const unsigned long long a = keys[i], b = keys[j];
-          if ((a > b) == up) {
-            keys[i] = b;
-            keys[j] = a;
-          }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  auto step = [&](int size, int stride) {
+    for (int i = threadIdx.x; i < m; i += blockDim.x) {
+      const int j = i ^ stride;
+      if (j > i) {
+        const bool up = (i & size) == 0;
+        const unsigned long long a = keys[i], b = keys[j];
+        if ((a > b) == up) {
+          keys[i] = b;
+          keys[j] = a;
         }
       }
-      __syncthreads();
     }
+    __syncthreads();
+  };
+  if (m < 64) {
+    for (int size = 2; size <= m; size <<= 1) {
+      for (int stride = size >> 1; stride > 0; stride >>= 1) step(size, stride);
+    }
+    return;
+  }
+  for (int size = 64; size <= m; size <<= 1) {
+    for (int stride = size >> 1; stride >= 64; stride >>= 1) step(size, stride);
+    for (int b = warp * 64; b < m; b += warps * 64) {
+      const int i0 = b + lane, i1 = i0 + 32;
+      unsigned long long x = keys[i0], y = keys[i1];
+      // the first pass: all sizes up to 64
+      for (int sz = size == 64 ? 2 : size; sz <= size; sz <<= 1) {
+        if (sz >= 64) {
+          if ((x > y) == ((i0 & sz) == 0)) {
+            const unsigned long long t = x;
+            x = y;
+            y = t;
+          }
+        }
+        for (int stride = min(sz >> 1, 16); stride > 0; stride >>= 1) {
+          x = ExchangeLanes(x, i0, sz, stride);
+          y = ExchangeLanes(y, i1, sz, stride);
+        }
+      }
+      keys[i0] = x;
+      keys[i1] = y;
+    }
+    __syncthreads();
   }
 }
 

@@ -824,3 +824,21 @@ def test_direct_bins_per_warp(ctx, port, bins, bits):
         u = ctx.bin_in_time(sig, bins, bits, 1e-5, a, b, c, q, precision=m.FP64_DIRECT)
         sig.free()
         assert rel_err(u, want32 if dtype == np.complex64 else want) < TOL_BINS[m.FP64]
+
+
+@pytest.mark.parametrize("count", [1, 2, 31, 33, 63, 64, 65, 129, 2047, 2049, 5000])
+def test_iterate_returns_sorted_modes(ctx, count):
+    """An iteration that finds nothing returns the modes it was given in
+    increasing frequency with their coefficients bit for bit, for tables of
+    fewer and more modes than the sort's runs."""
+    n = 1 << 16
+    rng = np.random.default_rng(count)
+    k = rng.choice(n, count, replace=False)
+    c = rng.standard_normal(count) + 1j * rng.standard_normal(count)
+    sig = ctx.upload(np.zeros(n, np.complex64))
+    mm = {int(a): complex(b) for a, b in zip(k, c)}
+    found, got = ctx.iterate(sig, m.Rng(3), 51, bin_threshold=1e9, mm=mm)
+    sig.free()
+    assert not found
+    assert list(got) == sorted(mm)
+    assert all(got[q] == mm[q] for q in mm)
