@@ -417,7 +417,7 @@ __device__ __forceinline__ void PdlEnter(const SigIter *its, int32_t id) {
 // 843 us, 64 signals 5532 -> 5455 us, an FP64 iteration at 101 bins 109 -> 106 us.
 template <bool Early = true>
 __device__ __forceinline__ const SigIter &PdlEnterLoaded(const SigIter *__restrict__ its,
-                                                         unsigned sig, int32_t id) {
+                                                         unsigned sig, int32_t id = 0) {
   if (!Early) PdlEnter();
   constexpr unsigned kWords = sizeof(SigIter) / sizeof(unsigned long long);
   static_assert(sizeof(SigIter) % sizeof(unsigned long long) == 0, "whole words");
@@ -427,7 +427,8 @@ __device__ __forceinline__ const SigIter &PdlEnterLoaded(const SigIter *__restri
   if (Early) PdlEnter();
   __syncthreads();
   const SigIter &it = *reinterpret_cast<const SigIter *>(words);
-  if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
+  if (id != 0 && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 &&
+      blockIdx.z == 0) {
     TraceEntry(it, id);
   }
   return it;

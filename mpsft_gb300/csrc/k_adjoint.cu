@@ -66,8 +66,7 @@ __device__ inline ModeSetup SetupMode(const SigIter &it, int32_t k0, int lane) {
 __global__ void __launch_bounds__(32) k_estimate(const SigIter *__restrict__ its,
                                                  const int32_t *k0s, int64_t m,
                                                  double2 *coef) {
-  PdlEnter();
-  const SigIter &it = *its;
+  const SigIter &it = PdlEnterLoaded(its, 0);
   const int lane = threadIdx.x;
   for (int64_t i = blockIdx.x; i < m; i += gridDim.x) {
     const ModeSetup ms = SetupMode(it, k0s[i], lane);
@@ -95,8 +94,7 @@ __global__ void __launch_bounds__(32) k_estimate(const SigIter *__restrict__ its
 __global__ void __launch_bounds__(32) k_adjoint_spread(const SigIter *__restrict__ its,
                                                        const int32_t *k0s,
                                                        const double2 *g, int64_t m) {
-  PdlEnter();
-  const SigIter &it = *its;
+  const SigIter &it = PdlEnterLoaded<false>(its, 0);
   const int lane = threadIdx.x;
   double2 *G = reinterpret_cast<double2 *>(it.fold);
   for (int64_t i = blockIdx.x; i < m; i += gridDim.x) {
@@ -121,8 +119,7 @@ __global__ void __launch_bounds__(32) k_adjoint_spread(const SigIter *__restrict
 // 33 us at 401 bins and 25 rows, now 8 us.
 __global__ void __launch_bounds__(256) k_adjoint_scatter(const SigIter *__restrict__ its,
                                                          double2 *dx) {
-  PdlEnter();
-  const SigIter &it = *its;
+  const SigIter &it = PdlEnterLoaded(its, 0);
   const int tt = blockIdx.x * blockDim.x + threadIdx.x;
   const int r = blockIdx.y, t = blockIdx.z;
   if (tt >= it.p) return;

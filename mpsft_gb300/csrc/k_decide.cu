@@ -625,8 +625,7 @@ __global__ void __launch_bounds__(1024) k_table_load(const SigIter *__restrict__
                                                      const int32_t *__restrict__ k0,
                                                      const double2 *__restrict__ coef,
                                                      int64_t m) {
-  PdlEnter();
-  const SigIter &it = *its;
+  const SigIter &it = PdlEnterLoaded<false>(its, 0);
   for (int i = threadIdx.x; i < it.tab_cap; i += blockDim.x) {
     it.tab_key[i] = kEmptyKey;
     it.tab_coef[i] = make_double2(0.0, 0.0);
