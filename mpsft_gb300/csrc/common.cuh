@@ -208,6 +208,8 @@ struct SigIter {
   // 1 when the table's coefficients already carry their window responses
   // (wf * coef, from a caller's window), so that the mode terms use wf = 1
   int32_t unit_wf;
+  // 1 in solves: window offsets as the reference rounds them (WindowOffset)
+  int32_t quot_xi;
   int32_t *esc_list;    // esc_cap bins
   uint32_t *esc_mask;   // per listed bin: bit s set = rows 2s+1, 2s+2 near
   int32_t esc_cap;
@@ -568,14 +570,28 @@ __device__ inline double WindowInFreq(const SigIter &it, double xi) {
   return 0.5 * (erf((xi + c) * it.erf_d) - erf((xi - c) * it.erf_d));
 }
 
+// xi = (bin + 1/2)/B - k1/n, the offset of a mode or candidate from the middle of
+// its bin. Single calls evaluate it from its exact numerator (|num| < 2^53): no
+// division and no cancellation, an error in BinInFreq's terms of 6e-16 instead of
+// 7e-14. Solves (quot_xi) form the difference of the two rounded quotients as the
+// reference does (src/binner.cc:565-591, src/iterate.cc:139-171): its error of
+// about 2^-53, times erf_d, is up to 5e-12 of a mode, and recoveries of nearly
+// noiseless modes decide at thresholds that such a difference crosses. With the
+// exact offset one of 100 uneven FP32 batches of 24 such signals, and eight of 100
+// in FP64, ended in other sets of frequencies.
+__device__ inline double WindowOffset(const SigIter &it, int64_t k1, int bin) {
+  if (it.quot_xi) {
+    return (double(bin) + 0.5) / double(it.bins) - double(k1) / double(it.n);
+  }
+  const int64_t num = (2 * int64_t(bin) + 1) * it.n - 2 * int64_t(it.bins) * k1;
+  return double(num) * it.xi_scale;
+}
+
 // FP64 row-0 terms wf c e^{2 pi i (q_t k1 + c k0)/n} of the mode in table
 // slot s (k1 and its bin given) into mode_base (BinInFreqV1::Run,
 // src/binner.cc:565-591).
 __device__ inline void ModeTerms64(const SigIter &it, int s, int64_t k1, int bin) {
-  // xi = (bin + 1/2)/B - k1/n from its exact numerator (|num| < 2^53): no FP64
-  // division, and no cancellation
-  const int64_t num = (2 * int64_t(bin) + 1) * it.n - 2 * int64_t(it.bins) * k1;
-  const double xi = double(num) * it.xi_scale;
+  const double xi = WindowOffset(it, k1, bin);
   const double2 wc =
       it.unit_wf ? it.tab_coef[s] : cscale(it.tab_coef[s], WindowInFreq(it, xi));
   const int32_t key = it.tab_key[s];

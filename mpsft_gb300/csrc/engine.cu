@@ -1653,6 +1653,7 @@ int SolveMany(mpsft_ctx *ctx, const mpsft_signal *const *sigs,
     std::memset(&its[i], 0, sizeof(SigIter));
     CarveSignal(cv, shapes[i], &its[i], &ctls[i]);
     its[i].n = int32_t(sigs[i]->n);
+    its[i].quot_xi = 1;
     phase_entries = std::max(phase_entries, PhaseTableEntries(sigs[i]->n));
   }
   // the signals of the first one's length share the context's phase tables

@@ -555,11 +555,15 @@ __device__ void MergeBin(const SigIter &it, int beta, bool go) {
   // this bin's range
   const int64_t k1 = v == 2 ? int64_t(k0) : int64_t(mod(int64_t(it.a) * k0 + it.b));
   const bool own = int64_t(mod.quot(k1 * int64_t(it.bins))) == beta;
-  // xi0 = k1/n - (beta + 1/2)/B from its exact integer numerator
-  // (|num| < 2^53) and 1/(2nB)
+  // (FP64 solves finish their candidates with the reference's operations too, as
+  // WindowOffset does with its offset; those of FP32 calls, nearly noiseless signals
+  // in FP64 kernels among them, always used the exact offset)
+  const bool quot = it.quot_xi && !(it.eps_rel > 0.f);
+  // xi0 = k1/n - (beta + 1/2)/B, exactly: its numerator (|num| < 2^53) and 1/(2nB)
   const int64_t num =
       2 * int64_t(it.bins) * k1 - (2 * int64_t(beta) + 1) * int64_t(it.n);
-  const double xi = double(num) * it.xi_scale, c = 0.5 * it.width;
+  const double xi = quot ? -WindowOffset(it, k1, beta) : double(num) * it.xi_scale;
+  const double c = 0.5 * it.width;
   const double e = erf((half ? xi - c : xi + c) * it.erf_d);
   const double wf = 0.5 * (e - __shfl_xor_sync(0xffffffffu, e, 1));
   if (!go || half) return;
@@ -570,14 +574,20 @@ __device__ void MergeBin(const SigIter &it, int beta, bool go) {
       it.cand_valid[beta] = 0;
       return;
     }
-    // one FP64 division per candidate (each is a long sequence on this part's
-    // FP64 pipes)
     const double m = double(it.trials * (1 + 2 * it.bits));
-    const double scale = 1.0 / (m * wf);  // the average and the window
     k0 = int32_t(mod(int64_t(it.a_inv) * mod(k1 - it.b)));
-    coef = cmul(coef, Phase64(it, -int64_t(it.c) * k0));
-    coef = make_double2(coef.x * scale, coef.y * scale);
-    err = err * fabs(m * scale);
+    const double2 ph = Phase64(it, -int64_t(it.c) * k0);
+    if (quot) {
+      coef = cmul(make_double2(coef.x / m, coef.y / m), ph);
+      coef = make_double2(coef.x / wf, coef.y / wf);
+    } else {
+      // one FP64 division per candidate (each is a long sequence on this part's
+      // FP64 pipes)
+      const double scale = 1.0 / (m * wf);  // the average and the window
+      coef = cmul(coef, ph);
+      coef = make_double2(coef.x * scale, coef.y * scale);
+      err = err * fabs(m * scale);
+    }
     it.cand_k0[beta] = k0;
     it.cand_coef[beta] = coef;
     it.cand_err[beta] = err;

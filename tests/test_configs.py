@@ -142,3 +142,34 @@ def test_config5_stress(ctx, port):
           f"true={int(hits.sum())}/{sg.k.size} precision_err={err:.2e} "
           f"near_ties={st.escalated}")
     assert err < 1e-5
+
+
+def _uneven_spec(i):
+    """A nearly noiseless signal of the uneven batch's kind: n in 2^16, 2^17,
+    50 to 400 modes of modulus 1, sigma 1e-6."""
+    g = np.random.default_rng([77, i])
+    n = 1 << int(g.integers(16, 18))
+    s = int(g.integers(50, 401))
+    k = np.sort(g.choice(n, s, replace=False)).astype(np.int32)
+    return n, k, np.exp(2j * np.pi * g.uniform(size=s))
+
+
+@pytest.mark.parametrize("prec", [m.FP32, m.FP64], ids=["fp32", "fp64"])
+def test_uneven_sub_batch_matches_oracle(ctx, port, prec):
+    """Every frequency set of a 48-signal uneven batch is the oracle's. Their
+    noise lies below the samples' own rounding, so that late iterations decide
+    within 1e-11 of thresholds: signal 7288 (in FP64 also 1662 and 3225) ends in
+    another set when the window offsets of found modes and candidates are
+    rounded differently from the reference's difference of quotients."""
+    ids = [7288] + list(range(47)) if prec == m.FP32 else [1662, 3225, 7288] + list(range(45))
+    specs = [_uneven_spec(i) for i in ids]
+    sigs = [ctx.generate(n, k, c, 1e-6, i, m.C64) for i, (n, k, c) in zip(ids, specs)]
+    opts = [_opts(ctx, k.size, 1e-6, prec) for _, k, _ in specs]
+    out, stats = ctx.solve_batched(sigs, [m.Rng(500 + i) for i in ids], opts)
+    for i, (n, k, _), sg, (got, _), st in zip(ids, specs, sigs, out, stats):
+        assert st["status"] == 0, i
+        want, _ = port.demo1_run(sg.read().astype(np.complex128), k.size, 1e-6, 500 + i,
+                                 min_bins=51, window_delta=1e-5, max_stale_iter=5)
+        assert got.tolist() == sorted(want), i
+    for sg in sigs:
+        sg.free()
