@@ -198,10 +198,11 @@ struct SigIter {
   // FP32 path only: 1 when this signal's FP32 rounding is not small against
   // its noise thresholds, so this iteration runs on the FP64 kernels
   int32_t force_fp64;
-  // 1 when the window and Bluestein tables (FP32; FP64 for a signal with
-  // force_fp64) for this iteration's bins are in place (the previous iteration's, the context's table cache, or built
-  // in this iteration by another signal of the batch): the table kernels skip
-  // this signal
+  // 1 when the window and Bluestein tables for this iteration's bins are in place
+  // (the previous iteration's, the context's table cache, or built in this
+  // iteration by another signal of the batch): the table kernels skip this signal.
+  // FP64 tables for a signal with force_fp64, which takes the FP64 kernels in every
+  // iteration of a call, FP32 ones otherwise
   int32_t tables_valid;
   // table cache slot (bins >> 1) this signal builds in this iteration, or -1
   int32_t win_slot;
@@ -659,9 +660,11 @@ __device__ inline bool Pencil(double2 u0, double2 u1, double2 u2,
 }
 
 // True when signal `it` takes the FP64 kernels of the FP32 path this
-// iteration: by the precision policy, or because its near-tie list overflowed.
+// iteration: by the precision policy, or because its near-tie list overflowed
+// and its transform is one that they have (the policy forces no other).
 __device__ inline bool RedoFP64(const SigIter &it) {
-  return it.force_fp64 || *(volatile int32_t *)&it.flags[2] > it.esc_cap;
+  return it.force_fp64 || (it.fft_m <= kMaxFFT64 &&
+                           *(volatile int32_t *)&it.flags[2] > it.esc_cap);
 }
 
 // ---- the FP32 binning's row cluster -------------------------------------

@@ -882,6 +882,15 @@ Maxima MaximaOf(const std::vector<SigIter> &h_its) {
   return mx;
 }
 
+// The shape of an FP32 call's FP64 kernels (RedoFP64): its signals with the
+// transforms that these have. A larger signal of the batch stays on the FP32
+// kernels and must not keep the forced ones from theirs.
+Maxima RedoMaxima(Maxima mx) {
+  mx.m = std::min(mx.m, kMaxFFT64);
+  mx.bins = std::min(mx.bins, kMaxFFT64 / 2);
+  return mx;
+}
+
 // The kernels of one iteration of every active signal, on stream s (and the
 // context's side stream, forked from and joined back into s). tables: the
 // window and Bluestein tables are in place (CtxTable). single: a call of one
@@ -956,7 +965,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
                            cudaStream_t s, const Ahead *ahead = nullptr,
                            bool tables = false, bool single = false) {
   if (mx.bins == 0) return MPSFT_OK;
-  if (forced == kAllForced && !fp64 && mx.m <= kMaxFFT64) {
+  if (forced == kAllForced && !fp64) {
     return LaunchForcedIteration(ctx, d_its, nsig, mx, x_c128, timer, launched, s, tables);
   }
   const bool any_forced = forced != kNoneForced;
@@ -1045,7 +1054,7 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
   // near-tie list overflowed) run the FP64 kernels (redo). Without redo the
   // other bins' merge runs beside the re-binning: the FP32 decide holds the
   // listed bins back and their FP64 decision merges them.
-  const bool redo = !fp64 && any_forced && mx.m <= kMaxFFT64;
+  const bool redo = !fp64 && any_forced;
   const bool side_merge = !fp64 && !redo;
   LaunchDecide(d_its, nsig, mx.bins, mx.trials, !fp64, false, s, false, side_merge);
   // Bluestein setup, mode preparation with bucketing, window(s), fold, FFT,
@@ -1071,23 +1080,24 @@ int LaunchIterationKernels(mpsft_ctx *ctx, const SigIter *d_its, int nsig,
     LaunchDecideListed(d_its, nsig, mx.trials, redo, side_merge, s);
     if (launched) *launched += 3;  // mode terms, re-binning, FP64 decisions
     if (redo) {
+      const Maxima rx = RedoMaxima(mx);
       LaunchModePrep(d_its, nsig, mx.cap, s, true);
-      LaunchBluesteinSetup(d_its, nsig, mx.m, true, ctx->tw32, ctx->tw64, s, true);
-      LaunchWindowMod(d_its, nsig, mx.bins, kWindowRead, true, s);
+      LaunchBluesteinSetup(d_its, nsig, rx.m, true, ctx->tw32, ctx->tw64, s, true);
+      LaunchWindowMod(d_its, nsig, rx.bins, kWindowRead, true, s);
       if (timer && ctx->profiling) LaunchDelay(20000, s);
       if (timer) {
         int rc = timer->Begin(1);
         if (rc) return rc;
       }
-      LaunchBinFold(d_its, nsig, mx.bins, mx.bits, mx.trials, x_c128, true, s,
+      LaunchBinFold(d_its, nsig, rx.bins, mx.bits, mx.trials, x_c128, true, s,
                     true);
       if (timer) {
         int rc = timer->End();
         if (rc) return rc;
       }
-      LaunchRowFFT(d_its, nsig, mx.rows, mx.trials, mx.m, true, ctx->tw32,
+      LaunchRowFFT(d_its, nsig, mx.rows, mx.trials, rx.m, true, ctx->tw32,
                    ctx->tw64, s, true);
-      LaunchDecide(d_its, nsig, mx.bins, mx.trials, false, false, s, true);
+      LaunchDecide(d_its, nsig, rx.bins, mx.trials, false, false, s, true);
       if (launched) *launched += 6;
     }
   }
@@ -1319,7 +1329,7 @@ int GraphLoop(mpsft_ctx *ctx, const mpsft_signal *const *sigs,
     }
   }
   // the fixed-bins phase runs pipelined on the FP32 path without FP64 redo
-  const bool pipe = !fp64 && !(forced != kNoneForced && mx.m <= kMaxFFT64);
+  const bool pipe = !fp64 && forced == kNoneForced;
   // graph (rebuilt when the launch shape or the arena changes)
   const std::vector<int64_t> key = {
       int64_t(reinterpret_cast<uintptr_t>(ctx->arena)), nsig, mx.bins, mx.bits,

@@ -463,8 +463,9 @@ __global__ void __launch_bounds__(32 * W) k_listed_terms(const SigIter *__restri
 // FP64 decisions of the listed near-tie bins: one warp per listed bin (lane s
 // holds bit s), on the re-binned rows (FromRebin) minus the bin's found modes
 // (esc_msub): energy threshold, then DecideTail, and the bin's candidate into
-// the table. Signals whose list overflowed are redone whole instead (redo),
-// or marked unresolved, their held-back bins keeping their FP32 candidates.
+// the table. Signals whose list overflowed are redone whole instead (redo, and
+// RedoFP64), or marked unresolved, their held-back bins keeping their FP32
+// candidates.
 template <int TMAX>
 __global__ void __launch_bounds__(256)
     k_decide_listed(const SigIter *__restrict__ its, int redo, int merge) {
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(256)
   if (it.force_fp64) return;
   const int nf = *(volatile int32_t *)&it.flags[2];
   if (nf > it.esc_cap) {
-    if (!redo && blockIdx.x == 0 && threadIdx.x == 0) {
+    if (!(redo && RedoFP64(it)) && blockIdx.x == 0 && threadIdx.x == 0) {
       atomicOr(&it.flags[1], kStatusUnresolved);
     }
     if (merge && threadIdx.x < 32) {

@@ -173,3 +173,41 @@ def test_uneven_sub_batch_matches_oracle(ctx, port, prec):
         assert got.tolist() == sorted(want), i
     for sg in sigs:
         sg.free()
+
+
+@pytest.mark.parametrize("stale", [5, 20])
+@pytest.mark.parametrize("host_loop", [False, True], ids=["graph", "host"])
+def test_forced_signals_beside_large_ones(ctx, host_loop, stale):
+    """Nearly noiseless signals, which the precision policy sends to the FP64
+    kernels, in one FP32 batch with a signal of 2100 modes at 40 dB, whose 4201
+    bins take a transform that those kernels do not have: each returns what its
+    own solve returns."""
+    sigs, opts, seeds = [], [], []
+    for i, (n, s) in enumerate([(1 << 18, 50), (1 << 21, 2100), (1 << 20, 100)]):
+        g = np.random.default_rng([78, i])
+        k = np.sort(g.choice(n, s, replace=False)).astype(np.int32)
+        c = np.exp(2j * np.pi * g.uniform(size=s))
+        sigma = 1e-2 * np.sqrt(s) if s > 1000 else 1e-6
+        sigs.append(ctx.generate(n, k, c, sigma, 780 + i, m.C64))
+        opts.append(ctx.solve_options(s, sigma, trials=1, min_bins=51, window_delta=1e-5,
+                                      window_threshold=0.1, max_stale_iter=stale,
+                                      precision=m.FP32))
+        seeds.append(600 + i)
+    single = [ctx.solve_arrays(sg, m.Rng(sd), o) for sg, sd, o in zip(sigs, seeds, opts)]
+    ctx.set_profiling(host_loop)
+    try:
+        out, stats = ctx.solve_batched(sigs, [m.Rng(sd) for sd in seeds], opts)
+    finally:
+        ctx.set_profiling(False)
+    assert stats[1]["fp64_iterations"] == 0
+    for i, ((k, c), st, (k1, c1, st1)) in enumerate(zip(out, stats, single)):
+        assert st["status"] == st1.status == 0, i
+        assert st["iterations"] == st1.iterations, i
+        assert np.array_equal(k, k1), i
+        if i == 1:
+            assert np.allclose(c, c1, rtol=1e-5, atol=1e-6), i
+        else:
+            assert st["fp64_iterations"] == st["iterations"], i
+            assert np.array_equal(c.view(np.uint64), c1.view(np.uint64)), i
+    for sg in sigs:
+        sg.free()
