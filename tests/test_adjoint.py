@@ -219,3 +219,23 @@ def test_estimate_rows_over_lanes(ctx, port, n, bins, trials, modes):
     ahg = ctx.adjoint(n, su, k, g)
     lhs, rhs = np.vdot(g, got), np.vdot(ahg, x)
     assert abs(lhs - rhs) <= 1e-12 * np.linalg.norm(g) * np.linalg.norm(got) * 10
+
+
+@pytest.mark.parametrize("modes", [1023, 1024, 1025, 1027, 8191, 8192, 8193, 8225])
+@pytest.mark.parametrize("trials", [1, 3])
+def test_estimate_many_modes(ctx, port, modes, trials):
+    """32, 8 and 1 lanes per mode, around the counts where they change and with
+    partly filled warps; both ways in which modes and gradients reach the device."""
+    n, bins = 1 << 14, 51
+    rng = np.random.default_rng(modes)
+    k = rng.choice(n, modes, replace=False).astype(np.int32)
+    x = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    su = _setup(ctx, n, bins, 1e-5, trials, 5)
+    sig = ctx.upload(x)
+    got = ctx.estimate(sig, su, k)
+    want = _reference_estimate(port, x, su, k)
+    assert np.abs(got - want).max() <= 1e-10 * np.abs(want).max()
+    g = rng.standard_normal(modes) + 1j * rng.standard_normal(modes)
+    ahg = ctx.adjoint(n, su, k, g)
+    lhs, rhs = np.vdot(g, got), np.vdot(ahg, x)
+    assert abs(lhs - rhs) <= 1e-12 * np.linalg.norm(g) * np.linalg.norm(got) * 10
