@@ -547,14 +547,11 @@ __global__ void __launch_bounds__(256)
 // on each lane of the pair (one recovery of 1000 modes 1055 -> 1032 us).
 __device__ void MergeBin(const SigIter &it, int beta, bool go) {
   const int half = threadIdx.x & 1;
-  const int v = go ? it.cand_valid[beta] : 0;
-  go = v == 1 || v == 2;
+  go = go && it.cand_valid[beta] == 2;
   if (!__any_sync(0xffffffffu, go)) return;
-  int32_t k0 = go ? it.cand_k0[beta] : 0;
   const ModN mod{uint32_t(it.n), it.n_inv};
-  // k1 of the candidate (pending: cand_k0 holds it), and whether it lies in
-  // this bin's range
-  const int64_t k1 = v == 2 ? int64_t(k0) : int64_t(mod(int64_t(it.a) * k0 + it.b));
+  // the candidate's k1, and whether it lies in this bin's range
+  const int64_t k1 = go ? it.cand_k0[beta] : 0;
   const bool own = int64_t(mod.quot(k1 * int64_t(it.bins))) == beta;
   // (FP64 solves finish their candidates with the reference's operations too, as
   // WindowOffset does with its offset; those of FP32 calls, nearly noiseless signals
@@ -568,31 +565,22 @@ __device__ void MergeBin(const SigIter &it, int beta, bool go) {
   const double e = erf((half ? xi - c : xi + c) * it.erf_d);
   const double wf = 0.5 * (e - __shfl_xor_sync(0xffffffffu, e, 1));
   if (!go || half) return;
+  if (fabs(wf) < it.win_thr) return;
   double2 coef = it.cand_coef[beta];
   double err = it.cand_err[beta];
-  if (v == 2) {
-    if (fabs(wf) < it.win_thr) {
-      it.cand_valid[beta] = 0;
-      return;
-    }
-    const double m = double(it.trials * (1 + 2 * it.bits));
-    k0 = int32_t(mod(int64_t(it.a_inv) * mod(k1 - it.b)));
-    const double2 ph = Phase64(it, -int64_t(it.c) * k0);
-    if (quot) {
-      coef = cmul(make_double2(coef.x / m, coef.y / m), ph);
-      coef = make_double2(coef.x / wf, coef.y / wf);
-    } else {
-      // one FP64 division per candidate (each is a long sequence on this part's
-      // FP64 pipes)
-      const double scale = 1.0 / (m * wf);  // the average and the window
-      coef = cmul(coef, ph);
-      coef = make_double2(coef.x * scale, coef.y * scale);
-      err = err * fabs(m * scale);
-    }
-    it.cand_k0[beta] = k0;
-    it.cand_coef[beta] = coef;
-    it.cand_err[beta] = err;
-    it.cand_valid[beta] = 1;
+  const double m = double(it.trials * (1 + 2 * it.bits));
+  const int32_t k0 = int32_t(mod(int64_t(it.a_inv) * mod(k1 - it.b)));
+  const double2 ph = Phase64(it, -int64_t(it.c) * k0);
+  if (quot) {
+    coef = cmul(make_double2(coef.x / m, coef.y / m), ph);
+    coef = make_double2(coef.x / wf, coef.y / wf);
+  } else {
+    // one FP64 division per candidate (each is a long sequence on this part's
+    // FP64 pipes)
+    const double scale = 1.0 / (m * wf);  // the average and the window
+    coef = cmul(coef, ph);
+    coef = make_double2(coef.x * scale, coef.y * scale);
+    err = err * fabs(m * scale);
   }
   it.flags[0] = 1;
   if (!own) {
