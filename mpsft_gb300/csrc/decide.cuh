@@ -139,7 +139,10 @@ template <typename V> __device__ inline float Abs32(V a) {
   return sqrtf(x * x + y * y);
 }
 
-enum DecideMode { kDecide = 0, kSubtractOnly = 1, kDecideExact = 2 };
+// kDecideHeld: kDecideExact beside k_merge; the bin's candidate stays marked as held
+// back (kCandListed), so that k_merge, whenever it gets to the bin, leaves it to the
+// decision.
+enum DecideMode { kDecide = 0, kSubtractOnly = 1, kDecideExact = 2, kDecideHeld = 3 };
 
 // k1 = round(n (beta + xi1) / B) with xi1 = (2 xs + 1) / 2^{L+1}, exactly in
 // integers: num = n (beta 2^{L+1} + 2 xs + 1) < 2^64, den = B 2^{L+1} < 2^33
@@ -339,7 +342,7 @@ __device__ __forceinline__ int DecideTail(const SigIter &it, int beta, int mode,
   // near-tie bins of the FP32 path: the rows that were not re-binned carry
   // the FP32 binning bound into the coefficient
   double err = 0.0;
-  if (!fp32 && mode == kDecideExact) {
+  if (!fp32 && mode >= kDecideExact) {
     float rm = 0.f, am = 0.f, msx = 0.f;
 #pragma unroll
     for (int t = 0; t < TMAX; ++t) {
@@ -366,7 +369,7 @@ __device__ __forceinline__ int DecideTail(const SigIter &it, int beta, int mode,
     it.cand_k0[beta] = int32_t(k1);
     it.cand_coef[beta] = make_double2(double(ax), double(ay));
     it.cand_err[beta] = err;
-    it.cand_valid[beta] = 2;
+    it.cand_valid[beta] = mode == kDecideHeld ? 2 + kCandListed : 2;
   }
   return listed;
 }

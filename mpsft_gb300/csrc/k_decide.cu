@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(256, MINB)
 // (k_decide_listed).
 constexpr int kListedBlocks = 8;
 
-__device__ void MergeBin(const SigIter &it, int beta, bool go);
+__device__ void MergeBin(const SigIter &it, int beta, bool go, int held);
 
 // FP64 mode subtraction of the listed bins, beside their re-binning: one
 // block of W warps per listed bin. The bin's found modes get their FP64
@@ -479,10 +479,7 @@ __global__ void __launch_bounds__(256)
     }
     if (merge && threadIdx.x < 32) {
       for (int e = blockIdx.x; e < it.esc_cap; e += kListedBlocks) {
-        const int beta = it.esc_list[e];
-        if (threadIdx.x == 0) it.cand_valid[beta] -= kCandListed;
-        __syncwarp();
-        MergeBin(it, beta, threadIdx.x < 2);
+        MergeBin(it, it.esc_list[e], threadIdx.x < 2, kCandListed);
       }
     }
     return;
@@ -525,29 +522,30 @@ __global__ void __launch_bounds__(256)
       go = false;
     }
     if (go) {
-      DecideTail<double, TMAX>(it, beta, kDecideExact, u0, up, um, 0.f, 0.f, false,
-                               -1);
+      DecideTail<double, TMAX>(it, beta, merge ? kDecideHeld : kDecideExact, u0, up, um,
+                               0.f, 0.f, false, -1);
     }
     // the bin's candidate (written by lane 0 above) into the table
     if (merge) {
       __syncwarp();
-      MergeBin(it, beta, lane < 2);
+      MergeBin(it, beta, lane < 2, kCandListed);
     }
   }
 }
 
 // ---------------------------------------------------------------- merge
 // Candidate of bin beta -> table, by a pair of neighbouring lanes (go: this
-// lane's bin has one to merge; every lane of the warp calls). A pending
+// lane's bin has one to merge; every lane of the warp calls; held: kCandListed for
+// the bins that k_merge, which may run at the same time, leaves alone). A pending
 // candidate is finished here in FP64 (src/iterate.cc:139-171): the window
 // response at xi0 = k1/n - (beta + 1/2)/B and its threshold, the average over
 // the T (1 + 2L) values, k0 = a^-1 (k1 - b) mod n, the factor e^{-2 pi i c k0/n}
 // and the division by the window response. The response's two erf, about 100
 // FP64 instructions each of 64 cycles, are much of what a merge waits for: one
 // on each lane of the pair (one recovery of 1000 modes 1055 -> 1032 us).
-__device__ void MergeBin(const SigIter &it, int beta, bool go) {
+__device__ void MergeBin(const SigIter &it, int beta, bool go, int held) {
   const int half = threadIdx.x & 1;
-  go = go && it.cand_valid[beta] == 2;
+  go = go && it.cand_valid[beta] == 2 + held;
   if (!__any_sync(0xffffffffu, go)) return;
   const ModN mod{uint32_t(it.n), it.n_inv};
   // the candidate's k1, and whether it lies in this bin's range
@@ -614,7 +612,7 @@ __global__ void __launch_bounds__(32) k_merge(const SigIter *__restrict__ its) {
   const SigIter &it = PdlEnterLoaded(its, blockIdx.y, kTraceMerge);
   if (!it.active) return;
   const int beta = blockIdx.x * 16 + (threadIdx.x >> 1);
-  MergeBin(it, beta, beta < it.bins);
+  MergeBin(it, beta, beta < it.bins, 0);
 }
 
 // One signal's mode table emptied, its control words cleared and the given
