@@ -33,13 +33,15 @@ constexpr int kRebinChunks = 32;   // re-binning: at most this many chunks of th
 // lane (32 lanes per chunk; a short support spreads over several warps, so
 // that each lane waits for few rounds of gathers), at most kRebinChunks (one
 // signal with a listed bin of 2001 bins, p = 62031: 41 us in 16 chunks, 27 us
-// in 32)
+// in 32). The direct evaluation of every bin has warps enough and pays an FP64
+// sincospi per lane and chunk: at most 16 (501 bins of 2^20 samples, p = 15531:
+// 1550 us, 2412 us in 31).
 constexpr int kStashHeader = 256;   // bytes before a stash buffer's samples
 // samples of a stash buffer at most (per trial: max(p, this))
 constexpr int64_t kStashMaxSamples = int64_t(1) << 20;
-__host__ __device__ inline int RebinChunks(int p) {
-  const int c = (p + 511) / 512;
-  return c < 1 ? 1 : (c > kRebinChunks ? kRebinChunks : c);
+__host__ __device__ inline int RebinChunks(int p, bool every_bin) {
+  const int c = (p + 511) / 512, most = every_bin ? kRebinChunks / 2 : kRebinChunks;
+  return c < 1 ? 1 : (c > most ? most : c);
 }
 constexpr int kMaxListed = 256;    // near-tie bins listed per signal/iteration
 constexpr int kRebinMaxSignals = 256;  // signals per FP64 re-binning launch
