@@ -23,8 +23,7 @@ from __future__ import annotations
 import collections.abc
 import ctypes
 import os
-import weakref
-from dataclasses import dataclass, field
+from dataclasses import dataclass
 
 import numpy as np
 
@@ -286,6 +285,22 @@ def _check(ctx, rc: int) -> None:
         raise MpsftError(rc, msg)
 
 
+class _SignalHandle:
+    """A signal's library handle, freed once: by the signal, or before that by
+    its context's close. Both hold it (the context strongly: when a cycle of the
+    two is collected, weak references are gone before either is finalized, and the
+    context may come first)."""
+    __slots__ = ("lib", "h", "freed")
+
+    def __init__(self, lib, h):
+        self.lib, self.h, self.freed = lib, h, False
+
+    def free(self) -> None:
+        if not self.freed and self.h:
+            self.freed = True
+            self.lib.mpsft_signal_free(self.h)
+
+
 class Context:
     """One CUDA device, one stream, reusable work buffers."""
 
@@ -301,7 +316,7 @@ class Context:
         self._out_k = np.empty(0, np.int32)
         self._out_c = np.empty(0, np.complex128)
         # live signals of this context: freed before the context itself
-        self._signals = weakref.WeakSet()
+        self._signals: set = set()
         tuning = os.environ.get("MPSFT_TUNING_FILE", TUNING_PATH)
         if tuning != "none" and os.path.exists(tuning):
             self.tuning_load(tuning)
@@ -353,6 +368,7 @@ class Context:
         if getattr(self, "_h", None):
             for sg in list(getattr(self, "_signals", ())):
                 sg.free()
+            self._signals = set()
             self._lib.mpsft_ctx_destroy(self._h)
             self._h = None
 
@@ -388,17 +404,13 @@ class Context:
         h = ctypes.c_void_p()
         _check(self, self._lib.mpsft_signal_upload(self._h, _ptr(x), x.size, dt,
                                                    ctypes.byref(h)))
-        sg = Signal(self, h, x.size, dt)
-        self._signals.add(sg)
-        return sg
+        return Signal(self, h, x.size, dt)
 
     def wrap_device(self, ptr: int, n: int, dtype: int) -> "Signal":
         h = ctypes.c_void_p()
         _check(self, self._lib.mpsft_signal_wrap_device(
             self._h, ctypes.c_void_p(ptr), int(n), int(dtype), ctypes.byref(h)))
-        sg = Signal(self, h, n, dtype)
-        self._signals.add(sg)
-        return sg
+        return Signal(self, h, n, dtype)
 
     def generate(self, n: int, k, coef, sigma: float, seed: int,
                  dtype: int = C64) -> "Signal":
@@ -413,9 +425,7 @@ class Context:
         _check(self, self._lib.mpsft_signal_generate(
             self._h, int(n), _ptr(k), _ptr(c), k.size, float(sigma),
             ctypes.c_uint64(int(seed) & (2**64 - 1)), int(dtype), ctypes.byref(h)))
-        sg = Signal(self, h, int(n), int(dtype))
-        self._signals.add(sg)
-        return sg
+        return Signal(self, h, int(n), int(dtype))
 
     def spectrum(self, sig: "Signal") -> np.ndarray:
         """xhat = FFT(x) / n in FP64, computed on the device."""
@@ -668,7 +678,14 @@ class Signal:
     _h: ctypes.c_void_p
     n: int
     dtype: int
-    _freed: bool = field(default=False)
+
+    def __post_init__(self) -> None:
+        self._handle = _SignalHandle(self.ctx._lib, self._h)
+        self.ctx._signals.add(self._handle)
+
+    @property
+    def _freed(self) -> bool:
+        return self._handle.freed
 
     def write(self, x: np.ndarray) -> None:
         """Refills the device copy from host memory (same n and dtype)."""
@@ -685,9 +702,8 @@ class Signal:
         return x
 
     def free(self) -> None:
-        if not self._freed and self._h:
-            self.ctx._lib.mpsft_signal_free(self._h)
-            self._freed = True
+        self._handle.free()
+        self.ctx._signals.discard(self._handle)
 
     def __del__(self):
         try:
