@@ -669,6 +669,18 @@ __device__ inline bool RedoFP64(const SigIter &it) {
                            *(volatile int32_t *)&it.flags[2] > it.esc_cap);
 }
 
+// The words of a copy of `bytes` bytes between addresses whose bitwise or is
+// `address`: 16 bytes each where both are 16-byte aligned, 4 where 4-byte aligned;
+// none (width 0) otherwise. The bytes past words * width are copied singly.
+struct CopyWords {
+  int width;
+  size_t words;
+};
+__host__ __device__ inline CopyWords CopySplit(uintptr_t address, size_t bytes) {
+  const int width = (address & 15u) == 0 ? 16 : ((address & 3u) == 0 ? 4 : 0);
+  return {width, width > 0 ? bytes / width : 0};
+}
+
 // ---- the FP32 binning's row cluster -------------------------------------
 // Row r's window covers u = off_r + t, |t| <= p2, of the permuted, modulated
 // samples y_u = x[a (q + u) + c] e^{2 pi i (b u / n - u / (2 bins))}, with
