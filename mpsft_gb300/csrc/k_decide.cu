@@ -764,8 +764,7 @@ void LaunchExportTables(const SigIter *d_its, int nsig, int max_cap,
                         int32_t *keys, double2 *coefs, int32_t *counts,
                         int32_t *sorted, cudaStream_t s) {
   const size_t sm = size_t(BucketKeys(max_cap)) * sizeof(unsigned long long);
-  cudaFuncSetAttribute(k_export_tables, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       int(sm));
+  AllowSmem(k_export_tables, size_t(BucketKeys(kMaxTableCap)) * sizeof(unsigned long long));
   Launch(k_export_tables, nsig, 1024, sm, s, d_its, nsig, keys, coefs, counts, sorted);
 }
 
@@ -791,11 +790,24 @@ inline size_t BucketSmem(int max_cap, int max_bins) {
          2 * sizeof(int) * size_t(max_bins);
 }
 
+// The most that a block may have beside the kernel's own shared memory: bins that no
+// transform bounds (BinInFreq with the caller's responses) take what there is.
+inline size_t BucketSmemMost() {
+  static const size_t most = [] {
+    cudaFuncAttributes fa{};
+    int dev = 0, optin = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaFuncGetAttributes(&fa, k_bucket);
+    return size_t(optin) - fa.sharedSizeBytes;
+  }();
+  return most;
+}
+
 void LaunchBucket(const SigIter *d_its, int nsig, int max_bins, int max_cap,
                   cudaStream_t s, BucketPrep prep) {
   const size_t sm = BucketSmem(max_cap, max_bins);
-  cudaFuncSetAttribute(k_bucket, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       int(sm));
+  AllowSmem(k_bucket, BucketSmemMost());
   Launch(k_bucket, nsig, kBucketThreads, sm, s, d_its, max_bins, int(prep));
 }
 
@@ -864,12 +876,10 @@ bool DecideKernelsLaunchable() {
   int a = 0, b = 0, c = 0;
   const size_t smb = size_t(BucketKeys(kMaxTableCap)) * sizeof(unsigned long long);
   const size_t smk = BucketSmem(kMaxTableCap, kMaxFFT / 2);
-  cudaFuncSetAttribute(k_bucket, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       int(smk));
+  AllowSmem(k_bucket, BucketSmemMost());
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_bucket, 1024, smk);
   int e = 0;
-  cudaFuncSetAttribute(k_export_tables, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       int(smb));
+  AllowSmem(k_export_tables, smb);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e, k_export_tables, 1024, smb);
   a = a < e ? a : e;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_decide<double, kMaxTrials, 1>, 256, 0);

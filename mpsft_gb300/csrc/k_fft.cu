@@ -594,8 +594,8 @@ template <typename V, int C>
 void LaunchRowSplit(const SigIter *d_its, dim3 grid, int max_m, const V *tw, cudaStream_t s,
                     bool cond) {
   const size_t sm = SplitSlots(max_m, C) * sizeof(V);
-  cudaFuncSetAttribute(k_row_fft_split<V, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       int(sm));
+  constexpr int kMost = sizeof(V) == sizeof(double2) ? kMaxFFT64 : kMaxFFT;
+  AllowSmem(k_row_fft_split<V, C>, SplitSlots(kMost, C) * sizeof(V));
   grid.x *= C;
   LaunchCluster(k_row_fft_split<V, C>, grid, kSplitThreads, sm, s, C, d_its, tw,
                 cond ? 1 : 0);
@@ -654,14 +654,12 @@ void LaunchRowFFT(const SigIter *d_its, int nsig, int max_rows,
   dim3 grid((max_rows + rpb - 1) / rpb, max_trials, nsig);
   if (fp64) {
     const size_t sm = RowFftSlots(max_m) * sizeof(double2);
-    cudaFuncSetAttribute(k_row_fft<double2>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+    AllowSmem(k_row_fft<double2>, RowFftSlots(kMaxFFT64) * sizeof(double2));
     Launch(k_row_fft<double2>, grid, kRowFftThreads, sm, s, d_its, max_trials, tw64,
                                                         cond ? 1 : 0, rpb_cap);
   } else {
     const size_t sm = RowFftSlots(max_m) * sizeof(float2);
-    cudaFuncSetAttribute(k_row_fft<float2>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+    AllowSmem(k_row_fft<float2>, RowFftSlots(kMaxFFT) * sizeof(float2));
     Launch(k_row_fft<float2>, grid, kRowFftThreads, sm, s, d_its, max_trials, tw32,
                                                        cond ? 1 : 0, rpb_cap);
   }
@@ -671,15 +669,12 @@ bool FftKernelsLaunchable() {
   int n1 = 0, n2 = 0;
   const size_t sm32 = RowFftSlots(kMaxFFT) * sizeof(float2);
   const size_t sm64 = RowFftSlots(kMaxFFT64) * sizeof(double2);
-  cudaFuncSetAttribute(k_row_fft<float2>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm32));
-  cudaFuncSetAttribute(k_row_fft<double2>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm64));
+  AllowSmem(k_row_fft<float2>, sm32);
+  AllowSmem(k_row_fft<double2>, sm64);
   // split rows: the largest transform over the smallest cluster
   int n3 = 0;
   const size_t sms = SplitSlots(kMaxFFT64, 2) * sizeof(double2);
-  cudaFuncSetAttribute(k_row_fft_split<double2, 2>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(sms));
+  AllowSmem(k_row_fft_split<double2, 2>, sms);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n3, k_row_fft_split<double2, 2>,
                                                 kSplitThreads, sms);
   if (n3 == 0) return false;

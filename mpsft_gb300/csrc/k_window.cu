@@ -281,13 +281,11 @@ void LaunchBluesteinSetup(const SigIter *d_its, int nsig, int max_m, bool fp64,
                           cudaStream_t s, bool cond) {
   if (fp64) {
     const size_t sm = size_t(PadLen(max_m)) * sizeof(double2);
-    cudaFuncSetAttribute(k_bluestein_setup<double2>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+    AllowSmem(k_bluestein_setup<double2>, size_t(PadLen(kMaxFFT64)) * sizeof(double2));
     Launch(k_bluestein_setup<double2>, nsig, 512, sm, s, d_its, tw64, cond ? 1 : 0);
   } else {
     const size_t sm = size_t(PadLen(max_m)) * sizeof(float2);
-    cudaFuncSetAttribute(k_bluestein_setup<float2>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+    AllowSmem(k_bluestein_setup<float2>, size_t(PadLen(kMaxFFT)) * sizeof(float2));
     Launch(k_bluestein_setup<float2>, nsig, 512, sm, s, d_its, tw32, cond ? 1 : 0);
   }
 }
@@ -367,10 +365,8 @@ bool WindowKernelsLaunchable() {
   int n1 = 0, n2 = 0;
   const size_t sm32 = size_t(PadLen(kMaxFFT)) * sizeof(float2);
   const size_t sm64 = size_t(PadLen(kMaxFFT64)) * sizeof(double2);
-  cudaFuncSetAttribute(k_bluestein_setup<float2>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm32));
-  cudaFuncSetAttribute(k_bluestein_setup<double2>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm64));
+  AllowSmem(k_bluestein_setup<float2>, sm32);
+  AllowSmem(k_bluestein_setup<double2>, sm64);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n1, k_bluestein_setup<float2>, 512, sm32);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n2, k_bluestein_setup<double2>, 512, sm64);
   return n1 > 0 && n2 > 0;

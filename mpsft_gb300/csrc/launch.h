@@ -52,6 +52,14 @@ inline void Launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   LaunchCluster(kernel, grid, block, smem, s, 1, args...);
 }
 
+// Lets a kernel be launched with up to `most` bytes of dynamic shared memory. The
+// limit is one per kernel and device for the whole process, so every launch sets the
+// most that the kernel ever takes: a context on another thread must not lower it
+// between this call and the launch.
+template <typename K> inline void AllowSmem(K kernel, size_t most) {
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most));
+}
+
 // The FFT twiddle table (kTwiddleEntries entries, TwiddleAt).
 void LaunchTwiddles(float2 *tw32, double2 *tw64, cudaStream_t s);
 // dst (device) = src_dev (device address of pinned, mapped host memory), any
