@@ -171,20 +171,22 @@ struct mpsft_ctx {
   double2 *ph_cache = nullptr;
   int64_t ph_cache_n = 0;
   // tables of the single-signal calls (bins, estimates, Iterate), kept like FFT
-  // plans under what they depend on (CtxTable): bounded, least recently used
-  // out first, freed with the context
+  // plans under what they depend on (CtxTable), in one allocation (table_pool, made
+  // by the first of these calls, freed with the context) that is filled in turns:
+  // a new table takes the place of the oldest that lie where it goes
   struct Table {
     int kind;
     int32_t bins;
     int64_t n;
     double delta;
-    unsigned char *ptr;
-    size_t bytes;
-    uint64_t used;  // the last call that asked for it
-    bool built;     // its builder's call has completed
+    size_t off, bytes;  // in the pool
+    uint64_t used;      // the last call that asked for it
+    bool built;         // its builder's call has completed
   };
   std::vector<Table> tables;
-  size_t table_bytes = 0;
+  unsigned char *table_pool = nullptr;
+  size_t table_head = 0;    // where the next table goes
+  bool tables_open = false; // a call has asked for tables and not completed
   uint64_t table_call = 0;
   size_t win_bytes = 0;
   double win_delta = 0.0;

@@ -63,3 +63,27 @@ def test_bucket_takes_bins_beyond_every_transform(ctx):
             ph = ((q + off) * k1 + cc * kk) % n
             want[r, k1 * bins // n] -= v * np.exp(2j * np.pi * ph / n)
     assert np.abs(got - want).max() <= 1e-13
+
+
+def test_tables_of_many_sizes_in_turn():
+    """More bytes of tables than a context keeps (their memory is reused in turns,
+    some calls' in two parts around its end): every call gives the bits that it
+    gave first, in another order and between other sizes, and a new context's."""
+    n = 1 << 16
+    rng = np.random.default_rng(6)
+    x = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    args = (1e-6, 4097, 77, 5, 4099)
+    calls = [(3001 + 8 * i, m.FP64 if i % 3 else m.FP32) for i in range(120)]
+    kept = m.Context(0)
+    sig = kept.upload(x)
+    want = [kept.bin_in_time(sig, b, 2, *args, precision=p) for b, p in calls]
+    for i in [119, 0, 60, 119, 3, 3] + list(range(118, -1, -3)) + [0, 119]:
+        got = kept.bin_in_time(sig, calls[i][0], 2, *args, precision=calls[i][1])
+        assert np.array_equal(got, want[i]), i
+    for i in (0, 1, 59, 119):
+        c = m.Context(0)
+        s = c.upload(x)
+        got = c.bin_in_time(s, calls[i][0], 2, *args, precision=calls[i][1])
+        assert np.array_equal(got, want[i]), i
+        c.close()
+    kept.close()
