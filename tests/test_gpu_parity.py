@@ -842,3 +842,36 @@ def test_iterate_returns_sorted_modes(ctx, count):
     assert not found
     assert list(got) == sorted(mm)
     assert all(got[q] == mm[q] for q in mm)
+
+
+def test_forced_iterate_tables(ctx):
+    """An FP32 Iterate that the precision policy sends to the FP64 kernels takes
+    their tables from the context: the first call at a number of bins, the next and
+    one after other sizes have evicted them give a new context's bits, and the FP64
+    call's coefficients beyond FP32 accuracy."""
+    from mpsft_gb300.signals import make_signal
+
+    sg = make_signal(1 << 16, 20, 9, magnitude="unit", sigma=1e-6)
+
+    def call(c, sig, bins, prec=m.FP32, mm=None):
+        return c.iterate(sig, m.Rng(77 + bins), bins, 1e-5, 1, 3e-6 / np.sqrt(bins), 0.1,
+                         1e-6 / np.sqrt(bins), mm, prec)
+
+    kept = m.Context(0)
+    sig = kept.upload(sg.x)
+    first = {bins: call(kept, sig, bins) for bins in (51, 101, 501)}
+    again = {bins: call(kept, sig, bins) for bins in (501, 51, 101)}
+    for size in range(53, 253, 2):
+        kept.bin_in_time(sig, size, 3, 1e-5, 77, 5, 9, 31, precision=PRECS[size % 4 == 1])
+    for bins, (found, mm) in first.items():
+        fresh = m.Context(0)
+        s = fresh.upload(sg.x)
+        assert found and (found, mm) == again[bins] == call(kept, sig, bins)
+        assert (found, mm) == call(fresh, s, bins), bins
+        _, want = call(fresh, s, bins, m.FP64)
+        assert sorted(mm) == sorted(want)
+        assert max(abs(mm[k] - want[k]) for k in want) < 1e-10
+        # and with the modes found so far
+        assert call(kept, sig, bins, mm=mm) == call(fresh, s, bins, mm=mm)
+        fresh.close()
+    kept.close()
