@@ -190,8 +190,8 @@ struct SigIter {
   int32_t *esc_cnt;
   // per listed bin e: s^k, k < 64, with s = e^{2 pi i (b/n - (2 beta + 1)/(2B))}
   // as float-float {re.hi, im.hi, re.lo, im.lo} at [e * 64 + k], and s^64
-  // (the direct evaluation of every bin; null in solves and iterations,
-  // whose re-binning evaluates them per work item)
+  // (FP32 solves and iterations: by the decision that lists the bin; the direct
+  // evaluation of every bin: by k_rebin_prep)
   float4 *esc_pow;
   double2 *esc_step;
   // per-value part of the FP32 error bound: eps_rel * (kEpsRowMax * max |U|
@@ -325,11 +325,9 @@ __host__ __device__ inline void SetBinsFixedPoint(SigIter *it) {
   it->xi_scale = 1.0 / (2.0 * double(it->n) * double(it->bins));
 }
 
-// phi_b = round(2^64 (b mod n) / n) (n and b set); for n = 2^k it is exactly
-// (b mod n) 2^(64 - k), without the 128-bit division.
-// round(2^64 (b mod n) / n). A length that is no power of two takes two 64-bit
-// divisions by a 31-bit number (a 128-bit one is a call of several hundred
-// instructions, on the one thread that plans a signal).
+// phi_b = round(2^64 (b mod n) / n); for n = 2^k it is exactly (b mod n) 2^(64 - k).
+// Another length takes two 64-bit divisions by a 31-bit number (a 128-bit one is a
+// call of several hundred instructions, on the one warp that plans a signal).
 __host__ __device__ inline uint64_t PhiOf(int32_t b, int32_t n32) {
   int32_t r32 = b % n32;
   if (r32 < 0) r32 += n32;
@@ -409,16 +407,16 @@ __device__ __forceinline__ void PdlEnter(const SigIter *its, int32_t id) {
   }
 }
 
-// PdlEnter for the kernels in the middle of an iteration: signal sig's
-// descriptor is copied to shared memory while the kernel before still runs (Early;
-// else after the wait, its lines at once), and read from there. Every block otherwise starts by walking from the descriptor
-// through its pointers to the data, some 900 cycles a step, and its eight lines
-// came one after the other. The descriptor does not change between the plan (or
-// the upload) and the end of the iteration; a kernel launched early starts when
-// the one before has passed its own wait, so what the kernels before that one
-// wrote is complete. The kernel right behind a writer of descriptors must not
-// copy early. Called by the whole block. (A load before the wait without the copy
-// gained nothing: the wait drops the L1 lines.) One recovery of 1000 modes 906 ->
+// PdlEnter for the kernels in the middle of an iteration: signal sig's descriptor is
+// copied to shared memory while the kernel before still runs (Early; else after the
+// wait, its lines at once), and read from there. Every block otherwise starts by
+// walking from the descriptor through its pointers to the data, some 900 cycles a
+// step, and its eight lines came one after the other. The descriptor does not change
+// between the plan (or the upload) and the end of the iteration; a kernel launched
+// early starts when the one before has passed its own wait, so what the kernels
+// before that one wrote is complete. The kernel right behind a writer of descriptors
+// must not copy early. Called by the whole block. (A load before the wait without the
+// copy gained nothing: the wait drops the L1 lines.) One recovery of 1000 modes 906 ->
 // 843 us, 64 signals 5532 -> 5455 us, an FP64 iteration at 101 bins 109 -> 106 us.
 template <bool Early = true>
 __device__ __forceinline__ const SigIter &PdlEnterLoaded(const SigIter *__restrict__ its,

@@ -29,8 +29,9 @@
 // consecutive runs; lane sums are combined by a fixed shuffle tree and the chunk
 // partials by another in whichever warp finishes a row's last chunk (so the result
 // does not depend on the scheduling). A group of warps takes a listed bin's trial,
-// each every so manieth of its items with one evaluation of the bin's phase-step
-// powers: these are 40 of the 70 FP64 instructions of a single item, 64 cycles each.
+// each every so manieth of its items: it reads the bin's phase-step powers once, and
+// rows that are not listed are no items (64 signals 1.017x against a warp per item
+// that stepped over them).
 #include "common.cuh"
 #include "launch.h"
 #include "rebin.cuh"
@@ -295,8 +296,8 @@ __global__ void __launch_bounds__(256, 2)
         tr += __shfl_xor_sync(0xffffffffu, tr, o);
         ti += __shfl_xor_sync(0xffffffffu, ti, o);
       }
-      // the warp that completes a (trial, row) adds its chunk partials in
-      // chunk order (the result does not depend on which warp that is)
+      // the warp that completes a (trial, row) adds its chunk partials by a fixed
+      // tree (the result does not depend on which warp that is)
       const size_t etr = (size_t(e) * it.trials + t) * it.rows + r;
       int last = 0;
       if (lane == 0) {
