@@ -417,7 +417,8 @@ __device__ __forceinline__ void PdlEnter(const SigIter *its, int32_t id) {
 // before that one wrote is complete. The kernel right behind a writer of descriptors
 // must not copy early. Called by the whole block. (A load before the wait without the
 // copy gained nothing: the wait drops the L1 lines.) One recovery of 1000 modes 906 ->
-// 843 us, 64 signals 5532 -> 5455 us, an FP64 iteration at 101 bins 109 -> 106 us.
+// 843 us, 64 signals 5532 -> 5455 us, an FP64 iteration at 101 bins 109 -> 106 us (the
+// FP32 decisions, a third of the first, no longer take part: k_decide).
 template <bool Early = true>
 __device__ __forceinline__ const SigIter &PdlEnterLoaded(const SigIter *__restrict__ its,
                                                          unsigned sig, int32_t id = 0) {

@@ -308,10 +308,22 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket(const SigIter *__rest
 
 // One warp per bin. cond: only signals whose iteration is redone in FP64
 // (more near-tie bins than their list holds) take part.
+// The FP32 decisions read their descriptor where it lies, in one version for any
+// number of bins: from a copy in shared memory, or with more registers for few bins,
+// the compiler contracts some of their products differently, and a near-tie bound
+// then falls on the other side (8 of 61440 recoveries of 300 modes listed another bin,
+// their coefficients up to 4e-8 off). One recovery of 1000 modes takes 874 us this
+// way and 842 with both, 64 signals 5206 and 5175.
 template <typename T, int TMAX, int MINB>
 __global__ void __launch_bounds__(256, MINB)
     k_decide(const SigIter *__restrict__ its, int mode, int cond, int mark) {
-  const SigIter &it = PdlEnterLoaded(its, blockIdx.y, kTraceDecide);
+  const SigIter *d = its + blockIdx.y;
+  if constexpr (sizeof(T) == sizeof(float)) {
+    PdlEnter(its, kTraceDecide);
+  } else {
+    d = &PdlEnterLoaded(its, blockIdx.y, kTraceDecide);
+  }
+  const SigIter &it = *d;
   if (!it.active) return;
   if (cond ? !RedoFP64(it) : it.force_fp64) return;
   const int beta = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -728,16 +740,10 @@ void LaunchDecideT(const SigIter *d_its, int nsig, int max_bins, int mode,
   // blocks of eight, 21 us in blocks of one)
   const int w = sizeof(T) == 8 && int64_t(max_bins) * nsig <= 152 * 16 ? 1 : 8;
   dim3 grid((max_bins + w - 1) / w, nsig);
-  // FP32, one trial: six blocks per SM (40 registers) while there are more than
-  // four for each, else four (64 registers: the row factors of four modes side by
-  // side). One recovery of 1000 modes 940 us with four throughout, 948 with six; 64
-  // signals 5185 and 5125 us.
-  constexpr bool kSix = sizeof(T) == 4 && TMAX == 1;
-  if (kSix && int64_t(max_bins) * nsig > 152 * 4 * 8) {
-    Launch(k_decide<T, TMAX, kSix ? 6 : 1>, grid, 32 * w, 0, s, d_its, mode, cond, mark);
-  } else {
-    Launch(k_decide<T, TMAX, kSix ? 4 : 1>, grid, 32 * w, 0, s, d_its, mode, cond, mark);
-  }
+  // (FP32, one trial: six blocks per SM, 40 registers, for one signal as for a batch,
+  // so that both round alike)
+  constexpr int kMinBlocks = sizeof(T) == 4 && TMAX == 1 ? 6 : 1;
+  Launch(k_decide<T, TMAX, kMinBlocks>, grid, 32 * w, 0, s, d_its, mode, cond, mark);
 }
 
 template <typename T>

@@ -875,3 +875,26 @@ def test_forced_iterate_tables(ctx):
         assert call(kept, sig, bins, mm=mm) == call(fresh, s, bins, mm=mm)
         fresh.close()
     kept.close()
+
+
+def test_fp32_decisions_keep_their_rounding(ctx):
+    """The near-tie bins that FP32 recoveries list, on signals (8 of 61440) of which
+    one lies within the last bit of its bound: another contraction of the decisions'
+    products, which the compiler may choose when their code changes, lists others.
+    The counts are those of the decisions as first written."""
+    listed = {1382: 2, 7456: 0, 8387: 1, 19610: 2, 25759: 2, 45998: 3, 53756: 2, 59339: 0}
+    n, s = 1 << 18, 300
+    sigs, opts = [], []
+    for i in listed:
+        g = np.random.default_rng([79, i])
+        k = np.sort(g.choice(n, s, replace=False)).astype(np.int32)
+        c = np.exp(g.uniform(np.log(1e-2), 0.0, s)) * np.exp(2j * np.pi * g.uniform(size=s))
+        sigma = float(1e-3 * np.sqrt(np.sum(np.abs(c) ** 2)))
+        sigs.append(ctx.generate(n, k, c, sigma, i, m.C64))
+        opts.append(ctx.solve_options(s, sigma, trials=1, min_bins=51, window_delta=1e-5,
+                                      window_threshold=0.1, max_stale_iter=5,
+                                      precision=m.FP32))
+    _, stats = ctx.solve_batched(sigs, [m.Rng(500 + i) for i in listed], opts)
+    for sg in sigs:
+        sg.free()
+    assert [st["escalated"] for st in stats] == list(listed.values())
